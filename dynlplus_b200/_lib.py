@@ -30,6 +30,8 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_spmm": ("ppppiipipqipddpqdpqiiidp", ct.c_int),
     "dlp_spmm_lowp": ("ppppiipqpqpddpqidp", ct.c_int),
     "dlp_frontier_jacobi": ("ppppipiipqpqpdpqipppidp", ct.c_int),
+    "dlp_frontier_solve_workspace_bytes": ("iii", ct.c_size_t),
+    "dlp_frontier_solve": ("ppppiiipqpqpidpiiidpzppp", ct.c_int),
     "dlp_push_scatter": ("ppppipiipqpqipidp", ct.c_int),
     "dlp_mark_neighbors": ("ppppipp", ct.c_int),
     "dlp_push_take": ("piipqpqppqipp", ct.c_int),

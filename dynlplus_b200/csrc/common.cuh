@@ -108,6 +108,46 @@ __device__ __forceinline__ void load_vec_coherent(const T *p, TA (&out)[VW]) {
 __device__ __forceinline__ void atomic_add(float *p, float v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add(double *p, double v) { atomicAdd(p, v); }
 
+// ---- grid barrier of a cooperative launch -------------------------------------------------------
+// A monotone arrival counter (zeroed by the host before the launch): barrier k is passed when
+// k * gridDim.x blocks have arrived. Every block of the launch is resident (cooperative launch), so a
+// wait ends with the slowest block; the spin is bounded all the same (kBarSpins polls, seconds), and a
+// block that gives up sets `abort`, which ends every other block's wait. Data written by other blocks
+// before the barrier is read through L2 (__ldcg) after it.
+struct GridBar {
+  uint32_t count;
+  int32_t abort;
+};
+constexpr int kBarSpins = 1 << 22;
+
+__device__ __forceinline__ bool grid_barrier(GridBar *b, uint32_t &target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&b->count, 1u);
+    int spins = 0, ok = 1;
+    while (true) {
+      uint32_t c;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&b->count) : "memory");
+      if ((int32_t)(c - target) >= 0) break;
+      if ((++spins & 1023) == 0) {
+        if (*(volatile int32_t *)&b->abort) ok = 0;
+        if (spins >= kBarSpins) {
+          atomicExch(&b->abort, 1);
+          ok = 0;
+        }
+        if (!ok) break;
+      }
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 // Hardware lane id (correct for 1-D and multi-dimensional blocks alike).
 __device__ __forceinline__ int lane_id() {
   unsigned l;

@@ -263,8 +263,9 @@ __device__ __forceinline__ void store_row12(float *yr, const float (&v)[3][4]) {
 // address.
 enum RowPath : int { kRowVec = 0, kRow12F = 1, kRow10D = 2, kRow16H = 3, kRow8F = 4 };
 
+// COH (kRowVec only): X is read through L2, for kernels that write X in the same launch.
 template <typename TW, typename TX, typename TA, int VW, int VPL, int U = gather_batch_wide<TA, VW, VPL>(),
-          int ROW = kRowVec>
+          int ROW = kRowVec, bool COH = false>
 __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, const TW *__restrict__ w,
                                            const TX *__restrict__ X, int64_t ldx, int beg, int end, int es,
                                            int ES, int cl, int LV, int NV, int G, TA (&acc)[VPL][VW]) {
@@ -337,7 +338,8 @@ __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, cons
         for (int k = 0; k < VPL; ++k) {
           const int vi = cl + k * LV;
           if (v[u] >= 0 && vi < NV) {
-            load_vec<TX, VW, TA>(xr + (long long)vi * VW, t[u][k]);
+            if constexpr (COH) load_vec_coherent<TX, VW, TA>(xr + (long long)vi * VW, t[u][k]);
+            else load_vec<TX, VW, TA>(xr + (long long)vi * VW, t[u][k]);
           } else {
 #pragma unroll
             for (int i = 0; i < VW; ++i) t[u][k][i] = TA(0);

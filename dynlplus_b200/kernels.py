@@ -147,6 +147,26 @@ class FrontierOps:
                   ptr(ch), ptr(out_list), ptr(out_count), self.gs, W.nnz / max(W.shape[0], 1), stream())
         return Y, ch.bool()
 
+    def solve(self, frontier, X, rhs, diag, delta, max_rounds):
+        """The frontier rounds from `frontier` until nothing moves by more than delta, X updated in place
+        (dynlp/solvers.py:213-241) in one device-side loop; returns the rounds run and adds their edge
+        visits to `edges`. X keeps its storage, so it must not need gather_view's copy."""
+        import ctypes as ct
+        W = self.W
+        f = frontier.to(torch.int32).contiguous()
+        if not f.numel():
+            return 0
+        rbeg, rend = _rows_of(W)
+        diag, rhs = diag.to(X.dtype).contiguous(), rhs.to(X.dtype)
+        ws = workspace("frontier").get(_lib.lib().dlp_frontier_solve_workspace_bytes(W.shape[0], self.C, code(X)))
+        rounds, edges = ct.c_int32(0), ct.c_ulonglong(0)
+        _lib.call("dlp_frontier_solve", ptr(rbeg), ptr(rend), ptr(W.indices), ptr(W.data), code(W.data), W.shape[0],
+                  self.C, ptr(X), ld(X), ptr(rhs), ld(rhs), ptr(diag), code(X), float(delta), ptr(f), int(f.numel()),
+                  int(max_rounds), self.gs, W.nnz / max(W.shape[0], 1), ptr(ws), ws.numel(), ct.byref(rounds),
+                  ct.byref(edges), stream())
+        self.edges += int(edges.value)
+        return int(rounds.value)
+
     def push(self, frontier, D, R, mark):
         """R += W[:, frontier] @ D (W symmetric) and mark touched vertices (:476-486)."""
         W = self.W

@@ -419,10 +419,13 @@ def push(sys: System, Z, R, eps, ops: FrontierOps, st: Stats, budget_edges=None,
 
 def _comp_avg(lab, nc, S_rows, T_rows, fallback):
     """Per component of the new vertices: sum of S over sum of T (T = 0: fallback)
-    (dynlp/solvers.py:128-135)."""
+    (dynlp/solvers.py:128-135). Summed in fp64, so the order of the atomic additions does not reach the
+    working precision: a last-bit difference here decides which rows a frontier sweep's threshold lets
+    move, and two runs of one stream differed by 1e-4."""
     lab = lab.long()
-    S = torch.zeros((nc,) + tuple(S_rows.shape[1:]), dtype=S_rows.dtype, device=S_rows.device).index_add_(0, lab, S_rows)
-    T = torch.zeros(nc, dtype=S_rows.dtype, device=S_rows.device).index_add_(0, lab, T_rows.to(S_rows.dtype))
+    S = torch.zeros((nc,) + tuple(S_rows.shape[1:]), dtype=F64, device=S_rows.device).index_add_(0, lab, S_rows.to(F64))
+    T = torch.zeros(nc, dtype=F64, device=S_rows.device).index_add_(0, lab, T_rows.to(F64))
+    S, T = S.to(S_rows.dtype), T.to(S_rows.dtype)
     ok = T > 0
     Tn = torch.where(ok, T, torch.ones_like(T))
     fb = torch.as_tensor(fallback, dtype=S_rows.dtype, device=S_rows.device)
@@ -528,7 +531,9 @@ class DynLP(Solver):
     """DynLP's frontier Jacobi (Algorithm 2, dynlp/solvers.py:213-241) on the frontier kernels: the
     new rows start at their component's label share (supernode_init, the paper's tau components or
     the adaptive ones with comp="fh"), the frontier starts at the seed rows; each round updates
-    the rows that changed by more than delta and the next frontier is their neighbourhood."""
+    the rows that changed by more than delta and the next frontier is their neighbourhood. The rounds
+    run on the device (FrontierOps.solve); `record`, a list, receives every round's frontier and keeps
+    the loop on the host."""
 
     def __init__(self, n_total, K, dtype="float32", delta=1e-4, group="auto", comp="tau", max_iter=10**7):
         super().__init__(n_total, K, dtype)
@@ -543,9 +548,10 @@ class DynLP(Solver):
             n = X.shape[0]
             frontier = kernels.flatnonzero(sys.seed.to(torch.uint8))
             mark = torch.zeros(max(n, 1), dtype=torch.uint8, device=X.device)
-            while frontier.numel() and st.iters < self.max_iter:
-                if record is not None:
-                    record.append(frontier.clone())
+            if record is None:
+                st.iters = ops.solve(frontier, X, sys.rhs, sys.diag, self.delta, self.max_iter)
+            while record is not None and frontier.numel() and st.iters < self.max_iter:
+                record.append(frontier.clone())
                 Y, ch = ops.jacobi(frontier, X, sys.rhs, sys.diag, self.delta)
                 st.iters += 1
                 chu = ch.to(torch.uint8)

@@ -99,6 +99,19 @@ int dlp_frontier_jacobi(const int32_t *rbeg, const int32_t *rend, const int32_t 
                         int64_t ldy, int dtype, uint8_t *changed, int32_t *out_list, int32_t *out_count,
                         int32_t group, double avg_deg, dlp_stream_t stream);
 
+/* The whole frontier solve (dynlp/solvers.py:213-241), its rounds on the device in one cooperative
+ * launch: from the seed rows (distinct), every round computes the frontier rows' new values from the
+ * values before the round, X takes those that move by more than delta, and the changed rows with their
+ * stored neighbours are the next frontier; ends when nothing moves or after max_rounds rounds. Per-row
+ * arithmetic as dlp_frontier_jacobi. rounds_out / edges_out (host): rounds run and stored entries
+ * visited (frontier rows, and changed rows when marking). Synchronises the stream. */
+size_t dlp_frontier_solve_workspace_bytes(int32_t n, int32_t C, int dtype);
+int dlp_frontier_solve(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w, int w_dtype,
+                       int32_t n, int32_t C, void *X, int64_t ldx, const void *rhs, int64_t ldr, const void *diag,
+                       int dtype, double delta, const int32_t *seed, int32_t nseed, int32_t max_rounds, int32_t group,
+                       double avg_deg, void *ws, size_t ws_bytes, int32_t *rounds_out, unsigned long long *edges_out,
+                       dlp_stream_t stream);
+
 /* ---- (b) residual push scatter and neighbour marking --------------------------------------
  * Replaces push_scatter (dynlp/kernels.py:105-126, :222-238; FrontierOps.push :476-486):
  *   R[col_j, :] += w_j * D[g, :] for every stored entry j of row frontier[g]; mark[col_j] = 1.
