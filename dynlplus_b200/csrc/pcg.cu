@@ -1,5 +1,5 @@
 // Block PCG with the Jacobi preconditioner, one CG per column (dynlp/solvers.py:66-97), fused for
-// B200: three kernels per iteration, inner products summed in fp64 (fp32 only in the per-lane pAp
+// B200: one launch for the whole solve on systems of up to some 100,000 rows (pcg_whole.cuh), else three kernels per iteration, inner products summed in fp64 (fp32 only in the per-lane pAp
 // partials of the fp32 whole-row apply, about a dozen rows each), convergence decided on the
 // device, and the iteration loop itself on the device (a CUDA graph WHILE node whose flag K2
 // sets), so the host waits once per solve instead of once per chunk of iterations.
@@ -41,6 +41,7 @@ struct PcgCtl {
   // first-level counters of the grid reductions (last_block_grouped), one per group of blocks;
   // zero between launches. The host reads only the fields above them (kCtlHead).
   uint32_t gcnt1[kMaxGroups], gcnt2[kMaxGroups];
+  GridBar bar;  // the one-launch solve's grid barrier
 };
 constexpr size_t kCtlHead = offsetof(PcgCtl, gcnt1);
 
@@ -69,7 +70,7 @@ static size_t pcg_ws_bytes(int C) {
   size_t b = align256(sizeof(PcgCtl));
   b += 7 * align256(sizeof(double) * C);
   b += align256(sizeof(double) * nb * 2 * C);        // part1 (pAp; q of the two-kernel iteration)
-  b += align256(sizeof(double) * nb * (2 * C + 1));  // part2 (rz, ss, violation)
+  b += align256(sizeof(double) * nb * (2 * C + 2));  // part2 (rz, ss, violation; the cancel word)
   b += align256(sizeof(double) * kMaxGroups * 2 * C);        // gpart1
   b += align256(sizeof(double) * kMaxGroups * (2 * C + 1));  // gpart2
   return b;
@@ -129,7 +130,7 @@ static PcgBufs carve(void *ws, int C) {
   B.part1 = (double *)p;
   p += align256(sizeof(double) * nb * 2 * C);
   B.part2 = (double *)p;
-  p += align256(sizeof(double) * nb * (2 * C + 1));
+  p += align256(sizeof(double) * nb * (2 * C + 2));
   B.gpart1 = (double *)p;
   p += align256(sizeof(double) * kMaxGroups * 2 * C);
   B.gpart2 = (double *)p;
@@ -208,6 +209,12 @@ __device__ __forceinline__ bool last_block_grouped(const double *part, long long
   if (threadIdx.x == 0) gcnt[g] = 0;
   return last_of(top, (uint32_t)grid_groups());
 }
+
+}  // namespace dlp
+
+#include "pcg_whole.cuh"
+
+namespace dlp {
 
 // ------------------------------------------------------------------------------------------------
 // K1: AP = diag*P - W P and pAp partials
@@ -1563,6 +1570,89 @@ static int get_loop_graph(const PcgProblem &q, const PcgBufs &B, GraphRef *out) 
   return DLP_OK;
 }
 
+// ---- the whole solve in one launch (pcg_whole.cuh) -----------------------------------------------
+// Values a lane gathers per access, lanes per row of P and per row of W, rows per block. A vector takes
+// 32 bytes where P's rows are whole 32-byte runs, else 16; a row's vectors are read by as many lanes side
+// by side, which the L1 serves line by line. The rows are spread over all SMs, at least kWholeMinRows each, and the lanes that leaves
+// free take more of a row's entries at once, down to one or two per lane.
+struct WholePlan {
+  int VW, LV, G, rows;
+};
+constexpr int kWholeMinRows = 8;
+
+static bool whole_plan(const PcgProblem &q, WholePlan *w) {
+  const int es = q.dtype == DLP_F32 ? 4 : 8;
+  const int small = 16 / es;
+  auto rows_of = [&](int vw) {  // whether P's rows are whole aligned vectors of vw values
+    const int64_t b = (int64_t)vw * es;
+    return q.ldp >= (int64_t)(q.C + vw - 1) / vw * vw && (uintptr_t)q.P % b == 0 && (q.ldp * es) % b == 0;
+  };
+  w->VW = q.C == 1 ? 1 : q.C > small && rows_of(2 * small) ? 2 * small : small;
+  if (!rows_of(w->VW)) return false;
+  w->LV = next_pow2((q.C + w->VW - 1) / w->VW);
+  if (w->LV > 32) return false;
+  const int sms = std::min(sm_count(), kWholeBlocks);
+  w->rows = std::max((q.n + sms - 1) / sms, kWholeMinRows);
+  int slots = std::max(1, (int)(q.avg_deg / 4.0));
+  const int room = kWholeThreads / (w->rows * w->LV);  // lanes a row can have in one pass
+  slots = std::max(slots, std::min(room, (int)q.avg_deg));
+  int p = 1;
+  while (p * 2 <= slots) p *= 2;
+  w->G = w->LV * std::min(p, 32 / w->LV);
+  return true;
+}
+static size_t whole_state(const PcgProblem &q, int rows) {
+  const size_t es = q.dtype == DLP_F32 ? 4 : 8;
+  return (size_t)rows * (4 * es * q.C + es + 8 + 8) + 64;
+}
+
+template <class T, int VW>
+static int launch_whole_t(WholeArgs<T> &a, cudaStream_t s) {
+  auto *kern = k_pcg_whole<T, VW>;
+  static const cudaError_t set =
+      cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSmem);
+  DLP_CUDA(set);
+  void *argv[] = {(void *)&a};
+  const int grid = (a.n + a.rows - 1) / a.rows;
+  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kWholeThreads), argv, kWholeSmem, s));
+  return check_launch();
+}
+
+template <class T>
+static int launch_whole(const PcgProblem &q, const PcgBufs &B, const WholePlan &w, bool zero, bool confirm,
+                        cudaStream_t s) {
+  using TX = typename T::TX;
+  WholeArgs<T> a{q.rbeg, q.rend, q.col, (const typename T::TW *)q.w, q.n, q.C, w.rows, (const TX *)q.diag,
+                 (const TX *)q.rhs, q.ldrhs, (TX *)q.Z, q.ldz, (TX *)q.R, q.ldr, (TX *)q.P, q.ldp, B,
+                 &B.ctl->bar, w.G, w.LV, zero ? 1 : 0,
+                 confirm ? 1 : 0};
+  constexpr int VWV = 16 / sizeof(TX);
+  if (w.VW == 1) return launch_whole_t<T, 1>(a, s);
+  if (w.VW == VWV) return launch_whole_t<T, VWV>(a, s);
+  return launch_whole_t<T, 2 * VWV>(a, s);
+}
+
+// Whether the solve runs in one launch: up to kWholeRows rows (the entries of a block's rows then fit its
+// shared memory at the degrees of the workloads) and a score block of at most kWholeBytes, or
+// kWholeBytesFused where the launches would be the two-kernel iteration on whole rows. Measured on B200
+// (degree 16, us per iteration, launches / one launch): 1 column at n = 100,000 37 / 22, at 200,000 47 / 51;
+// 5 columns at 100,000 (2.0 MB) 34 / 26, at 200,000 46 / 55; 9 columns at 60,000 (2.2 MB) 37 / 33, at
+// 100,000 (3.6 MB) 47 / 51; 17 columns at 60,000 (4.1 MB) 58 / 44, at 100,000 72 / 72; 5 fp64 columns at
+// 60,000 (2.4 MB) 46 / 38, at 100,000 (4.0 MB) 55 / 55.
+constexpr int kWholeRows = 100000;
+constexpr size_t kWholeBytes = 4200000, kWholeBytesFused = 2500000;
+static bool whole_fits(const PcgProblem &q, WholePlan *w) {
+  const size_t bytes = (size_t)q.n * q.C * (q.dtype == DLP_F32 ? 4 : 8);
+  if (q.w_lo || q.C > kWholeMaxC || q.n > kWholeRows || bytes > (q.fused ? kWholeBytesFused : kWholeBytes)) return false;
+  return whole_plan(q, w) && whole_state(q, w->rows) <= (size_t)kWholeSmem;
+}
+
+static int whole_solve(const PcgProblem &q, const PcgBufs &B, const WholePlan &L, bool zero, bool confirm, cudaStream_t s) {
+  if (q.dtype == DLP_F32) return launch_whole<T_F32>(q, B, L, zero, confirm, s);
+  if (q.w_dtype == DLP_F64) return launch_whole<T_F64>(q, B, L, zero, confirm, s);
+  return launch_whole<T_W32X64>(q, B, L, zero, confirm, s);
+}
+
 }  // namespace dlp
 
 using namespace dlp;
@@ -1632,6 +1722,20 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
     }
     DLP_CUDA(cudaMemcpyAsync(B.ctl, img, head_bytes(C), cudaMemcpyHostToDevice, s));
     DLP_CUDA(cudaEventRecord(hs->up, s));
+  }
+  WholePlan whole;
+  if (use_graph && !(mode & 8) && whole_fits(q, &whole)) {
+    DLP_TRY(whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s));
+    PcgCtl cur{};
+    DLP_TRY(read_ctl(B, hs, s, &cur));
+    if (cur.done == 0) return DLP_ERR_DEVICE;  // a barrier's wait ran out
+    if (iters_out) *iters_out = cur.iters;
+    if (viol_out) *viol_out = cur.viol;
+    if (relres_out) *relres_out = cur.relres;
+    if (status_out) *status_out = cur.done;
+    if (cur.done == 3) return DLP_ERR_CAP;
+    if (cur.done == 6) return DLP_ERR_CANCELLED;
+    return DLP_OK;
   }
   // R = rhs - A Z, best = violation, rz = R.(R/diag), P = R/diag; a zero start takes R = rhs in the
   // update sweep itself and sets Z = 0 in the direction sweep (no SpMM, no separate copy)

@@ -46,3 +46,84 @@ def test_frontier_rounds_on_the_device_equal_the_host_loop(n, K, dtype, deg, max
     assert torch.equal(a.F, b.F)
     assert sa.iters == sb.iters == len(rounds) and sa.edges == sb.edges
     assert sa.iters == min(sa.iters, max_iter)
+
+
+def pcg_case(n, C, dtype, deg=8, seed=0):
+    """A grounded system A = diag - W of n rows (some without entries) and right-hand sides."""
+    rng = np.random.default_rng(seed)
+    m = int(n * deg / 2)
+    import scipy.sparse as ssp
+    u, v = rng.integers(0, n, m), rng.integers(0, n, m)
+    W = ssp.coo_matrix((rng.uniform(0.2, 1.5, m), (u, v)), (n, n)).tocsr()
+    W = W + W.T
+    W.setdiag(0)
+    W.eliminate_zeros()
+    W = W.astype(np.float32)
+    diag = np.asarray(W.sum(1)).ravel().astype(np.float64) + rng.uniform(0.05, 0.5, n)
+    rhs = rng.uniform(0, 1, (n, C))
+    dt = getattr(torch, dtype)
+    from dynlplus_b200.backend import CSR
+    Wd = CSR.from_scipy(W)
+    if not Wd.indices.numel():  # the kernels want valid pointers
+        Wd = CSR(torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), Wd.indptr, Wd.shape)
+
+    class Sys:
+        pass
+    S = Sys()
+    S.W, S.nnz = Wd, int(W.nnz)
+    S.diag = torch.as_tensor(diag).to(dt).cuda()
+    return S, W, S.diag.double().cpu().numpy(), torch.as_tensor(rhs).to(dt).cuda()
+
+
+# block boundaries of the rows (8 per block, then 148 blocks), one and several vectors per row, both vector
+# widths, the size the launch path starts at (100,000 rows) and the next one
+@pytest.mark.parametrize("n,C,dtype", [(1, 1, "float32"), (7, 4, "float32"), (9, 5, "float64"), (8 * 148, 8, "float32"),
+                                       (8 * 148 + 1, 9, "float32"), (5000, 3, "float64"), (5001, 17, "float32"),
+                                       (3000, 33, "float32"), (2999, 64, "float32"), (4001, 64, "float64"),
+                                       (100_000, 1, "float32"), (100_001, 1, "float32")])
+def test_whole_solve_in_one_launch_equals_the_kernel_loop(n, C, dtype):
+    """The one-launch PCG against the same iteration launched kernel by kernel: iteration counts within one
+    and both at the target (a rounding can move the stop by an iteration), the iterates together, from
+    zero and from a given start, with the recheck and without."""
+    import scipy.sparse as ssp
+    S, W, diag, rhs = pcg_case(n, C, dtype, seed=n + C)
+    f32 = dtype == "float32"
+    target = 1e-4 if f32 else 1e-11
+    A = ssp.diags(diag) - W.astype(np.float64)
+    b = rhs.double().cpu().numpy()
+    for zero, confirm in ((True, True), (False, True), (True, False)):
+        out = []
+        for graph in (True, False):
+            Z = solvers.padded_empty(n, C, rhs.dtype, "cuda", fill=0.25)
+            st = solvers.Stats()
+            solvers.TWO_KERNEL = graph
+            try:
+                solvers.pcg(S, Z, rhs, None, solvers.jacobi_M(S), 3000, st, target_relres=target, use_graph=graph,
+                            zero_start=zero, confirm=confirm)
+            finally:
+                solvers.TWO_KERNEL = True
+            out.append((Z.double().cpu().numpy(), st.iters))
+        assert abs(out[0][1] - out[1][1]) <= 1
+        for Z, _ in out:
+            assert (np.linalg.norm(b - A @ Z, axis=0) / np.linalg.norm(b, axis=0)).max() <= 1.2 * target
+        # two iterates at relative residual t differ by at most 2 t cond(A); diagonal dominance by at
+        # least 0.05 bounds the inverse
+        assert np.abs(out[0][0] - out[1][0]).max() <= 2.4 * target * np.linalg.norm(b, axis=0).max() / 0.05
+
+
+def test_whole_solve_stop_rules():
+    """Iteration cap, patience, an unreachable target and a non-finite right-hand side, as in the loop."""
+    S, W, diag, rhs = pcg_case(4000, 5, "float32", seed=2)
+    for graph in (True, False):
+        st, Z = solvers.Stats(), solvers.padded_empty(4000, 5, torch.float32, "cuda")
+        solvers.pcg(S, Z, rhs, None, solvers.jacobi_M(S), 7, st, target_relres=1e-12, use_graph=graph, zero_start=True)
+        assert st.iters == 7
+        st = solvers.Stats()
+        solvers.pcg(S, Z, rhs, None, solvers.jacobi_M(S), 3000, st, target_relres=1e-30, patience=20, use_graph=graph,
+                    zero_start=True)
+        assert st.iters < 200
+        bad = rhs.clone()
+        bad[17, 3] = float("nan")
+        with pytest.raises(FloatingPointError):
+            solvers.pcg(S, Z, bad, None, solvers.jacobi_M(S), 50, solvers.Stats(), target_relres=1e-5, use_graph=graph,
+                        zero_start=True)
