@@ -87,7 +87,7 @@ def config(a):
             "batch_updates": a.batch, "insert_frac": 0.5, "target_relres": a.target_relres, "tol": a.tol,
             "l2": "flushed before every timed step (256 MB write)", "parallelism": "replicas",
             "pcg_iteration": "three kernels" if a.three_kernel else "two kernels (fp32 whole rows)",
-            "class_sum": "off" if a.no_class_sum else "auto (on for k = 4, 8, 12)",
+            "class_sum": "off" if a.no_class_sum else "auto (on for k = 4, 8, 12, 16, 32)",
             "refine_share": a.refine_share,
             "python_gc": "collected before the timed loops, paused during them"}
 

@@ -29,6 +29,8 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_set_cancel_word": ("p", ct.c_int),
     "dlp_spmm": ("ppppiipipqipddpqdpqiiidp", ct.c_int),
     "dlp_spmm_lowp": ("ppppiipqpqpddpqidp", ct.c_int),
+    "dlp_spmm_workspace_bytes": ("iipqid", ct.c_size_t),
+    "dlp_spmm_ws": ("ppppiiipqipddpqdpqiidpzp", ct.c_int),
     "dlp_frontier_jacobi": ("ppppipiipqpqpdpqipppidp", ct.c_int),
     "dlp_frontier_solve_workspace_bytes": ("iii", ct.c_size_t),
     "dlp_frontier_solve": ("ppppiiipqpqpidpiiidpzppp", ct.c_int),

@@ -345,6 +345,22 @@ static int run_spmm(const int32_t *rbeg, const int32_t *rend, const int32_t *col
   return launch_spmm_vw<T, VWV>(p, L.VPL, s);
 }
 
+// Rows of C values copied to a 16-byte pitch, the padding zero: one thread per output vector. Bound by
+// memory (some 15 us for 500,000 rows of 17 floats); the SpMM on such rows gathers vectors instead of
+// scalars: n = 500,000, degree 16, 17 fp32 columns 247 us -> 137 us and the copy; n = 400,000, 9 columns
+// 102 -> 79 us copy included, 9 bf16 columns 142 -> 68. fp64 rows gain nothing (17 columns 210 -> 259).
+template <typename U, int VW>
+__global__ void k_pad_rows(int32_t n, int32_t C, const U *__restrict__ X, int64_t ldx, uint4 *__restrict__ P, int NV) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)n * NV) return;
+  const long long r = t / NV;
+  const int c0 = (int)(t - r * NV) * VW;
+  __align__(16) U v[VW];
+#pragma unroll
+  for (int i = 0; i < VW; ++i) v[i] = c0 + i < C ? X[r * ldx + c0 + i] : U(0);
+  P[t] = *reinterpret_cast<const uint4 *>(v);
+}
+
 // ------------------------------------------------------------------------------------------------
 // Frontier Jacobi (dynlp/kernels.py:31-103, :186-220)
 // ------------------------------------------------------------------------------------------------
@@ -571,6 +587,41 @@ int dlp_spmm(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const
   if (w_dtype == DLP_BF16 && x_dtype == DLP_BF16 && y_dtype == DLP_BF16) return run_spmm<T_BF16B>(DLP_SPMM_ARGS);
 #undef DLP_SPMM_ARGS
   return DLP_ERR_DTYPE;
+}
+
+static int64_t padded_ld(int32_t C, size_t es) { return (int64_t)((C * es + 15) / 16 * 16 / es); }
+
+// Whether X's rows are worth a copy to a vector pitch: fp32 or bf16 rows of three columns or more that
+// cannot be gathered as vectors, at least four gathers per copied row, and 12 M gathered values (below,
+// the whole call is bound by its launches).
+static bool pad_pays(int32_t n, int32_t C, const void *X, int64_t ldx, int x_dtype, double avg_deg) {
+  const size_t es = dtype_size(x_dtype);
+  if (x_dtype == DLP_F64 || es == 0 || C < 3 || avg_deg < 4.0 || avg_deg * n * C < 12e6) return false;
+  return (uintptr_t)X % 16 != 0 || (ldx * (int64_t)es) % 16 != 0 || ldx < padded_ld(C, es);
+}
+
+size_t dlp_spmm_workspace_bytes(int32_t n, int32_t C, const void *X, int64_t ldx, int x_dtype, double avg_deg) {
+  if (n <= 0 || C <= 0 || !pad_pays(n, C, X, ldx, x_dtype, avg_deg)) return 0;
+  return (size_t)n * (size_t)padded_ld(C, dtype_size(x_dtype)) * dtype_size(x_dtype);
+}
+
+int dlp_spmm_ws(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w, int w_dtype, int32_t n,
+                int32_t C, const void *X, int64_t ldx, int x_dtype, const void *a, double alpha, double b,
+                const void *RHS, int64_t ldr, double cr, void *Y, int64_t ldy, int y_dtype, int32_t group,
+                double avg_deg, void *ws, size_t ws_bytes, dlp_stream_t stream) {
+  if (n < 0 || C <= 0 || ldx < C) return DLP_ERR_INVALID;
+  const size_t need = dlp_spmm_workspace_bytes(n, C, X, ldx, x_dtype, avg_deg);
+  if (need > 0 && X && ws && ws_bytes >= need && (uintptr_t)ws % 16 == 0) {
+    const int VW = (int)(16 / dtype_size(x_dtype)), NV = (C + VW - 1) / VW;
+    const int grid = ceil_div_i((long long)n * NV, 256);
+    if (VW == 4) k_pad_rows<uint32_t, 4><<<grid, 256, 0, (cudaStream_t)stream>>>(n, C, (const uint32_t *)X, ldx, (uint4 *)ws, NV);
+    else k_pad_rows<uint16_t, 8><<<grid, 256, 0, (cudaStream_t)stream>>>(n, C, (const uint16_t *)X, ldx, (uint4 *)ws, NV);
+    DLP_TRY(check_launch());
+    X = ws;
+    ldx = padded_ld(C, dtype_size(x_dtype));
+  }
+  return dlp_spmm(rbeg, rend, col, w, w_dtype, n, nullptr, C, X, ldx, x_dtype, a, alpha, b, RHS, ldr, cr, Y, ldy,
+                  y_dtype, 0, group, avg_deg, stream);
 }
 
 int dlp_spmm_lowp(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w_lo, int32_t n_rows,

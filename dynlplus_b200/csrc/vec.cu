@@ -162,11 +162,15 @@ __global__ void k_class_sum_rhs(int32_t n, int32_t K, const double *__restrict__
     }
     return;
   }
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
+  // eight lanes per row, each every eighth column: rows are read in 64-byte runs (one thread per row
+  // touched a line per lane and column)
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, rows = ((long long)gridDim.x * blockDim.x) >> 3;
+  for (long long r = t >> 3; r < n; r += rows) {
     const double *rr = R + r * ldr;
-    float *er = E + r * lde;
-    for (int j = 0; j < K - 1; ++j) er[j] = (float)(rr[j] / scale[j]);
-    er[K - 1] = (float)(rr[K] / scale[K]);
+    for (int j = (int)(t & 7); j < K; j += 8) {
+      const int c = j < K - 1 ? j : K;
+      E[r * lde + j] = (float)(rr[c] / scale[c]);
+    }
   }
 }
 
@@ -197,17 +201,25 @@ __global__ void k_class_sum_update(int32_t n, int32_t K, const float *__restrict
     }
     return;
   }
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
-    const float *dr = D + r * ldd;
-    double *zr = Z + r * ldz;
+  // eight lanes per row as in k_class_sum_rhs; the loop bound is the same for a warp's lanes (they
+  // shuffle)
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, rows = ((long long)gridDim.x * blockDim.x) >> 3;
+  for (long long r0 = (t >> 5) << 2; r0 < n; r0 += rows) {
+    const long long r = r0 + ((t >> 3) & 3);
     double sum = 0.0;
-    for (int j = 0; j < K - 1; ++j) {
-      const double z = zr[j] + (double)dr[j] * scale[j];
-      zr[j] = z;
-      sum += z;
+    if (r < n) {
+      const float *dr = D + r * ldd;
+      double *zr = Z + r * ldz;
+      for (int j = (int)(t & 7); j < K; j += 8) {
+        const int c = j < K - 1 ? j : K;
+        const double z = zr[c] + (double)dr[j] * scale[c];
+        zr[c] = z;
+        if (j < K - 1) sum += z;
+      }
     }
-    zr[K] = zr[K] + (double)dr[K - 1] * scale[K];
-    zr[K - 1] = (!solved || solved[r]) ? 1.0 - sum : 0.0;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (r < n && (t & 7) == 0) Z[r * ldz + K - 1] = (!solved || solved[r]) ? 1.0 - sum : 0.0;
   }
 }
 

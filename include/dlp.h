@@ -86,6 +86,15 @@ int dlp_spmm_lowp(const int32_t *rbeg, const int32_t *rend, const int32_t *col, 
                   int32_t C, const void *X_lo, int64_t ld_lo, const void *X_own, int64_t ld_own, const void *a,
                   double alpha, double b, void *Y, int64_t ldy, int32_t group, double avg_deg, dlp_stream_t stream);
 
+/* dlp_spmm over all n rows of a square operator (no row list), with scratch for X: where X's rows cannot
+ * be gathered as 16-byte vectors and are gathered often enough (dlp_spmm_workspace_bytes > 0), they are
+ * first copied to rows of whole vectors there. With less scratch it runs as dlp_spmm. */
+size_t dlp_spmm_workspace_bytes(int32_t n, int32_t C, const void *X, int64_t ldx, int x_dtype, double avg_deg);
+int dlp_spmm_ws(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w, int w_dtype, int32_t n,
+                int32_t C, const void *X, int64_t ldx, int x_dtype, const void *a, double alpha, double b,
+                const void *RHS, int64_t ldr, double cr, void *Y, int64_t ldy, int y_dtype, int32_t group,
+                double avg_deg, void *ws, size_t ws_bytes, dlp_stream_t stream);
+
 /* ---- (b) frontier Jacobi ------------------------------------------------------------------
  * Replaces the frontier_jacobi kernels (dynlp/kernels.py:31-103, :186-220; FrontierOps.jacobi
  * :464-474): for g < nf, r = frontier[g]:

@@ -127,3 +127,52 @@ def test_whole_solve_stop_rules():
         with pytest.raises(FloatingPointError):
             solvers.pcg(S, Z, bad, None, solvers.jacobi_M(S), 50, solvers.Stats(), target_relres=1e-5, use_graph=graph,
                         zero_start=True)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float64"])
+@pytest.mark.parametrize("C", [3, 7, 8, 9, 16, 17, 32, 33, 64])
+def test_spmm_layouts_and_padded_copies(C, dtype):
+    """The SpMM over rows on a vector pitch, on their own odd pitch and on an offset view, at a size where
+    odd rows are copied to a vector pitch, against an fp64 product. Tolerance: the working precision's unit
+    roundoff times the row's length and weight sum (fp32 accumulation for bf16)."""
+    from dynlplus_b200 import kernels
+    from dynlplus_b200.backend import CSR
+    n, dt = max(200_000, int(13e6 / C / 8)), getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(C)
+    deg = torch.randint(0, 16, (n,), generator=g, device="cuda")
+    ip = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    ip[1:] = torch.cumsum(deg, 0)
+    m = int(ip[-1])
+    col = torch.randint(0, n, (m,), generator=g, device="cuda")
+    w = torch.rand(m, generator=g, device="cuda").to(dt)
+    W = CSR(w, col.to(torch.int32), ip.to(torch.int32), (n, n))
+    base = torch.rand((n, C + 8), generator=g, device="cuda").to(dt)
+    a = torch.rand(n, generator=g, device="cuda").to(torch.float32 if dtype == "bfloat16" else dt)
+    A = torch.sparse_csr_tensor(ip, col, w.double(), (n, n))
+    tol = 16 * 16 * (2.0 ** -53 if dtype == "float64" else 2.0 ** -24)
+    pad = (C * base.element_size() + 15) // 16 * 16 // base.element_size()
+    for X in (base[:, :C].contiguous(), base[:, 1:C + 1], torch.nn.functional.pad(base[:, :C], (0, pad - C))[:, :C]):
+        Y = kernels.spmm_axpy(W, X, a=a, b=-1.0)
+        want = a.double()[:, None] * X.double() - A @ X.double()
+        assert float((Y.double() - want).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("K", [16, 32])
+def test_wide_class_sum_corrections(K):
+    """Corrections with the last class derived, at the widths where they are on by default: the target is
+    met on the fp64 residual of every column and the scores of solved rows sum to one."""
+    n = 5000
+    ds = graphs.planted_partition(n, K, 12, 4, weights="lognormal", seed=K)
+    lab = graphs.label_mask(n, 0.05, seed=K)
+    es = stream.EdgeStream(ds, lab)
+    solver = solvers.IncrementalLP(n, K, "float32", tol=1e-3, method="pcg", target_relres=1e-6)
+    assert solver.class_sum
+    solver.solve(es.system)
+    up = graphs.EdgeUpdates(ds.A, seed=1, weights="lognormal")
+    for _ in range(3):
+        S = es.apply_edges(**up.next(200))
+        st = solver.solve(S)
+        S64 = S.astype(torch.float64)
+        R = solvers.residual(S64, solver.Z[:, :K].contiguous(), S64.rhs.contiguous())
+        assert st.relres <= 1e-6 and float((R.norm(dim=0) / S64.rhs.norm(dim=0)).max()) <= 1.01e-6
+        assert float((solver.Z[:, :K][S.solved].sum(1) - 1).abs().max()) <= 1e-9
