@@ -23,16 +23,21 @@ size_t compact_ws_bytes(int32_t n);
 constexpr int kAT = 256;
 static int g1(long long w) { return ceil_div_i(w > 0 ? w : 1, kAT); }
 
-// mode 0: u unmatched, neighbours unmatched; mode 1: u unmatched, neighbours matched.
+// mode 0: u unmatched, neighbours unmatched; mode 1: u unmatched, neighbours matched. Eight lanes per
+// vertex scan its row in 32-byte runs and keep the heaviest admissible neighbour, the smallest id among
+// ties (the choice does not depend on the order). Bound by the row reads and the flags of the neighbours;
+// one thread per row walked a chain of dependent loads: n = 120,000, degree 32, its levels included,
+// 24 launches 3,080 -> 420 us.
 __global__ void k_best_choice(int32_t n, const int32_t *__restrict__ indptr, const int32_t *__restrict__ col,
                               const float *__restrict__ w, const uint8_t *__restrict__ matched, int mode,
                               int32_t *choice) {
-  const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= n) return;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long u = t >> 3;
+  const bool valid = u < n;
   int32_t pick = n;
-  if (!matched[u]) {
-    float best = -INFINITY;
-    for (int j = indptr[u]; j < indptr[u + 1]; ++j) {
+  float best = -INFINITY;
+  if (valid && !matched[u]) {
+    for (int j = indptr[u] + (int)(t & 7); j < indptr[u + 1]; j += 8) {
       const int32_t v = col[j];
       const bool ok = mode == 0 ? !matched[v] : matched[v];
       if (!ok) continue;
@@ -43,7 +48,16 @@ __global__ void k_best_choice(int32_t n, const int32_t *__restrict__ indptr, con
       }
     }
   }
-  choice[u] = pick;
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) {
+    const float x = __shfl_xor_sync(0xffffffffu, best, off);
+    const int32_t v = __shfl_xor_sync(0xffffffffu, pick, off);
+    if (x > best || (x == best && v < pick)) {
+      best = x;
+      pick = v;
+    }
+  }
+  if (valid && (t & 7) == 0) choice[u] = pick;
 }
 
 __global__ void k_mutual(int32_t n, const int32_t *__restrict__ choice, uint8_t *matched, int32_t *agg) {
@@ -91,11 +105,77 @@ __global__ void k_fill_members(int32_t n, const int32_t *__restrict__ agg, const
   }
 }
 
-__global__ void k_sort_members(int32_t nc, const int32_t *__restrict__ off, int32_t *members) {
+// Members in ascending order. Up to 32: a warp per aggregate counts, for each member, the smaller ids (they
+// are distinct). Longer lists (unmatched vertices join their heaviest neighbour, so a few aggregates gather
+// a thousand): a block marks the ids in a bitmap of all n in shared memory and writes the set bits back in
+// order; a list's length squared in one thread bounded the setup (n = 120,000, three levels: 2,970 us).
+__global__ void __launch_bounds__(kAT) k_sort_members(int32_t nc, const int32_t *__restrict__ off, int32_t *members) {
+  const long long a = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (a >= nc) return;
+  const int b = off[a], L = off[a + 1] - b;
+  if (L > 32) return;
+  const int32_t x = lane < L ? members[b + lane] : 0x7fffffff;
+  int rank = 0;
+  for (int k = 0; k < L; ++k) rank += __shfl_sync(0xffffffffu, x, k) < x;
+  if (lane < L) members[b + rank] = x;
+}
+
+// The aggregates of more than `more` members among this block's share (blockDim.x at a time), one after
+// another: fn(a) is called by the whole block.
+template <class Fn>
+__device__ __forceinline__ void for_long_aggregates(int32_t nc, const int32_t *off, int more, Fn fn) {
+  __shared__ int32_t s_list[kAT];
+  __shared__ int s_n;
+  for (long long a0 = (long long)blockIdx.x * kAT; a0 < nc; a0 += (long long)gridDim.x * kAT) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const long long a = a0 + threadIdx.x;
+    if (a < nc && off[a + 1] - off[a] > more) s_list[atomicAdd(&s_n, 1)] = (int32_t)a;
+    __syncthreads();
+    const int m = s_n;
+    for (int i = 0; i < m; ++i) fn(s_list[i]);
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kAT) k_sort_members_long(int32_t n, int32_t nc, const int32_t *__restrict__ off,
+                                                           int32_t *members) {
+  extern __shared__ uint32_t s_bits[];
+  __shared__ int32_t s_cnt[kAT];
+  const int words = (n + 31) / 32, tid = threadIdx.x;
+  const int per = (words + kAT - 1) / kAT;  // words of a thread: consecutive, so the order is the ids'
+  for_long_aggregates(nc, off, 32, [&](int32_t a) {
+    const int b = off[a], e = off[a + 1];
+    for (int i = tid; i < words; i += kAT) s_bits[i] = 0u;
+    __syncthreads();
+    for (int i = b + tid; i < e; i += kAT) atomicOr(&s_bits[members[i] >> 5], 1u << (members[i] & 31));
+    __syncthreads();
+    int c = 0;
+    const int w0 = min(tid * per, words), w1 = min(w0 + per, words);
+    for (int i = w0; i < w1; ++i) c += __popc(s_bits[i]);
+    s_cnt[tid] = c;
+    __syncthreads();
+    for (int o = 1; o < kAT; o <<= 1) {  // inclusive scan of the threads' counts
+      const int v = tid >= o ? s_cnt[tid - o] : 0;
+      __syncthreads();
+      s_cnt[tid] += v;
+      __syncthreads();
+    }
+    int at = b + s_cnt[tid] - c;
+    for (int i = w0; i < w1; ++i)
+      for (uint32_t m = s_bits[i]; m; m &= m - 1) members[at++] = i * 32 + __ffs(m) - 1;
+    __syncthreads();
+  });
+}
+
+// lists longer than 32 of graphs whose bitmap does not fit shared memory (some 1.8 M vertices): insertion sort
+__global__ void k_sort_members_serial(int32_t nc, const int32_t *__restrict__ off, int32_t *members) {
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= nc) return;
   const int b = off[a], e = off[a + 1];
-  for (int i = b + 1; i < e; ++i) {  // aggregates are small: insertion sort
+  if (e - b <= 32) return;
+  for (int i = b + 1; i < e; ++i) {
     const int32_t x = members[i];
     int j = i - 1;
     while (j >= b && members[j] > x) {
@@ -104,6 +184,25 @@ __global__ void k_sort_members(int32_t nc, const int32_t *__restrict__ off, int3
     }
     members[j + 1] = x;
   }
+}
+
+static int sort_members(int32_t n, int32_t nc, const int32_t *off, int32_t *members, cudaStream_t s) {
+  k_sort_members<<<g1(32LL * nc), kAT, 0, s>>>(nc, off, members);
+  DLP_TRY(check_launch());
+  const size_t bits = ((size_t)n + 31) / 32 * 4;
+  static const size_t most = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    v -= 4096;  // the kernel's own arrays
+    return v > 0 && cudaFuncSetAttribute((const void *)k_sort_members_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         v) == cudaSuccess ? (size_t)v : (size_t)0;
+  }();
+  if (bits <= most)
+    k_sort_members_long<<<std::min(sm_count(), g1(nc)), kAT, bits, s>>>(n, nc, off, members);
+  else
+    k_sort_members_serial<<<g1(nc), kAT, 0, s>>>(nc, off, members);
+  return check_launch();
 }
 
 // upper bound of coarse row lengths (sum of member degrees) and the table capacity per row
@@ -211,15 +310,61 @@ __global__ void k_run_starts(long long m, const long long *__restrict__ key, int
   flag[i] = (k != kNoKey && (i == 0 || key[i - 1] != k)) ? 1 : 0;
 }
 
-// one thread per run: the run's sum (front to back) becomes coarse entry pos[i]; rows counted
+// One thread per run: the run's sum becomes coarse entry pos[i]; rows counted. The first kRunHead entries
+// are summed front to back, eight loaded before the first is used; the rest of a longer run (between two
+// aggregates that gathered many vertices: thousands) is summed by the warp, 128 entries at a time in a
+// fixed tree. Entry by entry, a run's length in dependent loads bounded the launch (n = 120,000, nine
+// launches: 6,490 us).
+constexpr int kRunHead = 64;
 __global__ void k_run_emit(long long m, const long long *__restrict__ key, const double *__restrict__ val,
                            const int32_t *__restrict__ flag, const int32_t *__restrict__ pos, int32_t nc,
                            int32_t *col_c, float *w_c, int32_t *rowcnt) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m || !flag[i]) return;
-  const long long k = key[i];
-  double acc = val[i];
-  for (long long j = i + 1; j < m && key[j] == k; ++j) acc += val[j];
+  const int lane = threadIdx.x & 31;
+  const bool mine = i < m && flag[i];
+  const long long k = mine ? key[i] : kNoKey;
+  double acc = mine ? val[i] : 0.0;
+  bool in = mine;
+  long long j0 = i + 1;
+  for (; in && j0 < i + 1 + kRunHead; j0 += 8) {
+    long long kk[8];
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const long long j = j0 + u;
+      kk[u] = j < m ? key[j] : kNoKey;
+      v[u] = j < m ? val[j] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      in = in && kk[u] == k;
+      if (in) acc += v[u];
+    }
+  }
+  __syncwarp();
+  for (unsigned todo = __ballot_sync(0xffffffffu, in); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const long long kr = __shfl_sync(0xffffffffu, k, src);
+    long long j = __shfl_sync(0xffffffffu, j0, src);
+    double part = 0.0;
+    for (bool more = true; more; j += 128) {
+      long long kk[4];
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const long long q = j + u * 32 + lane;
+        kk[u] = q < m ? key[q] : kNoKey;
+        v[u] = q < m ? val[q] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) part += kk[u] == kr ? v[u] : 0.0;
+      more = __shfl_sync(0xffffffffu, kk[3] == kr ? 1 : 0, 31) != 0;  // keys are sorted: the last one tells
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+    if (lane == src) acc += part;
+  }
+  if (!mine) return;
   const int32_t a = (int32_t)(k / nc);
   col_c[pos[i]] = (int32_t)(k - (long long)a * nc);
   w_c[pos[i]] = (float)acc;
@@ -237,6 +382,9 @@ __global__ void k_member_sum(int32_t nc, const int32_t *__restrict__ off, const 
 }
 
 // ---- cycle kernels ------------------------------------------------------------------------------
+// Rc[a, c] = sum of R[member, c]: one thread per value up to kShortSum members, four members' rows in
+// flight, summed in member order; a block per longer aggregate (k_restrict_long).
+constexpr int kShortSum = 64;
 template <typename T>
 __global__ void k_restrict(int32_t nc, int32_t C, const int32_t *__restrict__ off, const int32_t *__restrict__ members,
                            const T *__restrict__ R, int64_t ldr, T *Rc, int64_t ldc) {
@@ -245,8 +393,51 @@ __global__ void k_restrict(int32_t nc, int32_t C, const int32_t *__restrict__ of
   const long long a = t / C;
   const int c = (int)(t % C);
   T s = T(0);
-  for (int i = off[a]; i < off[a + 1]; ++i) s += R[(long long)members[i] * ldr + c];
+  const int b = off[a], e = off[a + 1];
+  if (e - b > kShortSum) return;
+  for (int i = b; i < e; i += 4) {
+    T v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = i + u < e ? R[(long long)members[i + u] * ldr + c] : T(0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u < e) s += v[u];
+  }
   Rc[a * ldc + c] = s;
+}
+
+// The aggregates of more than kShortSum members: the block brings tiles of member rows to shared memory (all
+// rows of a tile in flight) and one thread per column adds them in member order, as k_restrict does, up to
+// 64 columns a pass. The longest list in one thread's dependent loads bounded the restriction (the
+// 120,000-row hierarchy, 51 launches: 1,390 us).
+constexpr int kSumTile = 4096;
+template <typename T>
+__global__ void __launch_bounds__(kAT) k_restrict_long(int32_t nc, int32_t C, const int32_t *__restrict__ off,
+                                                       const int32_t *__restrict__ members, const T *__restrict__ R,
+                                                       int64_t ldr, T *Rc, int64_t ldc) {
+  __shared__ T s_row[kSumTile];
+  const int tid = threadIdx.x;
+  for_long_aggregates(nc, off, kShortSum, [&](int32_t a) {
+    const int b = off[a], e = off[a + 1];
+    for (int c0 = 0; c0 < C; c0 += 64) {
+      const int cw = min(64, C - c0), tile = kSumTile / cw;
+      T s = T(0);
+      for (int i0 = b; i0 < e; i0 += tile) {
+        const int m = min(tile, e - i0) * cw;
+        for (int t = tid; t < m; t += kAT) {
+          const int i = t / cw;
+          s_row[t] = R[(long long)members[i0 + i] * ldr + c0 + (t - i * cw)];
+        }
+        __syncthreads();
+        if (tid < cw) {
+#pragma unroll 8
+          for (int t = tid; t < m; t += cw) s += s_row[t];
+        }
+        __syncthreads();
+      }
+      if (tid < cw) Rc[(long long)a * ldc + c0 + tid] = s;
+    }
+  });
 }
 
 template <typename T>
@@ -364,11 +555,11 @@ int dlp_amg_match(int32_t n, const int32_t *indptr, const int32_t *col, const fl
   DLP_CUDA(cudaMemsetAsync(agg, 0xff, sizeof(int32_t) * (size_t)n, s));
   int launches = 0;
   for (int r = 0; r < rounds; ++r) {
-    k_best_choice<<<g1(n), kAT, 0, s>>>(n, indptr, col, w, matched, 0, choice);
+    k_best_choice<<<g1(8LL * n), kAT, 0, s>>>(n, indptr, col, w, matched, 0, choice);
     k_mutual<<<g1(n), kAT, 0, s>>>(n, choice, matched, agg);
     launches += 2;
   }
-  k_best_choice<<<g1(n), kAT, 0, s>>>(n, indptr, col, w, matched, 1, choice);
+  k_best_choice<<<g1(8LL * n), kAT, 0, s>>>(n, indptr, col, w, matched, 1, choice);
   k_join<<<g1(n), kAT, 0, s>>>(n, choice, agg);
   DLP_CUDA(cudaMemsetAsync(flag, 0, sizeof(int32_t) * (size_t)n, s));
   k_self_and_flag<<<g1(n), kAT, 0, s>>>(n, agg, flag);
@@ -393,8 +584,8 @@ int dlp_amg_members(int32_t n, int32_t nc, const int32_t *agg, int32_t *off, int
   DLP_TRY(exclusive_scan_i32(cnt, nc, off, (char *)ws + vb, ws_bytes - vb, s));
   DLP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(nc > 0 ? nc : 1), s));
   k_fill_members<<<g1(n), kAT, 0, s>>>(n, agg, off, cnt, members);
-  k_sort_members<<<g1(nc), kAT, 0, s>>>(nc, off, members);
-  return check_launch(3);
+  DLP_TRY(check_launch(2));
+  return nc > 0 ? sort_members(n, nc, off, members, s) : DLP_OK;
 }
 
 // Table capacity (slots) for the coarse operator: toff[0..nc] is written; returns the total in
@@ -435,13 +626,17 @@ int dlp_amg_restrict(int32_t nc, int32_t C, const int32_t *off, const int32_t *m
   if (nc == 0) return DLP_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const long long t = (long long)nc * C;
-  if (dtype == DLP_F32)
+  const int gl = std::min(2 * sm_count(), g1(nc));
+  if (dtype == DLP_F32) {
     k_restrict<float><<<g1(t), kAT, 0, s>>>(nc, C, off, members, (const float *)R, ldr, (float *)Rc, ldc);
-  else if (dtype == DLP_F64)
+    k_restrict_long<float><<<gl, kAT, 0, s>>>(nc, C, off, members, (const float *)R, ldr, (float *)Rc, ldc);
+  } else if (dtype == DLP_F64) {
     k_restrict<double><<<g1(t), kAT, 0, s>>>(nc, C, off, members, (const double *)R, ldr, (double *)Rc, ldc);
-  else
+    k_restrict_long<double><<<gl, kAT, 0, s>>>(nc, C, off, members, (const double *)R, ldr, (double *)Rc, ldc);
+  } else {
     return DLP_ERR_DTYPE;
-  return check_launch();
+  }
+  return check_launch(2);
 }
 
 int dlp_amg_prolong_add(int32_t n, int32_t C, const int32_t *agg, const void *Xc, int64_t ldc, void *X, int64_t ldx,

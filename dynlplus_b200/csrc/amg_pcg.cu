@@ -7,13 +7,11 @@
 // CUDA graph can hold. The PCG iteration is
 //   AP = A P; pAp = P.AP; alpha = rz / pAp; Z += alpha P; R -= alpha AP;
 //   stop metric of R (decided on the device); Y = M(R); rz' = R.Y; beta = rz' / rz; P = Y + beta P
-// with the fp64 column reductions of reduce.cu (fixed order). The loop runs as a CUDA graph whose
-// WHILE node repeats the iteration while the decision kernel keeps its flag set; once a stop is
-// proposed the rest of that pass leaves P and rz alone, so a failed confirmation on the true
-// residual resumes exactly as the reference's loop does.
+// with fp64 column reductions (fixed order). The host queues an iteration up to the decision, reads it
+// (about 15 us, while a cycle takes hundreds) and queues the cycle only while the solve runs: no
+// cycle is spent after the stop, and a solve on a new hierarchy captures no graph (some milliseconds per
+// solve before). A failed confirmation on the true residual resumes as the reference's loop does.
 #include <cstring>
-#include <mutex>
-#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -181,8 +179,6 @@ struct GBufs {
   size_t red_bytes;
   char *vc;                                           // the V-cycle's vectors
   const int32_t *cancel;
-  int has_cond;
-  cudaGraphConditionalHandle cond;
 };
 
 constexpr int kGThreads = 256;
@@ -280,14 +276,10 @@ __global__ void __launch_bounds__(kGThreads)
 // The stop decision (one thread), from viol[c] = max_u |R_uc| / diag_u and ss[c] = sum_u R_uc^2:
 //   phase 0 (an iteration): stop proposed when the metric is <= 1, else the patience rule and the
 //   cap; phase 1 (a true residual after a proposal): converged when <= 1, else the run goes on;
-//   phase 2 (the initial residual). Sets the device loop's flag while the solve runs.
+//   phase 2 (the initial residual).
 __global__ void k_gpcg_decide(int phase, int32_t C, GBufs B) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   GCtl *ctl = B.ctl;
-  if (phase == 0 && ctl->done != 0) {
-    if (B.has_cond) cudaGraphSetConditional(B.cond, 0u);
-    return;
-  }
   double mv = 0.0, rel = 0.0;
   bool bad = false;
   for (int c = 0; c < C; ++c) {
@@ -321,7 +313,6 @@ __global__ void k_gpcg_decide(int phase, int32_t C, GBufs B) {
   }
   if (ctl->done == 0 && ctl->iters >= ctl->max_iter) ctl->done = 3;
   if (ctl->done == 0 && read_cancel(B.cancel)) ctl->done = 6;
-  if (phase == 0 && B.has_cond) cudaGraphSetConditional(B.cond, ctl->done == 0 ? 1u : 0u);
 }
 
 }  // namespace dlp
@@ -351,12 +342,10 @@ static int g_grid(int32_t n, int32_t C) {
   return (int)std::max(blocks, 1LL);
 }
 
-// viol[c] = max_u |R_uc| / diag_u, ss[c] = sum_u R_uc^2 (fp64, fixed order)
+// viol[c] = max_u |R_uc| / diag_u, ss[c] = sum_u R_uc^2 (fp64, fixed order) in one pass over R
 static int g_stats(const GProblem &q, const GBufs &B, cudaStream_t s) {
-  DLP_TRY(dlp_colreduce(0, q.n, q.C, q.R, q.ldr, nullptr, q.C, q.diag, q.dtype, nullptr, B.viol, B.red_ws,
-                        B.red_bytes, (dlp_stream_t)s));
-  return dlp_colreduce(2, q.n, q.C, q.R, q.ldr, nullptr, q.C, nullptr, q.dtype, nullptr, B.ss, B.red_ws, B.red_bytes,
-                       (dlp_stream_t)s);
+  return dlp_residual_stats(q.n, q.C, q.R, q.ldr, nullptr, q.C, q.diag, nullptr, 1, q.dtype, B.viol, B.red_ws,
+                            B.red_bytes, (dlp_stream_t)s);
 }
 
 // R = rhs - A Z (the true residual)
@@ -390,7 +379,7 @@ static int g_decide(int phase, const GProblem &q, const GBufs &B, cudaStream_t s
   return check_launch();
 }
 
-// One iteration: AP = A P; pAp; alpha, Z, R; the stop decision; Y = M(R); rz; beta, P.
+// One iteration up to its decision: AP = A P; pAp; alpha, Z, R; the stop decision.
 template <typename T>
 static int g_iteration(const GProblem &q, const GBufs &B, cudaStream_t s) {
   const dlp_stream_t st = (dlp_stream_t)s;
@@ -407,121 +396,19 @@ static int g_iteration(const GProblem &q, const GBufs &B, cudaStream_t s) {
                                                         q.ldp, (const T *)q.AP, q.ldap, B);
   DLP_TRY(check_launch());
   DLP_TRY(g_stats(q, B, s));
-  DLP_TRY(g_decide(0, q, B, s));
-  DLP_TRY(g_precond(q, B, s));
-  return g_dir<T>(0, q, B, s);
+  return g_decide(0, q, B, s);
 }
 
 static int g_iteration_any(const GProblem &q, const GBufs &B, cudaStream_t s) {
   return q.dtype == DLP_F32 ? g_iteration<float>(q, B, s) : g_iteration<double>(q, B, s);
 }
 
-// Cache of the loop graphs, one per problem signature (the level descriptors included).
-struct GKey {
-  std::vector<uintptr_t> v;
-  bool operator==(const GKey &o) const { return v == o.v; }
-};
-struct GKeyHash {
-  size_t operator()(const GKey &k) const {
-    size_t h = 1469598103934665603ull;
-    for (auto x : k.v) h = (h ^ x) * 1099511628211ull;
-    return h;
-  }
-};
-static std::mutex g_gmu;
-static std::unordered_map<GKey, GraphRef, GKeyHash> g_ggraphs;
-static cudaStream_t g_gcapture[64];
-
-static int g_key(const GProblem &q, const GBufs &B, GKey *key) {
-  int dev = 0;
-  DLP_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return DLP_ERR_INVALID;
-  std::vector<uintptr_t> v = {(uintptr_t)dev, (uintptr_t)q.rbeg, (uintptr_t)q.rend, (uintptr_t)q.col,
-                              (uintptr_t)q.w, (uintptr_t)q.n, (uintptr_t)q.C, (uintptr_t)q.diag, (uintptr_t)q.Z,
-                              (uintptr_t)q.ldz, (uintptr_t)q.R, (uintptr_t)q.ldr, (uintptr_t)q.P, (uintptr_t)q.ldp,
-                              (uintptr_t)q.AP, (uintptr_t)q.ldap, (uintptr_t)q.Y, (uintptr_t)q.ldy,
-                              (uintptr_t)q.dtype, (uintptr_t)B.ctl, (uintptr_t)B.cancel, (uintptr_t)q.vc.inv,
-                              (uintptr_t)q.vc.nu, (uintptr_t)q.vc.coarse_sweeps, (uintptr_t)q.vc.nlev,
-                              (uintptr_t)q.w_lo, (uintptr_t)q.P_lo, (uintptr_t)q.ld_lo};
-  uint64_t om;
-  std::memcpy(&om, &q.vc.omega, sizeof(om));
-  v.push_back((uintptr_t)om);
-  v.push_back((uintptr_t)(int64_t)(q.avg_deg * 1024.0));
-  for (int l = 0; l < q.vc.nlev; ++l) {
-    const dlp_amg_level &L = q.vc.lv[l];
-    for (uintptr_t x : {(uintptr_t)L.n, (uintptr_t)L.nnz, (uintptr_t)L.indptr, (uintptr_t)L.col, (uintptr_t)L.w,
-                        (uintptr_t)L.diag, (uintptr_t)L.agg, (uintptr_t)L.off, (uintptr_t)L.members})
-      v.push_back(x);
-  }
-  key->v = std::move(v);
-  return DLP_OK;
-}
-
-static int g_loop_graph(const GProblem &q, const GBufs &B0, GraphRef *out) {
-  GKey key;
-  DLP_TRY(g_key(q, B0, &key));
-  const int dev = (int)key.v[0];
-  std::lock_guard<std::mutex> lk(g_gmu);
-  auto it = g_ggraphs.find(key);
-  if (it != g_ggraphs.end()) {
-    *out = it->second;
-    return DLP_OK;
-  }
-  if (!g_gcapture[dev]) DLP_CUDA(cudaStreamCreateWithFlags(&g_gcapture[dev], cudaStreamNonBlocking));
-  cudaStream_t cs = g_gcapture[dev];
-  cudaGraph_t g = nullptr;
-  DLP_CUDA(cudaGraphCreate(&g, 0));
-  auto fail = [&](cudaError_t e) {
-    cudaGraphDestroy(g);
-    set_cuda_error(e);
-    return DLP_ERR_CUDA;
-  };
-  cudaGraphConditionalHandle h = 0;
-  cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 1u, cudaGraphCondAssignDefault);
-  if (e != cudaSuccess) return fail(e);
-  cudaGraphNodeParams np{};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = h;
-  np.conditional.type = cudaGraphCondTypeWhile;
-  np.conditional.size = 1;
-  cudaGraphNode_t node = nullptr;
-  e = cudaGraphAddNode(&node, g, nullptr, 0, &np);
-  if (e != cudaSuccess) return fail(e);
-  GBufs B = B0;
-  B.has_cond = 1;
-  B.cond = h;
-  e = cudaStreamBeginCaptureToGraph(cs, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                    cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return fail(e);
-  const int st = g_iteration_any(q, B, cs);
-  cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(cs, &captured);
-  if (st != DLP_OK) {
-    cudaGraphDestroy(g);
-    return st;
-  }
-  if (e != cudaSuccess) return fail(e);
-  cudaGraphExec_t ex = nullptr;
-  e = cudaGraphInstantiate(&ex, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    set_cuda_error(e);
-    return DLP_ERR_CUDA;
-  }
-  auto ref = std::make_shared<GraphExec>();
-  ref->ex = ex;
-  if (g_ggraphs.size() >= 16) g_ggraphs.clear();  // holders keep their own references
-  g_ggraphs.emplace(key, ref);
-  *out = ref;
-  return DLP_OK;
-}
-
 static size_t g_ws_layout(const dlp_amg_level *lv, int32_t nlev, int32_t C, int dtype, size_t *off_red,
                           size_t *red_bytes, size_t *off_vc) {
   const size_t cc = (size_t)(C > 0 ? C : 1);
-  size_t b = al256a(sizeof(GCtl)) + 7 * al256a(sizeof(double) * cc);
+  size_t b = al256a(sizeof(GCtl)) + 5 * al256a(sizeof(double) * cc) + al256a(sizeof(double) * (3 * cc + 1));
   *off_red = b;
-  *red_bytes = al256a(dlp_colreduce_workspace_bytes(C));
+  *red_bytes = al256a(std::max(dlp_colreduce_workspace_bytes(C), dlp_residual_stats_workspace_bytes(C)));
   b += *red_bytes;
   *off_vc = b;
   VcPlan p;
@@ -586,11 +473,13 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
   GBufs B{};
   B.ctl = (GCtl *)base;
   size_t o = al256a(sizeof(GCtl));
-  double **vecs[7] = {&B.pAp, &B.rzA, &B.rzB, &B.viol, &B.ss, &B.eps, &B.rhsn};
+  double **vecs[5] = {&B.pAp, &B.rzA, &B.rzB, &B.eps, &B.rhsn};
   for (auto v : vecs) {
     *v = (double *)(base + o);
     o += al256a(sizeof(double) * (size_t)C);
   }
+  B.viol = (double *)(base + o);  // the residual statistics: violations, sums of squares (3 C + 1 values)
+  B.ss = B.viol + C;
   B.red_ws = base + off_red;
   B.red_bytes = red_bytes;
   B.vc = base + off_vc;
@@ -615,10 +504,14 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
     DLP_CUDA(cudaMemcpyAsync(B.eps, e.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
     DLP_CUDA(cudaMemcpyAsync(B.rhsn, e.data() + C, sizeof(double) * C, cudaMemcpyHostToDevice, s));
   }
+  // the decision read back through a pinned word block of this thread (kept for its lifetime)
+  static thread_local GCtl *t_pin = nullptr;
+  if (!t_pin) DLP_CUDA(cudaHostAlloc((void **)&t_pin, sizeof(GCtl), cudaHostAllocPortable));
   GCtl cur{};
   auto read = [&]() -> int {
-    DLP_CUDA(cudaMemcpyAsync(&cur, B.ctl, sizeof(cur), cudaMemcpyDeviceToHost, s));
+    DLP_CUDA(cudaMemcpyAsync(t_pin, B.ctl, sizeof(cur), cudaMemcpyDeviceToHost, s));
     DLP_CUDA(cudaStreamSynchronize(s));
+    cur = *t_pin;
     return DLP_OK;
   };
   // the initial residual and its decision
@@ -631,29 +524,20 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
     DLP_TRY(g_precond(q, B, s));  // Y = M(R), rz = R.Y
     DLP_TRY(g_dir_any(1, q, B, s));  // P = Y
   }
-  GraphRef loop;
-  if (use_graph && cur.done == 0) DLP_TRY(g_loop_graph(q, B, &loop));
+  (void)use_graph;  // the loop is driven by the host either way
   long long guard = 0;
   while (cur.done == 0 && guard++ < (long long)max_iter + 8) {
-    const int it0 = cur.iters;
-    if (loop) {
-      DLP_CUDA(cudaGraphLaunch(loop->ex, s));
-    } else {
-      for (int k = 0; k < 4; ++k) DLP_TRY(g_iteration_any(q, B, s));
-    }
+    DLP_TRY(g_iteration_any(q, B, s));
     DLP_TRY(read());
-    if (loop) note_launches(16ull * (unsigned long long)std::max(cur.iters - it0, 1));
     if (cur.done == 1) {  // a proposed stop: confirmed on the true residual (dynlp/solvers.py:85-89)
       DLP_TRY(g_residual(q, s));
       DLP_TRY(g_stats(q, B, s));
       DLP_TRY(g_decide(1, q, B, s));
       DLP_TRY(read());
-      if (cur.done == 0) {  // not confirmed: resume from the true residual
-        DLP_TRY(g_precond(q, B, s));
-        DLP_TRY(g_dir_any(0, q, B, s));
-      }
-    } else if (cur.done == 0 && cur.iters == it0) {
-      return DLP_ERR_DEVICE;  // a pass ended without a decision
+    }
+    if (cur.done == 0) {  // Y = M(R), rz; P = Y + beta P
+      DLP_TRY(g_precond(q, B, s));
+      DLP_TRY(g_dir_any(0, q, B, s));
     }
   }
   if (iters_out) *iters_out = cur.iters;
@@ -695,11 +579,53 @@ __global__ void k_gj_update(int32_t n, int32_t k, double *A, const double *__res
   }
 }
 
+// The whole elimination in one cooperative launch, the matrix in shared memory: a block holds its rows,
+// and after each pivot the owner of the next pivot row publishes it (two rows in turn), so a pivot costs
+// one grid barrier and one row read instead of two launches and a pass over the matrix through L2. The
+// same operations per element as the two kernels above. Bound by the barrier and the row's division
+// (2.5 us per pivot); n = 1,500: 15 -> 4 ms.
+constexpr int kGjThreads = 512;
+__global__ void __launch_bounds__(kGjThreads, 1) k_gj_whole(int32_t n, int32_t rows, double *A, double *pub, GridBar *bar) {
+  extern __shared__ double sh[];
+  double *M = sh, *row = sh + (size_t)rows * n;  // the block's rows; the scaled pivot row
+  const int tid = threadIdx.x, row0 = blockIdx.x * rows;
+  const int nr = max(0, min(rows, n - row0));
+  uint32_t target = 0;
+  for (int i = tid; i < nr * n; i += kGjThreads) M[i] = A[(long long)row0 * n + i];
+  __syncthreads();
+  if (row0 == 0)
+    for (int j = tid; j < n; j += kGjThreads) __stcg(pub + j, M[j]);
+  if (!grid_barrier(bar, target)) return;
+  for (int k = 0; k < n; ++k) {
+    const double *src = pub + (size_t)(k & 1) * n;
+    double *dst = pub + (size_t)((k + 1) & 1) * n;
+    const double piv = __ldcg(src + k);
+    for (int j = tid; j < n; j += kGjThreads) row[j] = (j == k ? 1.0 : __ldcg(src + j)) / piv;
+    __syncthreads();
+    const int own = k - row0, next = k + 1 - row0;  // this block's row of the pivot, and of the next one
+    const int wid = tid >> 5, lane = tid & 31;
+    for (int i = wid; i < nr; i += kGjThreads / 32) {  // a warp per row: the pivot column's entry first
+      double *m = M + (size_t)i * n;
+      const double f = m[k];
+      __syncwarp();
+      for (int j = lane; j < n; j += 32) {
+        const double v = i == own ? row[j] : (j == k ? 0.0 : m[j]) - f * row[j];
+        m[j] = v;
+        if (i == next) __stcg(dst + j, v);
+      }
+    }
+    if (!grid_barrier(bar, target)) return;
+  }
+  for (int i = tid; i < nr * n; i += kGjThreads) A[(long long)row0 * n + i] = M[i];
+}
+
 }  // namespace dlp
 
 extern "C" {
 
-size_t dlp_dense_spd_inverse_workspace_bytes(int32_t n) { return 2 * al256a(sizeof(double) * (size_t)(n > 0 ? n : 1)); }
+size_t dlp_dense_spd_inverse_workspace_bytes(int32_t n) {
+  return 2 * al256a(sizeof(double) * (size_t)(n > 0 ? n : 1)) + al256a(sizeof(GridBar));
+}
 
 int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_stream_t stream) {
   if (n < 0 || (n > 0 && !A)) return DLP_ERR_INVALID;
@@ -708,6 +634,32 @@ int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_s
   cudaStream_t s = (cudaStream_t)stream;
   double *fcol = (double *)ws;
   double *rowk = (double *)((char *)ws + al256a(sizeof(double) * (size_t)(n > 0 ? n : 1)));
+  if (n == 0) return DLP_OK;
+  {
+    // one launch where the blocks' rows and the pivot row fit shared memory (up to some 1,900 rows)
+    const int rows = (n + sm_count() - 1) / sm_count();
+    const size_t smem = ((size_t)rows + 1) * n * sizeof(double);
+    static const int most = [] {
+      int dev = 0, v = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+      v -= 1024;
+      return cudaFuncSetAttribute((const void *)k_gj_whole, cudaFuncAttributeMaxDynamicSharedMemorySize, v) == cudaSuccess ? v : 0;
+    }();
+    if (smem <= (size_t)most) {
+      GridBar *bar = (GridBar *)((char *)ws + 2 * al256a(sizeof(double) * (size_t)n));
+      DLP_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), s));
+      int32_t nn = n, rr = rows;
+      void *args[] = {(void *)&nn, (void *)&rr, (void *)&A, (void *)&fcol, (void *)&bar};
+      DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_gj_whole, dim3((n + rows - 1) / rows), dim3(kGjThreads), args,
+                                           smem, s));
+      DLP_TRY(check_launch());
+      int32_t lost = 0;  // setup reads back anyway; a wait that ran out must not pass as an inverse
+      DLP_CUDA(cudaMemcpyAsync(&lost, &bar->abort, sizeof(lost), cudaMemcpyDeviceToHost, s));
+      DLP_CUDA(cudaStreamSynchronize(s));
+      return lost ? DLP_ERR_DEVICE : DLP_OK;
+    }
+  }
   const int g1 = ceil_div_i(n, 256);
   const int g2 = ceil_div_i((long long)n * n, 256);
   for (int k = 0; k < n; ++k) {

@@ -176,3 +176,67 @@ def test_wide_class_sum_corrections(K):
         R = solvers.residual(S64, solver.Z[:, :K].contiguous(), S64.rhs.contiguous())
         assert st.relres <= 1e-6 and float((R.norm(dim=0) / S64.rhs.norm(dim=0)).max()) <= 1.01e-6
         assert float((solver.Z[:, :K][S.solved].sum(1) - 1).abs().max()) <= 1e-9
+
+
+@pytest.mark.parametrize("n", [1, 2, 147, 149, 500, 1500, 1900])
+def test_dense_inverse_in_one_launch(n):
+    """The in-place inverse of a diagonally dominant symmetric matrix (the sizes around one row per block,
+    and past what shared memory holds) against numpy; tolerance: n unit roundoffs times the condition
+    number, at most 41 by the dominance margin."""
+    from dynlplus_b200 import _lib
+    from dynlplus_b200.backend import ptr, workspace
+    from dynlplus_b200.backend import stream as cur
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-1, 0, (n, n))
+    A = (A + A.T) / 2
+    np.fill_diagonal(A, 0)
+    A[np.arange(n), np.arange(n)] = np.abs(A).sum(1) * 1.05 + 0.01
+    D = torch.as_tensor(A).cuda()
+    ws = workspace("amg_inverse").get(_lib.lib().dlp_dense_spd_inverse_workspace_bytes(n))
+    _lib.call("dlp_dense_spd_inverse", n, ptr(D), ptr(ws), ws.numel(), cur())
+    want = np.linalg.inv(A)
+    assert np.abs(D.cpu().numpy() - want).max() <= n * 2.3e-16 * 41 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("sizes", [[1, 31, 32, 33], [2, 512, 513, 40], [700, 1, 0, 5]])
+def test_aggregate_members_of_every_length(sizes):
+    """Members of each aggregate in ascending order, at the lengths the three sorts take."""
+    from dynlplus_b200 import amg
+    agg = np.repeat(np.arange(len(sizes)), sizes)
+    agg = agg[np.random.default_rng(0).permutation(agg.size)]
+    off, mem = amg.members(torch.as_tensor(agg.astype(np.int32)).cuda(), len(sizes))
+    off, mem = off.cpu().numpy(), mem.cpu().numpy()
+    for a in range(len(sizes)):
+        assert np.array_equal(mem[off[a]:off[a + 1]], np.flatnonzero(agg == a))
+
+
+@pytest.mark.parametrize("C,dtype", [(1, "float32"), (17, "float32"), (64, "float64"), (70, "float32")])
+def test_restriction_and_coarse_entries_of_long_aggregates(C, dtype):
+    """Sums over aggregates of 1, 64, 65 and 3,000 members, and coarse entries from runs of as many fine
+    ones, against numpy; tolerance: the run's length in unit roundoffs of the working precision."""
+    from dynlplus_b200 import _lib, amg
+    from dynlplus_b200.backend import CSR, code, ptr
+    from dynlplus_b200.backend import stream as cur
+    import scipy.sparse as ssp
+    sizes = [1, 64, 65, 3000, 300]
+    n, nc = sum(sizes), len(sizes)
+    rng = np.random.default_rng(C)
+    agg = np.repeat(np.arange(nc), sizes)[rng.permutation(n)].astype(np.int32)
+    off, mem = amg.members(torch.as_tensor(agg).cuda(), nc)
+    R = rng.uniform(0, 1, (n, C))
+    Rd = torch.as_tensor(R).to(getattr(torch, dtype)).cuda()
+    out = torch.empty((nc, C), dtype=Rd.dtype, device="cuda")
+    _lib.call("dlp_amg_restrict", nc, C, ptr(off), ptr(mem), ptr(Rd), C, ptr(out), C, code(Rd), cur())
+    Rr = Rd.double().cpu().numpy()
+    want = np.stack([Rr[agg == a].sum(0) for a in range(nc)])
+    eps = 2.0 ** -24 if dtype == "float32" else 2.0 ** -53
+    assert (np.abs(out.double().cpu().numpy() - want) <= 3000 * eps * want).all()
+    m = 60_000
+    W = ssp.coo_matrix((rng.uniform(0.5, 1.5, m).astype(np.float32), (rng.integers(0, n, m), rng.integers(0, n, m))),
+                       (n, n)).tocsr()
+    Wc, _ = amg.coarsen(CSR.from_scipy(W), None, torch.as_tensor(agg).cuda(), nc)
+    P = ssp.coo_matrix((np.ones(n), (np.arange(n), agg)), (n, nc)).tocsr()
+    D = np.asarray((P.T @ W.astype(np.float64) @ P).todense())
+    np.fill_diagonal(D, 0)
+    got = np.asarray(Wc.to_scipy().astype(np.float64).todense())
+    assert np.abs(got - D).max() <= 2.0 ** -23 * D.max()
