@@ -26,6 +26,7 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_last_cuda_error": ("", ct.c_int),
     "dlp_sm_count": ("", ct.c_int),
     "dlp_launch_count": ("", ct.c_ulonglong),
+    "dlp_stream_synchronize": ("p", ct.c_int),
     "dlp_set_cancel_word": ("p", ct.c_int),
     "dlp_spmm": ("ppppiipipqipddpqdpqiiidp", ct.c_int),
     "dlp_spmm_lowp": ("ppppiipqpqpddpqidp", ct.c_int),
@@ -50,6 +51,7 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_cc_graph_warm": ("ippppippppzp", ct.c_int),
     "dlp_ground_reach_workspace_bytes": ("i", ct.c_size_t),
     "dlp_ground_reach": ("ippppippppppppzp", ct.c_int),
+    "dlp_ground_reach_async": ("ippppippppppppzp", ct.c_int),
     "dlp_cc_mask_labels_workspace_bytes": ("i", ct.c_size_t),
     "dlp_cc_mask_labels": ("ippppppzp", ct.c_int),
     "dlp_cc_relabel": ("ippppzp", ct.c_int),

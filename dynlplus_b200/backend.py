@@ -54,14 +54,32 @@ def ld(t: torch.Tensor) -> int:
     return t.stride(0)
 
 
-def stream():
-    return torch.cuda.current_stream().cuda_stream
+_HAVE_CUDA = None
+
+
+def have_cuda() -> bool:
+    """torch.cuda.is_available(), asked once (it reads the environment on every call), with torch's
+    CUDA state initialised where it is true."""
+    global _HAVE_CUDA
+    if _HAVE_CUDA is None:
+        _HAVE_CUDA = torch.cuda.is_available()
+        if _HAVE_CUDA:
+            torch.cuda.init()
+    return _HAVE_CUDA
+
+
+def stream() -> int:
+    """The current stream's handle on the current device, without building a Stream object (some 5 us
+    each, 35 of them in one edge batch and its solve)."""
+    if not have_cuda():
+        return torch.cuda.current_stream().cuda_stream  # raises torch's own error
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def sync():
     """Wait for the current stream (not the whole device: another thread may be capturing a CUDA
     graph on its own stream, and a device-wide synchronisation would invalidate that capture)."""
-    torch.cuda.current_stream().synchronize()
+    _lib.call("dlp_stream_synchronize", stream())
 
 
 def mem_used_gb() -> float:
@@ -76,13 +94,13 @@ class Timer:
         self.ms = 0.0
 
     def __enter__(self):
-        if torch.cuda.is_available():
+        if have_cuda():
             sync()
         self._t = time.perf_counter()
         return self
 
     def __exit__(self, *exc):
-        if torch.cuda.is_available():
+        if have_cuda():
             sync()
         self.ms += (time.perf_counter() - self._t) * 1e3
 
@@ -106,8 +124,7 @@ _WS: dict = {}
 def workspace(tag: str = "default") -> Workspace:
     """Scratch buffer per (tag, device, current stream): work on different streams (the serving
     loop's workers) never shares a buffer."""
-    key = (tag, torch.cuda.current_device() if torch.cuda.is_available() else -1,
-           torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else 0)
+    key = (tag, torch._C._cuda_getDevice(), stream()) if have_cuda() else (tag, -1, 0)
     if key not in _WS:
         _WS[key] = Workspace()
     return _WS[key]

@@ -224,50 +224,100 @@ __global__ void k_cc_gather_rank(const int32_t *__restrict__ parent, int32_t n, 
 // Marks are read and written in place, so one sweep carries a mark along many hops; a sweep that
 // marks nothing ends it (the reached set is then closed under adjacency, i.e. whole components).
 // ------------------------------------------------------------------------------------------------
+// The whole grounding in one cooperative launch: bottom-up sweeps until one reaches nothing new (at most
+// kReachMaxSweeps), the union-find over every live edge where they do not settle (long chains), and the
+// membership update, with a grid barrier where a launch boundary or a host read was. A settled graph takes
+// four sweeps; launch by launch, each batch of sweeps ended in a host read in the middle of the patch.
+// Bound by the first sweep's row scans (n = 1M, degree 10: 114 us of 160); at n = 3,000 by the barriers
+// (four launches, the read and two clears, 90 us of host time -> one launch of 15 us).
+// info: [0] vertices of vmask or sink, [1] vertices of vmask left ungrounded, [2] sweeps run (negative:
+// the union-find finished), [3] a barrier's wait ran out.
+constexpr int kGroundThreads = 1024;
+constexpr int kReachMaxSweeps = 32;  // then the union-find finishes the job
 template <typename TW>
-__global__ void __launch_bounds__(kCcThreads)
-    k_reach_sweep(int32_t n, const int32_t *__restrict__ rbeg, const int32_t *__restrict__ rend,
-                  const int32_t *__restrict__ col, const TW *__restrict__ w, const uint8_t *__restrict__ vmask,
-                  const uint8_t *__restrict__ sink, uint8_t *reached_, int32_t *flag, int32_t *err) {
-  volatile uint8_t *reached = reached_;
-  bool any = false;
-  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < n;
-       u += (long long)gridDim.x * blockDim.x) {
-    if ((vmask && !vmask[u]) || reached[u]) continue;
-    const int end = rend[u];
-    for (int j = rbeg[u]; j < end; ++j) {
-      if (!live(w, j)) continue;
-      const int32_t v = col[j];
-      if ((unsigned)v >= (unsigned)n) {
-        if (err) atomicExch(err, DLP_ERR_DEVICE);
-        continue;
-      }
-      const bool inm = !vmask || vmask[v];
-      if (inm ? reached[v] != 0 : (sink && sink[v])) {
-        reached[u] = 1;
-        any = true;
-        break;
+__global__ void __launch_bounds__(kGroundThreads, 2)
+    k_ground_whole(int32_t n, const int32_t *__restrict__ rbeg, const int32_t *__restrict__ rend,
+                   const int32_t *__restrict__ col, const TW *__restrict__ w, const uint8_t *__restrict__ vmask,
+                   const uint8_t *__restrict__ sink, volatile uint8_t *reached, int32_t *flags, int32_t *parent,
+                   uint8_t *umask, uint8_t *in_t, int32_t *count, int32_t *err, int32_t *info, GridBar *bar) {
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  const bool first = t0 == 0;
+  uint32_t target = 0;
+  int sweeps = 0;
+  bool settled = false;
+  while (!settled && sweeps < kReachMaxSweeps) {  // flags and reached were cleared before the launch
+    bool any = false;
+    for (long long u = t0; u < n; u += step) {
+      if ((vmask && !vmask[u]) || reached[u]) continue;
+      const int end = rend[u];
+      for (int j = rbeg[u]; j < end; ++j) {
+        if (!live(w, j)) continue;
+        const int32_t v = col[j];
+        if ((unsigned)v >= (unsigned)n) {
+          if (err) atomicExch(err, DLP_ERR_DEVICE);
+          continue;
+        }
+        const bool inm = !vmask || vmask[v];
+        if (inm ? reached[v] != 0 : (sink && sink[v])) {
+          reached[u] = 1;
+          any = true;
+          break;
+        }
       }
     }
+    if (__syncthreads_or(any) && threadIdx.x == 0) atomicAdd(flags + sweeps, 1);
+    if (!grid_barrier(bar, target)) {
+      if (first) info[3] = 1;
+      return;
+    }
+    settled = __ldcg(flags + sweeps) == 0;
+    ++sweeps;
   }
-  if (__any_sync(0xffffffffu, any) && lane_id() == 0) atomicAdd(flag, 1);
-}
-
-// umask[v] = reached[v] (or root(v) == root(sink) when parent is given); in_t[v] = membership
-// changed; *count += |changed|
-__global__ void k_ground_apply(int32_t n, const uint8_t *__restrict__ reached, const int32_t *__restrict__ parent,
-                               const uint8_t *__restrict__ vmask, uint8_t *umask, uint8_t *in_t, int32_t *count) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool ch = false;
-  if (v < n) {
-    const bool nu = parent ? ((!vmask || vmask[v]) && parent[v] == parent[n]) : reached[v] != 0;
-    const bool ou = umask[v] != 0;
-    ch = nu != ou;
+  if (!settled) {
+    for (long long v = t0; v <= n; v += step) parent[v] = (int32_t)v;
+    if (!grid_barrier(bar, target)) {
+      if (first) info[3] = 1;
+      return;
+    }
+    for (long long u = t0; u < n; u += step) {
+      if (vmask && !vmask[u]) continue;
+      for (int j = rbeg[u]; j < rend[u]; ++j) {
+        if (!live(w, j)) continue;
+        const int32_t v = col[j];
+        if ((unsigned)v >= (unsigned)n) continue;  // flagged by the sweeps
+        if (!vmask || vmask[v]) unite(parent, (int32_t)u, v, err);
+        else if (sink && sink[v]) unite(parent, (int32_t)u, n, err);
+      }
+    }
+    if (!grid_barrier(bar, target)) {
+      if (first) info[3] = 1;
+      return;
+    }
+  }
+  const int32_t root = settled ? 0 : find_root(parent, n, err);
+  int changes = 0, active = 0, lost = 0;
+  for (long long v = t0; v < n; v += step) {
+    const bool m = !vmask || vmask[v];
+    const bool nu = m && (settled ? reached[v] != 0 : find_root(parent, (int32_t)v, err) == root);
+    const bool ch = nu != (umask[v] != 0);
     umask[v] = nu ? 1 : 0;
     in_t[v] = ch ? 1 : 0;
+    changes += ch;
+    active += (m ? 1 : 0) + (sink && sink[v] ? 1 : 0);
+    lost += m && !nu;
   }
-  const unsigned b = __ballot_sync(0xffffffffu, ch);
-  if ((threadIdx.x & 31) == 0 && b) atomicAdd(count, __popc(b));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    changes += __shfl_xor_sync(0xffffffffu, changes, off);
+    active += __shfl_xor_sync(0xffffffffu, active, off);
+    lost += __shfl_xor_sync(0xffffffffu, lost, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (changes) atomicAdd(count, changes);
+    if (active) atomicAdd(info, active);
+    if (lost) atomicAdd(info + 1, lost);
+  }
+  if (first) info[2] = settled ? sweeps : -sweeps;
 }
 
 // label[lpos[v]] = rank[parent[v]] for every masked v: the rank of its component's minimum id,
@@ -474,8 +524,6 @@ static size_t warm_ws_layout(int32_t n, size_t *off_bits, size_t *off_f0, size_t
   return b + (nn * 4 + 255) / 256 * 256;
 }
 
-constexpr int kReachBatch = 4;      // sweeps between host checks
-constexpr int kReachMaxSweeps = 32; // then the union-find finishes the job
 
 static size_t reach_ws_layout(int32_t n, size_t *off_flags, size_t *off_parent, size_t *off_cc) {
   size_t b = ((size_t)n + 255) / 256 * 256;  // reached
@@ -484,7 +532,7 @@ static size_t reach_ws_layout(int32_t n, size_t *off_flags, size_t *off_parent, 
   *off_parent = b;
   b += ((size_t)n + 1 + 63) / 64 * 256;      // parent of the fallback (n + 1 ints)
   *off_cc = b;
-  return b + 256;                            // dlp_cc_graph workspace
+  return b + 256;                            // dlp_ground_reach's info words
 }
 
 size_t dlp_cc_graph_warm_workspace_bytes(int32_t n) {
@@ -541,58 +589,58 @@ size_t dlp_ground_reach_workspace_bytes(int32_t n) {
   return reach_ws_layout(n < 0 ? 0 : n, &a, &b, &c);
 }
 
+int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w,
+                           int w_dtype, const uint8_t *vmask, const uint8_t *sink, uint8_t *umask, uint8_t *in_t,
+                           int32_t *count, int32_t *err, int32_t *info, void *ws, size_t ws_bytes,
+                           dlp_stream_t stream) {
+  if (n < 0 || !info || (n > 0 && (!rbeg || !rend || !col || !umask || !in_t || !count))) return DLP_ERR_INVALID;
+  if (w && w_dtype != DLP_F32 && w_dtype != DLP_F64 && w_dtype != DLP_BF16) return DLP_ERR_DTYPE;
+  size_t off_flags, off_parent, off_cc;
+  if (!ws || ws_bytes < reach_ws_layout(n, &off_flags, &off_parent, &off_cc)) return DLP_ERR_WORKSPACE;
+  cudaStream_t s = (cudaStream_t)stream;
+  DLP_CUDA(cudaMemsetAsync(info, 0, 4 * sizeof(int32_t), s));
+  if (n == 0) return DLP_OK;
+  char *base = (char *)ws;
+  uint8_t *reached = (uint8_t *)base;
+  int32_t *flags = (int32_t *)(base + off_flags);
+  int32_t *parent = (int32_t *)(base + off_parent);
+  GridBar *bar = (GridBar *)(flags + kReachMaxSweeps);  // in the flags' 256 bytes
+  static_assert(kReachMaxSweeps * sizeof(int32_t) + sizeof(GridBar) <= 256, "flags and barrier share a line of 256 bytes");
+  DLP_CUDA(cudaMemsetAsync(reached, 0, off_flags + 256, s));  // reached, the flags and the barrier
+  auto launch = [&](auto kern, auto *wp) -> int {
+    static const int per = [&] {
+      int k = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kGroundThreads, 0) != cudaSuccess) (void)cudaGetLastError();
+      return k;
+    }();
+    if (per < 1) return DLP_ERR_CUDA;
+    const int grid = std::max(1, std::min(ceil_div_i(n, kGroundThreads), sm_count() * per));
+    void *args[] = {(void *)&n,     (void *)&rbeg,  (void *)&rend,   (void *)&col,   (void *)&wp,   (void *)&vmask,
+                    (void *)&sink,  (void *)&reached, (void *)&flags, (void *)&parent, (void *)&umask, (void *)&in_t,
+                    (void *)&count, (void *)&err,   (void *)&info,   (void *)&bar};
+    DLP_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kGroundThreads), args, 0, s));
+    return check_launch();
+  };
+  if (!w || w_dtype == DLP_F32) return launch(k_ground_whole<float>, (const float *)w);
+  if (w_dtype == DLP_F64) return launch(k_ground_whole<double>, (const double *)w);
+  return launch(k_ground_whole<bf16>, (const bf16 *)w);
+}
+
 int dlp_ground_reach(int32_t n, const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w,
                      int w_dtype, const uint8_t *vmask, const uint8_t *sink, uint8_t *umask, uint8_t *in_t,
                      int32_t *count, int32_t *err, int32_t *sweeps_out, void *ws, size_t ws_bytes,
                      dlp_stream_t stream) {
-  if (n < 0 || (n > 0 && (!rbeg || !rend || !col || !umask || !in_t || !count))) return DLP_ERR_INVALID;
-  if (w && w_dtype != DLP_F32 && w_dtype != DLP_F64 && w_dtype != DLP_BF16) return DLP_ERR_DTYPE;
-  size_t off_flags, off_parent, off_cc;
-  if (!ws || ws_bytes < reach_ws_layout(n, &off_flags, &off_parent, &off_cc)) return DLP_ERR_WORKSPACE;
   if (sweeps_out) *sweeps_out = 0;
-  if (n == 0) return DLP_OK;
-  cudaStream_t s = (cudaStream_t)stream;
-  char *base = (char *)ws;
-  uint8_t *reached = (uint8_t *)base;
-  int32_t *flags = (int32_t *)(base + off_flags);
-  DLP_CUDA(cudaMemsetAsync(reached, 0, (size_t)n, s));
-  DLP_CUDA(cudaMemsetAsync(flags, 0, sizeof(int32_t) * kReachMaxSweeps, s));
-  const int grid = grid_persist(n);
-  int done = 0;
-  bool converged = false;
-  while (!converged && done < kReachMaxSweeps) {
-    for (int k = 0; k < kReachBatch; ++k, ++done) {
-      if (!w || w_dtype == DLP_F32)
-        k_reach_sweep<float><<<grid, kCcThreads, 0, s>>>(n, rbeg, rend, col, (const float *)w, vmask, sink, reached,
-                                                          flags + done, err);
-      else if (w_dtype == DLP_F64)
-        k_reach_sweep<double><<<grid, kCcThreads, 0, s>>>(n, rbeg, rend, col, (const double *)w, vmask, sink,
-                                                           reached, flags + done, err);
-      else
-        k_reach_sweep<bf16><<<grid, kCcThreads, 0, s>>>(n, rbeg, rend, col, (const bf16 *)w, vmask, sink, reached,
-                                                         flags + done, err);
-    }
-    DLP_TRY(check_launch(kReachBatch));
-    int32_t h[kReachBatch];
-    DLP_CUDA(cudaMemcpyAsync(h, flags + done - kReachBatch, sizeof(h), cudaMemcpyDeviceToHost, s));
-    DLP_CUDA(cudaStreamSynchronize(s));
-    for (int k = 0; k < kReachBatch; ++k) {
-      if (h[k] == 0) {
-        converged = true;
-        if (sweeps_out) *sweeps_out = done - kReachBatch + k + 1;
-        break;
-      }
-    }
-  }
-  const int32_t *parent = nullptr;
-  if (!converged) {  // long chains: the union-find settles the rest exactly
-    int32_t *par = (int32_t *)(base + off_parent);
-    DLP_TRY(dlp_cc_graph(n, rbeg, rend, col, w, w_dtype, vmask, sink, par, err, base + off_cc, 256, stream));
-    parent = par;
-    if (sweeps_out) *sweeps_out = -done;
-  }
-  k_ground_apply<<<ceil_div_i(n, 256), 256, 0, s>>>(n, reached, parent, vmask, umask, in_t, count);
-  return check_launch();
+  size_t off_flags, off_parent, off_cc;
+  if (n >= 0 && (!ws || ws_bytes < reach_ws_layout(n, &off_flags, &off_parent, &off_cc))) return DLP_ERR_WORKSPACE;
+  int32_t *info = n >= 0 ? (int32_t *)((char *)ws + off_cc) : nullptr;
+  DLP_TRY(dlp_ground_reach_async(n, rbeg, rend, col, w, w_dtype, vmask, sink, umask, in_t, count, err, info, ws,
+                                 ws_bytes, stream));
+  int32_t h[4] = {0, 0, 0, 0};
+  DLP_CUDA(cudaMemcpyAsync(h, info, sizeof(h), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  DLP_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  if (sweeps_out) *sweeps_out = h[2];
+  return h[3] ? DLP_ERR_DEVICE : DLP_OK;
 }
 
 size_t dlp_cc_mask_labels_workspace_bytes(int32_t n) {

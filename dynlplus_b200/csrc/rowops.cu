@@ -566,6 +566,11 @@ unsigned long long dlp_launch_count(void) { return g_launches.load(); }
 
 int dlp_sm_count(void) { return sm_count(); }
 
+int dlp_stream_synchronize(dlp_stream_t stream) {
+  DLP_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  return DLP_OK;
+}
+
 int dlp_set_cancel_word(const int32_t *word) {
   g_cancel.store(word, std::memory_order_release);
   return DLP_OK;

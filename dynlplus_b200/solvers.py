@@ -19,7 +19,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib, kernels
-from .backend import Timer, code, ld, ptr, stream, workspace
+from .backend import Timer, code, ld, ptr, stream, sync, workspace
 from .kernels import FrontierOps
 from .stream import System
 
@@ -67,7 +67,7 @@ def _read_host(x):
     if h is None or h.numel() < x.numel():
         h = bufs[key] = torch.empty(max(x.numel(), 64), dtype=x.dtype, pin_memory=True)
     h[: x.numel()].copy_(x.reshape(-1), non_blocking=True)
-    torch.cuda.current_stream(x.device).synchronize()
+    sync()
     return h[: x.numel()].tolist()
 
 
@@ -78,7 +78,7 @@ def _scratch(tag, n, C, dt, dev, padded=False):
     systems of every size) reuse one allocation instead of keeping one per size. Its contents are
     whatever the last user of the key left."""
     dev = torch.device(dev)
-    sid = torch.cuda.current_stream().cuda_stream if dev.type == "cuda" else 0  # per stream, like workspaces
+    sid = stream() if dev.type == "cuda" else 0  # per stream, like workspaces
     key = (tag, C, dt, dev, sid, padded)
     buf = _SCRATCH.get(key)
     if buf is None or buf.shape[0] < n:

@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib, cc, kernels
-from .backend import CSR, code, ld, ptr, stream, to_dtype, workspace
+from .backend import CSR, code, ld, ptr, stream, sync, to_dtype, workspace
 from .graphs import Dataset, csr_rows
 
 
@@ -339,7 +339,7 @@ class EdgeStream:
         self.in_t = torch.zeros(n, dtype=torch.uint8, device=dev)
         self.changed = torch.zeros(n, dtype=torch.uint8, device=dev)
         self._squeeze = torch.zeros(n, dtype=torch.uint8, device=dev)  # rows to squeeze after deletions
-        self._stat = torch.zeros(8, dtype=torch.int32, device=dev)
+        self._stat = torch.zeros(12, dtype=torch.int32, device=dev)
         self.counters = {"rebuilds": 0, "ground_changes": 0, "applied": 0, "ground_sweeps": 0, "ground_fallbacks": 0}
         self._ground()
         sr = self.G.slot_rows()
@@ -463,14 +463,16 @@ class EdgeStream:
         if not keep_pending:
             self.changed.zero_()
         self._stat.zero_()
-        st = self._stat  # [error, overflow, deleted, inserted, ground changes, ground error, changed rows, -]
+        # [error, overflow, deleted, inserted, ground changes, ground error, changed rows, moved rows,
+        #  active vertices, ungrounded vertices, ground sweeps, ground wait lost]
+        st = self._stat
         s = stream()
         if nd:
             _lib.call("dlp_graph_delete", n, ptr(G.rbeg), ptr(G.rend), ptr(G.indices), ptr(G.aw), ptr(G.data), ptr(du),
                       ptr(dv), nd, ptr(self.umask), ptr(self.labeled), ptr(self.y), self.K, ptr(self.rowsum),
                       ptr(self.B), ptr(self.changed), ptr(st[2:3]), ptr(st[0:1]), ptr(self._squeeze), s)
         # Everything below is queued in dependency order before one host read of every flag and
-        # count: the insertion, the grounding (its sweeps synchronise internally), the membership
+        # count: the insertion, the grounding, the membership
         # toggle of the rows it flagged, the changed rows and the solver CSR. An overflow (rare)
         # undoes the toggle, repacks and redoes the rest.
         for attempt in range(4):
@@ -483,7 +485,6 @@ class EdgeStream:
             mv, _ = kernels.flatnonzero(self.in_t, count=st[7:8], sync=False)
             Qb, _ = kernels.flatnonzero(self.changed, count=st[6:7], sync=False)
             self._csr_launch()
-            self._queue_counts()
             flags = self._read_counts()
             if flags["overflow"] == 0:
                 break
@@ -495,16 +496,18 @@ class EdgeStream:
             G.rebuild()  # a row ran out of slack: repack with more and apply the insertions again
             self.counters["rebuilds"] += 1
             st[1].zero_()
-            st[3:8].zero_()  # counts the next attempt makes again
+            st[3:].zero_()  # counts the next attempt makes again
         else:
             raise RuntimeError("edge insertion kept overflowing after repacking")
         if flags["error"]:
             raise ValueError(f"edge batch rejected: {_lib.STATUS.get(flags['error'])} (vertex id out of range?)")
         if flags["ground_error"]:
             raise ValueError("grounding: entry column outside [0, n)")
+        if flags["ground_lost"]:
+            raise _lib.DLPError("dlp_ground_reach_async", 8)
         nmoved = flags["moved"]
-        self.counters["ground_sweeps"] += abs(self._sweeps.value)
-        self.counters["ground_fallbacks"] += self._sweeps.value < 0
+        self.counters["ground_sweeps"] += abs(flags["sweeps"])
+        self.counters["ground_fallbacks"] += flags["sweeps"] < 0
         moved = mv[:nmoved]
         if nmoved:
             self.counters["ground_changes"] += nmoved
@@ -532,14 +535,13 @@ class EdgeStream:
     def _ground_launch(self):
         """The grounding check (reachability from the labelled vertices through unlabelled ones,
         dynlp/stream.py:150-159): umask and in_t updated, the number of membership changes counted
-        into the batch's stat word 4 (its sweeps synchronise the stream internally)."""
-        import ctypes as ct
-        G, n, st = self.G, self.n, self._stat
-        self._sweeps = ct.c_int32(0)
+        into the batch's stat word 4, the batch's active and ungrounded vertices, the sweeps and a lost
+        wait into words 8 to 11 (no host read)."""
+        G, n, base = self.G, self.n, ptr(self._stat)
         ws = workspace("ground_reach").get(_lib.lib().dlp_ground_reach_workspace_bytes(n))
-        _lib.call("dlp_ground_reach", n, ptr(G.rbeg), ptr(G.rend), ptr(G.indices), ptr(G.aw), code(G.aw),
-                  ptr(self.vmask), ptr(self.labeled), ptr(self.umask), ptr(self.in_t), ptr(st[4:5]), ptr(st[5:6]),
-                  ct.addressof(self._sweeps), ptr(ws), ws.numel(), stream())
+        _lib.call("dlp_ground_reach_async", n, ptr(G.rbeg), ptr(G.rend), ptr(G.indices), ptr(G.aw), code(G.aw),
+                  ptr(self.vmask), ptr(self.labeled), ptr(self.umask), ptr(self.in_t), base + 16, base + 20, base + 32,
+                  ptr(ws), ws.numel(), stream())
 
     def _toggle_flagged(self):
         """Membership change of every row the grounding flagged in in_t (dlp_graph_toggle without a
@@ -548,34 +550,18 @@ class EdgeStream:
         _lib.call("dlp_graph_toggle", ptr(G.rbeg), ptr(G.rend), ptr(G.indices), ptr(G.aw), ptr(G.data), None, self.n,
                   ptr(self.in_t), ptr(self.umask), ptr(self.rowsum), ptr(self.changed), stream())
 
-    def _queue_counts(self):
-        """Queue the active and ungrounded vertex counts of the batch's final membership on the
-        device (no host read: they come back with the batch's flags in _read_counts)."""
-        um = self.umask.view(torch.bool)
-        if getattr(self, "_cnt_dev", None) is None:
-            self._cnt_dev = torch.zeros(2, dtype=torch.int64, device=self.dev)
-        self._cnt_dev[0] = self.vmask.sum() + self.labeled.sum()
-        self._cnt_dev[1] = (self.vmask.view(torch.bool) & ~um).sum()
-
     def _read_counts(self):
-        """One host read of the batch's flags and counts (the solver CSR's entry count, and the
-        active and ungrounded counts when queued)."""
+        """One host read of the batch's flags and counts and the solver CSR's entry count."""
         if getattr(self, "_h_stat", None) is None:
-            self._h_stat = torch.zeros(9, dtype=torch.int32, pin_memory=torch.cuda.is_available())
-            self._h_cnt = torch.zeros(2, dtype=torch.int64, pin_memory=torch.cuda.is_available())
+            self._h_stat = torch.zeros(13, dtype=torch.int32, pin_memory=torch.cuda.is_available())
         h = self._h_stat
-        h[0:8].copy_(self._stat, non_blocking=True)
-        h[8:9].copy_(self._csr_ptr[self.n:self.n + 1], non_blocking=True)
-        cnt = getattr(self, "_cnt_dev", None)
-        if cnt is not None:
-            self._h_cnt.copy_(cnt, non_blocking=True)
-        torch.cuda.current_stream(self.dev).synchronize()
+        h[0:12].copy_(self._stat, non_blocking=True)
+        h[12:13].copy_(self._csr_ptr[self.n:self.n + 1], non_blocking=True)
+        sync()
         v = h.tolist()
-        out = {"error": v[0], "overflow": v[1], "deleted": v[2], "inserted": v[3], "moved": v[7],
-               "ground_error": v[5], "changed": v[6], "nnz": v[8]}
-        if cnt is not None:
-            out["active"], out["ungrounded"] = self._h_cnt.tolist()
-        return out
+        return {"error": v[0], "overflow": v[1], "deleted": v[2], "inserted": v[3], "moved": v[7],
+                "ground_error": v[5], "changed": v[6], "active": v[8], "ungrounded": v[9], "sweeps": v[10],
+                "ground_lost": v[11], "nnz": v[12]}
 
     def apply_vertices(self, ins, dele, tau=None, wmax=None) -> System:
         """One vertex-arrival batch (IncrementalStream.batches, dynlp/stream.py:300-346): the

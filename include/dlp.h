@@ -55,6 +55,9 @@ int dlp_sm_count(void);
 /* kernels this library has launched in the process so far (graph replays count their kernels) */
 unsigned long long dlp_launch_count(void);
 
+/* Waits for the stream's work (a host wait that releases the caller's interpreter lock). */
+int dlp_stream_synchronize(dlp_stream_t stream);
+
 /* Cancellation of the device-side loops (no reference counterpart: the reference has no way to stop
  * a solve). `word` points at an int32 the device can read: device memory, or pinned host memory
  * (cudaHostAlloc / cudaMallocHost, usable on the device under unified addressing). While it holds a
@@ -216,15 +219,22 @@ int dlp_cc_graph_warm(int32_t n, const int32_t *rbeg, const int32_t *rend, const
  * holds the previous grounded set; on exit umask[u] = 1 iff vmask[u] and u's component in the
  * graph form of dlp_cc_graph (same arguments, same symmetric row ranges) reaches the sink, i.e.
  * exactly the vertices with parent[u] == parent[n] there; in_t[u] = 1 where membership changed;
- * *count (device int, caller-zeroed) += number of changes. Bottom-up reachability sweeps, checked
- * on the host every few sweeps; when they have not settled after 32, dlp_cc_graph finishes the
- * job (same result). *sweeps_out (host, may be NULL) = sweeps run, negated if the fallback ran.
- * Workspace: dlp_ground_reach_workspace_bytes(n). Synchronises the stream. */
+ * *count (device int, caller-zeroed) += number of changes. Bottom-up reachability sweeps in one
+ * cooperative launch; when they have not settled after 32, a union-find over the live entries finishes
+ * the job there (same result). *sweeps_out (host, may be NULL) = sweeps run, negated if the fallback ran.
+ * Workspace: dlp_ground_reach_workspace_bytes(n). Synchronises the stream; the _async form does not and
+ * leaves in info (device, four ints): the vertices of vmask or sink, the vertices of vmask left
+ * ungrounded, the sweeps (negated as above), and non-zero if a wait on the device ran out (the result is
+ * then unusable). */
 size_t dlp_ground_reach_workspace_bytes(int32_t n);
 int dlp_ground_reach(int32_t n, const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w,
                      int w_dtype, const uint8_t *vmask, const uint8_t *sink, uint8_t *umask, uint8_t *in_t,
                      int32_t *count, int32_t *err, int32_t *sweeps_out, void *ws, size_t ws_bytes,
                      dlp_stream_t stream);
+int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w,
+                           int w_dtype, const uint8_t *vmask, const uint8_t *sink, uint8_t *umask, uint8_t *in_t,
+                           int32_t *count, int32_t *err, int32_t *info, void *ws, size_t ws_bytes,
+                           dlp_stream_t stream);
 
 /* The reference's component labels of the masked vertices: connected_components over the
  * subgraph that vmask induces, numbered as dynlp/stream.py:150-153 with dynlp/cc.py:22 number them

@@ -240,3 +240,58 @@ def test_restriction_and_coarse_entries_of_long_aggregates(C, dtype):
     np.fill_diagonal(D, 0)
     got = np.asarray(Wc.to_scipy().astype(np.float64).todense())
     assert np.abs(got - D).max() <= 2.0 ** -23 * D.max()
+
+
+@pytest.mark.parametrize("kind,n", [("random", 1), ("random", 1023), ("random", 1025), ("random", 60_000), ("path", 5000),
+                                    ("path", 20)])
+def test_grounding_in_one_launch(kind, n):
+    """The grounded set, its changes and counts against SciPy's components: random graphs (sweeps settle),
+    and a path longer than 32 sweeps may cover (the union-find in the same launch)."""
+    import scipy.sparse as ssp
+    from scipy.sparse.csgraph import connected_components
+    from dynlplus_b200 import _lib, cc
+    from dynlplus_b200.backend import CSR, code, ptr, workspace
+    from dynlplus_b200.backend import stream as cur
+    rng = np.random.default_rng(n)
+    if kind == "path":
+        order = rng.permutation(n)
+        u, v = order[:-1], order[1:]
+    else:
+        m = int(0.9 * n)
+        u, v = rng.integers(0, n, m), rng.integers(0, n, m)
+    A = ssp.coo_matrix((np.ones(len(u), np.float32), (u, v)), (n, n)).tocsr()
+    A = ((A + A.T) > 0).astype(np.float32).tocsr()
+    A.setdiag(0)
+    A.eliminate_zeros()
+    dead = rng.random(A.nnz) < (0.0 if kind == "path" else 0.1)  # dead entries, both directions
+    C = A.tocoo()
+    key = np.minimum(C.row, C.col).astype(np.int64) * n + np.maximum(C.row, C.col)
+    dead = np.isin(key, key[dead])
+    sink = np.zeros(n, np.uint8)
+    sink[(order[:1] if kind == "path" else rng.integers(0, n, max(1, n // 50)))] = 1
+    vmask = (1 - sink).astype(np.uint8)
+    if n > 100:
+        vmask[rng.integers(0, n, n // 20)] = 0  # neither masked nor sink
+    Wd = CSR.from_scipy(A)
+    if not A.nnz:
+        Wd = CSR(torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), Wd.indptr, Wd.shape)
+    else:
+        Wd.data[torch.as_tensor(dead).cuda()] = 0
+    old = (rng.random(n) < 0.5).astype(np.uint8)
+    T = lambda x: torch.as_tensor(x.copy()).cuda()  # noqa: E731
+    um, it = T(old), torch.zeros(n, dtype=torch.uint8, device="cuda")
+    ce, info = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.full((4,), 7, dtype=torch.int32, device="cuda")
+    ws = workspace("ground_reach").get(_lib.lib().dlp_ground_reach_workspace_bytes(n))
+    vm, sk = T(vmask), T(sink)
+    _lib.call("dlp_ground_reach_async", n, ptr(Wd.rbeg), ptr(Wd.rend), ptr(Wd.indices), ptr(Wd.data), code(Wd.data),
+              ptr(vm), ptr(sk), ptr(um), ptr(it), ptr(ce[:1]), ptr(ce[1:]), ptr(info), ptr(ws), ws.numel(), cur())
+    live = A.tocoo()
+    keep = ~dead & (vmask[live.row] > 0) & ((vmask[live.col] > 0) | (sink[live.col] > 0))
+    r, c = live.row[keep], np.where(vmask[live.col[keep]] > 0, live.col[keep], n)
+    _, lab = connected_components(ssp.coo_matrix((np.ones(len(r)), (r, c)), (n + 1, n + 1)), directed=False)
+    want = ((vmask > 0) & (lab[:n] == lab[n])).astype(np.uint8)
+    assert np.array_equal(um.cpu().numpy(), want)
+    assert np.array_equal(it.cpu().numpy(), (want != old).astype(np.uint8))
+    active, lost, sweeps, bad = info.tolist()
+    assert (active, lost, bad) == (int(vmask.sum() + sink.sum()), int((vmask > want).sum()), 0)
+    assert ce.tolist() == [int((want != old).sum()), 0] and 1 <= abs(sweeps) <= 32
