@@ -8,7 +8,8 @@
 // dependent loads (row range, column, score) and the two barriers, no bandwidth; the host loop it
 // replaces spent some 20 launches and three host reads per round on the same work.
 // Measured on B200 (vertex arrivals, n = 20,000, degree 10, one column, five batches of some 350
-// rounds each): see the figures at k_frontier_rounds.
+// rounds each): host loop 411 ms; lists 33 ms of kernel time (18.6 us a round); without lists, below
+// kFrDenseRows rows, 10 ms.
 #include "gather.cuh"
 
 namespace dlp {
@@ -157,6 +158,180 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
   }
 }
 
+// The same rounds for systems small enough that looking at every row's mark is cheaper than keeping lists:
+// a lane group owns its rows, X is kept in two buffers that the rounds read and write in turn (so a round
+// needs one barrier, not two), and joining a frontier is a plain store of the round's number to the row's
+// mark of the next round's parity. The number of blocks with a changed row travels with the barrier's
+// arrival count, one counter per parity. A round is then a mark load, the gather of active rows and the
+// barrier.
+struct FrDenseCtl {
+  unsigned long long bar[2];  // arrivals (low 32 bits) and arrivals with a change (high) of each parity
+  int32_t abort, round, status, pad;
+  unsigned long long edges;
+};
+
+template <class T>
+struct FrDense {
+  const int32_t *rbeg, *rend, *col;
+  const typename T::TW *w;
+  int32_t n, C, rows;
+  typename T::TX *X[2];  // the caller's X and the second buffer
+  int64_t ldx[2];
+  const typename T::TX *rhs;
+  int64_t ldr;
+  const typename T::TX *diag;
+  double delta;
+  int32_t *mark[2];  // mark[r & 1][v] == r + 1: v is in the frontier of round r
+  FrDenseCtl *ctl;
+  int32_t max_rounds;
+  int G, LV;
+};
+constexpr int kFrDenseThreads = 512;
+
+template <class T, int VW>
+__global__ void __launch_bounds__(kFrDenseThreads, 1) k_frontier_dense(FrDense<T> p) {
+  using TA = typename T::TA;
+  using TX = typename T::TX;
+  constexpr int NT = kFrDenseThreads;
+  FrDenseCtl *ctl = p.ctl;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int G = p.G, LV = p.LV, ES = G / LV, gpw = 32 / G;
+  const int gl = lane & (G - 1), cl = gl & (LV - 1), es = gl / LV;
+  const bool on = cl * VW < p.C;
+  const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (lane & ~(G - 1));
+  const int row0 = blockIdx.x * p.rows, nr = max(0, min(p.rows, p.n - row0));
+  extern __shared__ uint8_t s_moved[];  // per row: it changed in the round before (its old buffer is stale)
+  __shared__ int s_any, s_go;
+  for (int i = threadIdx.x; i < nr; i += NT) s_moved[i] = 0;
+  const int r0 = __ldcg(&ctl->round);
+  unsigned long long edges = 0;
+  unsigned long long seen[2] = {0, 0};  // each parity's count after its last round (zero at the launch)
+  int done = 0, status = 0;
+  for (; done < p.max_rounds; ++done) {
+    const int rd = r0 + done;
+    const TX *X = p.X[rd & 1];
+    TX *Xn = p.X[(rd + 1) & 1];
+    const int64_t ldx = p.ldx[rd & 1], ldn = p.ldx[(rd + 1) & 1];
+    const int32_t *mark = p.mark[rd & 1];
+    int32_t *next = p.mark[(rd + 1) & 1];
+    if (threadIdx.x == 0) s_any = 0;
+    __syncthreads();
+    for (int g0 = wid * gpw; g0 < nr; g0 += (NT / 32) * gpw) {
+      const int i = g0 + lane / G;
+      const bool valid = i < nr;
+      const long long r = row0 + i;
+      const bool act = valid && __ldcg(mark + r) == rd + 1;
+      const bool stale = valid && s_moved[i] != 0;
+      if (!__any_sync(0xffffffffu, act || stale)) continue;
+      const int beg = act ? p.rbeg[r] : 0, end = act ? p.rend[r] : 0;
+      TA acc[VW];
+#pragma unroll
+      for (int k = 0; k < VW; ++k) acc[k] = TA(0);
+      for (int j = beg + es; j < end && on; j += ES) {
+        TX x[VW];
+        if constexpr (VW > 1) {
+          load_vec_coherent<TX, VW, TX>(X + (long long)p.col[j] * ldx + cl * VW, x);
+        } else {
+          x[0] = __ldcg(X + (long long)p.col[j] * ldx + cl);
+        }
+        const TA wv = cvt<TA>(p.w[j]);
+#pragma unroll
+        for (int k = 0; k < VW; ++k) acc[k] = fmaa(wv, cvt<TA>(x[k]), acc[k]);
+      }
+      for (int off = LV; off < G; off <<= 1) {
+#pragma unroll
+        for (int k = 0; k < VW; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+      }
+      bool ch = false;
+      TX xo[VW], xn[VW];
+      if (valid && es == 0 && (act || stale)) {
+        const TA inv = act ? TA(1) / cvt<TA>(p.diag[r]) : TA(0);
+#pragma unroll
+        for (int k = 0; k < VW; ++k) {
+          const int c = cl * VW + k;
+          xo[k] = xn[k] = c < p.C ? __ldcg(X + r * ldx + c) : TX(0);
+          if (act && c < p.C) {
+            const TA yv = (cvt<TA>(p.rhs[r * p.ldr + c]) + acc[k]) * inv;
+            xn[k] = cvt<TX>(yv);
+            ch |= fabs(yv - cvt<TA>(xo[k])) > (TA)p.delta;
+          }
+        }
+      }
+      const bool any = (__ballot_sync(0xffffffffu, ch) & gmask) != 0;  // the row changed (any of its lanes)
+      if (valid && es == 0 && (any || stale)) {
+#pragma unroll
+        for (int k = 0; k < VW; ++k)
+          if (cl * VW + k < p.C) __stcg(Xn + r * ldn + cl * VW + k, any ? xn[k] : xo[k]);
+      }
+      if (gl == 0 && act) edges += (unsigned long long)(end - beg);
+      if (any && gl == 0) {
+        edges += (unsigned long long)(end - beg);
+        s_any = 1;
+      }
+      if (any) {  // the row and its stored neighbours are the next frontier
+        for (int j = beg + gl; j < end; j += G) __stcg(next + p.col[j], rd + 2);
+        if (gl == 0) __stcg(next + r, rd + 2);
+      }
+      if (valid && gl == 0) s_moved[i] = any;
+    }
+    // the barrier, with this block's word on whether any row changed
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long *bar = &ctl->bar[rd & 1];
+      const unsigned long long was = seen[rd & 1];
+      __threadfence();
+      atomicAdd(bar, 1ull + (s_any ? 1ull << 32 : 0ull));
+      int spins = 0, go = 0;
+      unsigned long long v = 0;
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
+        if ((uint32_t)v - (uint32_t)was >= gridDim.x) break;
+        if ((++spins & 1023) == 0) {
+          if (*(volatile int32_t *)&ctl->abort) go = -1;
+          if (spins >= kBarSpins) {
+            atomicExch(&ctl->abort, 1);
+            go = -1;
+          }
+          if (go < 0) break;
+        }
+      }
+      __threadfence();
+      seen[rd & 1] = v;
+      s_go = go < 0 ? -1 : (uint32_t)(v >> 32) != (uint32_t)(was >> 32);
+    }
+    __syncthreads();
+    if (s_go < 0) return;
+    if (s_go == 0) {  // nothing changed in this round
+      ++done;
+      status = 1;
+      break;
+    }
+  }
+  // the newest values are those the next round would read; the other buffer takes them too (the result is
+  // in the caller's X, and a further launch starts from equal buffers)
+  const int rd = r0 + done;
+  const TX *src = p.X[rd & 1];
+  TX *dst = p.X[(rd + 1) & 1];
+  const int64_t lds = p.ldx[rd & 1], ldd = p.ldx[(rd + 1) & 1];
+  for (int i = threadIdx.x; i < nr * p.C; i += NT) {
+    const long long r = row0 + i / p.C;
+    const int c = i % p.C;
+    __stcg(dst + r * ldd + c, __ldcg(src + r * lds + c));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) edges += __shfl_xor_sync(0xffffffffu, edges, off);
+  if (lane == 0 && edges) atomicAdd(&ctl->edges, edges);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->round = rd;
+    ctl->status = status;
+  }
+}
+
+__global__ void k_frontier_marks(const int32_t *__restrict__ seed, int32_t ns, int32_t *mark) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < ns) mark[seed[i]] = 1;
+}
+
 __global__ void k_frontier_seed(const int32_t *__restrict__ seed, int32_t ns, FrCtl *ctl, int32_t *front) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) ctl->fcnt[0] = ns;
@@ -167,7 +342,8 @@ static size_t fr_align(size_t x) { return (x + 255) / 256 * 256; }
 
 static size_t fr_bytes(int32_t n, int32_t C, size_t es) {
   const size_t nn = (size_t)(n > 0 ? n : 1);
-  return fr_align(sizeof(FrCtl)) + 4 * fr_align(4 * nn) + fr_align(es * nn * (size_t)C);
+  // the dense form's second buffer is padded by up to three columns
+  return fr_align(sizeof(FrCtl)) + 4 * fr_align(4 * nn) + fr_align(es * nn * (size_t)(C + 3));
 }
 
 template <class T>
@@ -205,6 +381,48 @@ struct FrRun {
   }
 };
 
+// Whether the rounds run without lists: up to kFrDenseRows rows, and the gather layout's entry slots leave
+// room for one lane per vector of a row.
+constexpr int kFrDenseRows = 300000;
+
+template <class T, int VW>
+static int launch_dense(FrDense<T> &a, cudaStream_t s) {
+  void *args[] = {(void *)&a};
+  const int grid = (a.n + a.rows - 1) / a.rows;
+  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_frontier_dense<T, VW>, dim3(grid), dim3(kFrDenseThreads), args,
+                                       (size_t)a.rows, s));
+  return check_launch();
+}
+
+template <class T>
+static int run_dense(FrDense<T> &a, int VW, const int32_t *seed, int32_t nseed, int32_t max_rounds, char *marks,
+                     int32_t *rounds_out, unsigned long long *edges_out, cudaStream_t s) {
+  using TX = typename T::TX;
+  DLP_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(FrDenseCtl), s));
+  const size_t mb = fr_align(4 * (size_t)a.n);
+  DLP_CUDA(cudaMemsetAsync(marks, 0, 2 * mb, s));
+  a.mark[0] = (int32_t *)marks;
+  a.mark[1] = (int32_t *)(marks + mb);
+  k_frontier_marks<<<ceil_div_i(nseed, 256), 256, 0, s>>>(seed, nseed, a.mark[0]);
+  DLP_TRY(check_launch());
+  DLP_CUDA(cudaMemcpy2DAsync(a.X[1], a.ldx[1] * sizeof(TX), a.X[0], a.ldx[0] * sizeof(TX), a.C * sizeof(TX), a.n,
+                             cudaMemcpyDeviceToDevice, s));
+  FrDenseCtl h{};
+  while (h.round < max_rounds) {
+    a.max_rounds = std::min(kFrChunk, max_rounds - h.round);
+    if (h.round > 0) DLP_CUDA(cudaMemsetAsync(a.ctl->bar, 0, sizeof(a.ctl->bar), s));
+    if (VW == 1) DLP_TRY((launch_dense<T, 1>(a, s)));
+    else DLP_TRY((launch_dense<T, 16 / sizeof(TX)>(a, s)));
+    DLP_CUDA(cudaMemcpyAsync(&h, a.ctl, sizeof(h), cudaMemcpyDeviceToHost, s));
+    DLP_CUDA(cudaStreamSynchronize(s));
+    if (h.abort) return DLP_ERR_DEVICE;
+    if (h.status) break;
+  }
+  if (rounds_out) *rounds_out = h.round;
+  if (edges_out) *edges_out = h.edges;
+  return DLP_OK;
+}
+
 template <class T>
 static int run_frontier(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const void *w, int32_t n,
                         int32_t C, void *X, int64_t ldx, const void *rhs, int64_t ldr, const void *diag, double delta,
@@ -220,6 +438,35 @@ static int run_frontier(const int32_t *rbeg, const int32_t *rend, const int32_t 
     q += fr_align(b);
     return r;
   };
+  {
+    const int LV = next_pow2(L.NV), ES = L.G / L.LV;
+    if (n <= kFrDenseRows && LV * ES <= 32) {
+      FrDense<T> d{};
+      d.rbeg = rbeg;
+      d.rend = rend;
+      d.col = col;
+      d.w = (const typename T::TW *)w;
+      d.n = n;
+      d.C = C;
+      d.rows = std::max((n + sm_count() - 1) / sm_count(), 8);
+      d.rhs = (const TX *)rhs;
+      d.ldr = ldr;
+      d.diag = (const TX *)diag;
+      d.delta = delta;
+      d.G = LV * ES;
+      d.LV = LV;
+      d.ctl = (FrDenseCtl *)take(sizeof(FrCtl) > sizeof(FrDenseCtl) ? sizeof(FrCtl) : sizeof(FrDenseCtl));
+      char *marks = take(4 * nn);
+      take(4 * nn);
+      take(4 * nn);
+      take(4 * nn);
+      d.X[0] = (TX *)X;
+      d.ldx[0] = ldx;
+      d.X[1] = (TX *)take(sizeof(TX) * nn * (size_t)(C + 3));
+      d.ldx[1] = (int64_t)L.NV * L.VW;
+      return run_dense<T>(d, L.VW, seed, nseed, max_rounds, marks, rounds_out, edges_out, s);
+    }
+  }
   FrRun<T> R;
   R.s = s;
   FrArgs<T> &a = R.a;

@@ -33,7 +33,9 @@ def test_first_solve_asks_for_what_its_precision_resolves(method, lowp, target):
 
 @pytest.mark.parametrize("n,K,dtype,deg,max_iter", [(40, 2, "float32", 6, 10**7), (257, 2, "float32", 6, 10**7),
                                                     (5000, 3, "float32", 10, 10**7), (5000, 9, "float64", 10, 10**7),
-                                                    (3001, 33, "float32", 24, 10**7), (20_000, 4, "float32", 10, 7)])
+                                                    (3001, 33, "float32", 24, 10**7), (20_000, 4, "float32", 10, 7),
+                                                    (20_000, 2, "float32", 10, 8), (300_001, 2, "float32", 6, 12),
+                                                    (299_999, 2, "float32", 6, 12)])
 def test_frontier_rounds_on_the_device_equal_the_host_loop(n, K, dtype, deg, max_iter):
     """DynLP with its rounds in one launch against the same rounds launched one by one: the same
     per-row arithmetic on the same frontiers, so scores, rounds and edge visits are equal."""
