@@ -52,6 +52,8 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_ground_reach_workspace_bytes": ("i", ct.c_size_t),
     "dlp_ground_reach": ("ippppippppppppzp", ct.c_int),
     "dlp_ground_reach_async": ("ippppippppppppzp", ct.c_int),
+    "dlp_fh_components_workspace_bytes": ("i", ct.c_size_t),
+    "dlp_fh_components": ("iqpppdppppzp", ct.c_int),
     "dlp_cc_mask_labels_workspace_bytes": ("i", ct.c_size_t),
     "dlp_cc_mask_labels": ("ippppppzp", ct.c_int),
     "dlp_cc_relabel": ("ippppzp", ct.c_int),

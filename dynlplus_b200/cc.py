@@ -89,56 +89,27 @@ def ground_reach(G, vmask, sink, umask, in_t, w=None):
 # ---------------------------------------------------------------------------------------------
 # adaptive components of new vertices (dynlp/cc.py:26-83)
 # ---------------------------------------------------------------------------------------------
-def _lightest(nc, cu, cv, de):
-    """Per component with an outgoing edge: (component, the other side, weight) of its lightest one,
-    ties to the smallest other side (dynlp/cc.py:26-34). min-reductions: order-independent."""
-    dev = cu.device
-    best = torch.full((nc,), float("inf"), dtype=torch.float32, device=dev)
-    best.scatter_reduce_(0, cu, de, "amin")
-    nb = torch.full((nc,), nc, dtype=torch.int64, device=dev)
-    sel = de <= best[cu]
-    nb.scatter_reduce_(0, cu[sel], cv[sel], "amin")
-    c = torch.nonzero(nb < nc, as_tuple=False).flatten()
-    return c, nb[c], best[c]
-
-
 def fh_components(m, rows, cols, d, k, ground=None):
     """Felzenszwalb-Huttenlocher merging in Boruvka rounds (dynlp/cc.py:37-73): each round every
-    component takes its lightest outgoing edge and merges across it when d(e) <= min over both
-    sides of Int(C) + k/|C| (Int = largest internal dissimilarity, fp32 as the reference keeps it);
-    with `ground`, components holding none then join their lightest neighbour until every one has
-    some. The merges of a round are one call of the component kernel (rank labels)."""
+    component takes its lightest outgoing edge (ties to the smallest other side) and merges across it
+    when d(e) <= min over both sides of Int(C) + k/|C| (Int = largest internal dissimilarity, fp32 as
+    the reference keeps it); with `ground`, components holding none then join their lightest neighbour
+    until every one has some. One launch (dlp_fh_components) and the rank labels."""
     dev = rows.device
-    lab = torch.arange(m, dtype=torch.int64, device=dev)
-    Int = torch.zeros(m, dtype=torch.float32, device=dev)
-    size = torch.ones(m, dtype=torch.float32, device=dev)
-    rows, cols, d = rows.long(), cols.long(), d.to(torch.float32)
-    g_v = ground.to(torch.float32) if ground is not None else None
-    nc, fh = m, True
-    while rows.numel():
-        cu, cv = lab[rows], lab[cols]
-        ext = cu != cv
-        if not fh:
-            g = torch.zeros(nc, dtype=torch.float32, device=dev).index_add_(0, lab, g_v)
-            ext &= g[cu] == 0
-        if not bool(ext.any()):
-            break
-        c, t, dc = _lightest(nc, cu[ext], cv[ext], d[ext])
-        if fh:
-            ok = dc <= torch.minimum(Int[c] + k / size[c], Int[t] + k / size[t])
-            if not bool(ok.any()):
-                if g_v is None:
-                    break
-                fh = False
-                continue
-            c, t, dc = c[ok], t[ok], dc[ok]
-        root, nc = connected_components(nc, c.to(torch.int32), t.to(torch.int32))
-        root = root.long()
-        Int2 = torch.zeros(nc, dtype=torch.float32, device=dev).scatter_reduce_(0, root, Int, "amax")
-        Int2.scatter_reduce_(0, root[c], dc, "amax")
-        size2 = torch.zeros(nc, dtype=torch.float32, device=dev).index_add_(0, root, size)
-        lab, Int, size = root[lab], Int2, size2
-    return lab.to(torch.int32), nc
+    if m == 0 or not rows.numel():
+        return torch.arange(m, dtype=torch.int32, device=dev), m
+    rows, cols = rows.to(torch.int32).contiguous(), cols.to(torch.int32).contiguous()
+    d = d.to(torch.float32).contiguous()
+    g = ground.to(torch.float32).contiguous() if ground is not None else None
+    root = torch.empty(m, dtype=torch.int32, device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    ws = workspace("fh").get(_lib.lib().dlp_fh_components_workspace_bytes(m))
+    _lib.call("dlp_fh_components", int(m), int(rows.numel()), ptr(rows), ptr(cols), ptr(d), float(k), ptr(g), ptr(root),
+              ptr(err), ptr(ws), ws.numel(), stream())
+    lab, nc = relabel(root)
+    if int(err.item()):
+        raise _lib.DLPError("dlp_fh_components", 8)
+    return lab, nc
 
 
 def adaptive_components(m, rows, cols, w, s_r, s_c, wmax, ground=None):

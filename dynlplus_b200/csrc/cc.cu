@@ -320,6 +320,125 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
   if (first) info[2] = settled ? sweeps : -sweeps;
 }
 
+// ------------------------------------------------------------------------------------------------
+// Felzenszwalb-Huttenlocher merging in Boruvka rounds (dynlp/cc.py:37-73) in one cooperative launch. A
+// component is named by its smallest vertex (the order of the reference's ranks), so no round renumbers.
+// A round: every component's lightest outgoing edge (ordered-float atomicMin), the smallest component on
+// the other side among its ties, the merge test, the unions, then internal dissimilarity, size and
+// grounding folded into the new roots and the vertices relabelled; six grid barriers. Bound by them (some
+// 15 us a round); the tensor operations it replaces took 25 launches and three host reads a round (vertex
+// arrivals, n = 20,000, 40 rounds in five batches: 25 ms of 45).
+// ------------------------------------------------------------------------------------------------
+struct FhCtl {
+  GridBar bar;
+  int32_t ext[2], ok[2];  // this round saw an outgoing edge / a permitted merge, by the round's parity
+};
+
+__device__ __forceinline__ uint32_t float_order(float x) {  // monotone in the float's order
+  const uint32_t b = __float_as_uint(x);
+  return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+
+constexpr int kFhThreads = 512;
+__global__ void __launch_bounds__(kFhThreads, 1)
+    k_fh_components(int32_t m, long long E, const int32_t *__restrict__ rows, const int32_t *__restrict__ cols,
+                    const float *__restrict__ d, float k, const float *__restrict__ ground, int32_t *parent,
+                    int32_t *lab, float *internal, int32_t *size, int32_t *grounded, uint32_t *best, float *bestd,
+                    int32_t *nb, int32_t *err, FhCtl *ctl) {
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  uint32_t target = 0;
+  auto barrier = [&]() -> bool {
+    if (grid_barrier(&ctl->bar, target)) return true;
+    if (t0 == 0) atomicExch(err, DLP_ERR_DEVICE);
+    return false;
+  };
+  for (long long v = t0; v < m; v += step) {
+    parent[v] = lab[v] = (int32_t)v;
+    internal[v] = 0.f;
+    size[v] = 1;
+    grounded[v] = ground && ground[v] != 0.f;
+    best[v] = 0xffffffffu;
+    nb[v] = m;
+  }
+  if (!barrier()) return;
+  bool fh = true;
+  for (int round = 0;; ++round) {
+    const int p = round & 1;
+    // the lightest outgoing edge of every component (of the ungrounded ones once fh is over)
+    bool any = false;
+    for (long long e = t0; e < E; e += step) {
+      const int32_t cu = __ldcg(lab + rows[e]), cv = __ldcg(lab + cols[e]);
+      if (cu == cv || (!fh && __ldcg(grounded + cu))) continue;
+      any = true;
+      atomicMin(best + cu, float_order(d[e]));
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) atomicExch(&ctl->ext[p], 1);
+    if (t0 == 0) ctl->ext[p ^ 1] = ctl->ok[p ^ 1] = 0;
+    if (!barrier()) return;
+    if (__ldcg(&ctl->ext[p]) == 0) break;
+    for (long long e = t0; e < E; e += step) {
+      const int32_t cu = __ldcg(lab + rows[e]), cv = __ldcg(lab + cols[e]);
+      if (cu == cv || (!fh && __ldcg(grounded + cu))) continue;
+      if (float_order(d[e]) == __ldcg(best + cu)) {
+        atomicMin(nb + cu, cv);
+        __stcg(bestd + cu, d[e]);  // ties store the same value
+      }
+    }
+    if (!barrier()) return;
+    any = false;
+    for (long long c = t0; c < m; c += step) {
+      const int32_t t = __ldcg(nb + c);
+      if (t >= m) continue;
+      if (fh) {
+        const float a = __fadd_rn(__ldcg(internal + c), __fmul_rn(__frcp_rn((float)__ldcg(size + c)), k));
+        const float b = __fadd_rn(__ldcg(internal + t), __fmul_rn(__frcp_rn((float)__ldcg(size + t)), k));
+        if (!(__ldcg(bestd + c) <= fminf(a, b))) {
+          __stcg(nb + c, m);  // not permitted
+          continue;
+        }
+      }
+      any = true;
+    }
+    if (__syncthreads_or(any) && threadIdx.x == 0) atomicExch(&ctl->ok[p], 1);
+    if (!barrier()) return;
+    if (__ldcg(&ctl->ok[p]) == 0) {  // only under fh: a component with an outgoing edge always merges after
+      if (!ground) break;
+      fh = false;
+      for (long long c = t0; c < m; c += step) {
+        best[c] = 0xffffffffu;
+        nb[c] = m;
+      }
+      if (!barrier()) return;
+      continue;
+    }
+    for (long long c = t0; c < m; c += step) {
+      const int32_t t = __ldcg(nb + c);
+      if (t < m) unite(parent, (int32_t)c, t, err);
+    }
+    if (!barrier()) return;
+    for (long long c = t0; c < m; c += step) {
+      const int32_t v = __ldcg(lab + c);  // before this round's relabelling: c is a component if v == c
+      if (v == (int32_t)c) {
+        const int32_t r = find_root(parent, (int32_t)c, err);
+        if (r != (int32_t)c) {
+          atomicMax((int *)internal + r, __float_as_int(__ldcg(internal + c)));  // non-negative: ordered as ints
+          atomicAdd(size + r, __ldcg(size + c));
+          if (__ldcg(grounded + c)) atomicExch(grounded + r, 1);
+        }
+        if (__ldcg(nb + c) < m) {
+          atomicMax((int *)internal + r, __float_as_int(fmaxf(__ldcg(bestd + c), 0.f)));
+          __stcg(nb + c, m);
+        }
+        __stcg(best + c, 0xffffffffu);
+      }
+      __stcg(bestd + c, 0.f);
+    }
+    if (!barrier()) return;
+    for (long long v = t0; v < m; v += step) __stcg(lab + v, find_root(parent, __ldcg(lab + v), err));
+    if (!barrier()) return;
+  }
+}
+
 // label[lpos[v]] = rank[parent[v]] for every masked v: the rank of its component's minimum id,
 // written at the vertex's place among the masked vertices.
 __global__ void k_cc_mask_gather(int32_t n, const int32_t *__restrict__ parent, const uint8_t *__restrict__ vmask,
@@ -641,6 +760,43 @@ int dlp_ground_reach(int32_t n, const int32_t *rbeg, const int32_t *rend, const 
   DLP_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   if (sweeps_out) *sweeps_out = h[2];
   return h[3] ? DLP_ERR_DEVICE : DLP_OK;
+}
+
+static size_t fh_vec(int32_t m) { return ((size_t)(m > 0 ? m : 1) * 4 + 255) / 256 * 256; }
+
+size_t dlp_fh_components_workspace_bytes(int32_t m) { return 7 * fh_vec(m) + 256; }
+
+int dlp_fh_components(int32_t m, int64_t E, const int32_t *rows, const int32_t *cols, const float *d, double k,
+                      const float *ground, int32_t *root, int32_t *err, void *ws, size_t ws_bytes, dlp_stream_t stream) {
+  if (m < 0 || E < 0 || (m > 0 && !root) || (E > 0 && (!rows || !cols || !d)) || !err) return DLP_ERR_INVALID;
+  if (!ws || ws_bytes < dlp_fh_components_workspace_bytes(m)) return DLP_ERR_WORKSPACE;
+  if (m == 0) return DLP_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  char *p = (char *)ws;
+  auto take = [&]() {
+    char *q = p;
+    p += fh_vec(m);
+    return q;
+  };
+  int32_t *lab = (int32_t *)take();
+  float *internal = (float *)take();
+  int32_t *size = (int32_t *)take(), *grounded = (int32_t *)take();
+  uint32_t *best = (uint32_t *)take();
+  float *bestd = (float *)take();
+  int32_t *nb = (int32_t *)take();
+  FhCtl *ctl = (FhCtl *)p;
+  DLP_CUDA(cudaMemsetAsync(ctl, 0, sizeof(FhCtl), s));
+  long long EE = E;
+  float kf = (float)k;
+  void *args[] = {(void *)&m,        (void *)&EE,   (void *)&rows,     (void *)&cols, (void *)&d,     (void *)&kf,
+                  (void *)&ground,   (void *)&root, (void *)&lab,      (void *)&internal, (void *)&size,
+                  (void *)&grounded, (void *)&best, (void *)&bestd,    (void *)&nb,   (void *)&err,   (void *)&ctl};
+  const int grid = (int)std::max(1LL, std::min((long long)sm_count(), (std::max((long long)m, EE) + kFhThreads - 1) / kFhThreads));
+  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_fh_components, dim3(grid), dim3(kFhThreads), args, 0, s));
+  DLP_TRY(check_launch());
+  // root[v] is the parent after the last unions: relabelled to the component's smallest vertex
+  DLP_CUDA(cudaMemcpyAsync(root, lab, sizeof(int32_t) * (size_t)m, cudaMemcpyDeviceToDevice, s));
+  return DLP_OK;
 }
 
 size_t dlp_cc_mask_labels_workspace_bytes(int32_t n) {

@@ -236,6 +236,15 @@ int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, 
                            int32_t *count, int32_t *err, int32_t *info, void *ws, size_t ws_bytes,
                            dlp_stream_t stream);
 
+/* Felzenszwalb-Huttenlocher merging (dynlp/cc.py:37-73) of m vertices over E weighted edges (both
+ * directions stored): Boruvka rounds on the device in one cooperative launch; with ground (m floats,
+ * may be NULL) components without any then join their lightest neighbour. root[v] = the smallest vertex
+ * of v's component (dlp_cc_relabel numbers them). *err (device int, caller-zeroed) is set when a wait on
+ * the device ran out. Asynchronous. */
+size_t dlp_fh_components_workspace_bytes(int32_t m);
+int dlp_fh_components(int32_t m, int64_t E, const int32_t *rows, const int32_t *cols, const float *d, double k,
+                      const float *ground, int32_t *root, int32_t *err, void *ws, size_t ws_bytes, dlp_stream_t stream);
+
 /* The reference's component labels of the masked vertices: connected_components over the
  * subgraph that vmask induces, numbered as dynlp/stream.py:150-153 with dynlp/cc.py:22 number them
  * (local ids = the masked vertices in ascending order; a component's label = the rank of its smallest

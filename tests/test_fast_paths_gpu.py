@@ -297,3 +297,25 @@ def test_grounding_in_one_launch(kind, n):
     active, lost, sweeps, bad = info.tolist()
     assert (active, lost, bad) == (int(vmask.sum() + sink.sum()), int((vmask > want).sum()), 0)
     assert ce.tolist() == [int((want != old).sum()), 0] and 1 <= abs(sweeps) <= 32
+
+
+@pytest.mark.parametrize("m,deg,grounds,ties", [(1, 0, True, False), (2, 2, False, False), (513, 4, True, False),
+                                                (2000, 3, True, True), (2000, 3, False, True), (75_777, 6, True, False)])
+def test_fh_components_on_the_device(m, deg, grounds, ties):
+    """The merging rounds in one launch against the oracle's, label for label: random graphs, tied
+    weights, with and without grounding, from one vertex to more than one block's worth per SM."""
+    from dynlplus_b200 import cc
+    from oracle import ref_np as O
+    rng = np.random.default_rng(m + deg)
+    e = m * deg // 2
+    u, v = rng.integers(0, m, e), rng.integers(0, m, e)
+    d = rng.integers(1, 5, e).astype(np.float32) if ties else rng.uniform(0.05, 2, e).astype(np.float32)
+    keep = u != v
+    u, v, d = u[keep], v[keep], d[keep]
+    rows, cols, dd = np.r_[u, v], np.r_[v, u], np.r_[d, d]
+    g = (rng.random(m) < 0.02).astype(np.float32) if grounds else None
+    k = 1.5
+    want, nc = O.fh_components(m, rows, cols, dd, np.float32(k), g)
+    T = lambda x: torch.as_tensor(x).cuda()  # noqa: E731
+    lab, n2 = cc.fh_components(m, T(rows), T(cols), T(dd), k, T(g) if g is not None else None)
+    assert n2 == nc and np.array_equal(lab.cpu().numpy(), want)
