@@ -227,35 +227,51 @@ __global__ void __launch_bounds__(kFrDenseThreads, 1) k_frontier_dense(FrDense<T
       TA acc[VW];
 #pragma unroll
       for (int k = 0; k < VW; ++k) acc[k] = TA(0);
-      for (int j = beg + es; j < end && on; j += ES) {
-        TX x[VW];
-        if constexpr (VW > 1) {
-          load_vec_coherent<TX, VW, TX>(X + (long long)p.col[j] * ldx + cl * VW, x);
-        } else {
-          x[0] = __ldcg(X + (long long)p.col[j] * ldx + cl);
-        }
-        const TA wv = cvt<TA>(p.w[j]);
+      // the row's own values and right-hand side, in flight with the gather
+      TX xo[VW], xn[VW], rh[VW];
+      const bool own = valid && es == 0 && (act || stale);
 #pragma unroll
-        for (int k = 0; k < VW; ++k) acc[k] = fmaa(wv, cvt<TA>(x[k]), acc[k]);
+      for (int k = 0; k < VW; ++k) {
+        const int c = cl * VW + k;
+        xo[k] = own && c < p.C ? __ldcg(X + r * ldx + c) : TX(0);
+        rh[k] = own && act && c < p.C ? p.rhs[r * p.ldr + c] : TX(0);
+      }
+      const TA inv = own && act ? TA(1) / cvt<TA>(p.diag[r]) : TA(0);
+      constexpr int U = VW == 1 ? 8 : 4;  // entries in flight per lane
+      for (int j0 = beg + es; j0 < end && on; j0 += U * ES) {
+        int v[U];
+        TA wv[U];
+        TX x[U][VW];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = j0 + u * ES;
+          v[u] = j < end ? p.col[j] : -1;
+          wv[u] = j < end ? cvt<TA>(p.w[j]) : TA(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+          for (int k = 0; k < VW; ++k) x[u][k] = TX(0);
+          if (v[u] >= 0) {
+            if constexpr (VW > 1) load_vec_coherent<TX, VW, TX>(X + (long long)v[u] * ldx + cl * VW, x[u]);
+            else x[u][0] = __ldcg(X + (long long)v[u] * ldx + cl);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int k = 0; k < VW; ++k) acc[k] = fmaa(wv[u], cvt<TA>(x[u][k]), acc[k]);
       }
       for (int off = LV; off < G; off <<= 1) {
 #pragma unroll
         for (int k = 0; k < VW; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
       }
       bool ch = false;
-      TX xo[VW], xn[VW];
-      if (valid && es == 0 && (act || stale)) {
-        const TA inv = act ? TA(1) / cvt<TA>(p.diag[r]) : TA(0);
 #pragma unroll
-        for (int k = 0; k < VW; ++k) {
-          const int c = cl * VW + k;
-          xo[k] = xn[k] = c < p.C ? __ldcg(X + r * ldx + c) : TX(0);
-          if (act && c < p.C) {
-            const TA yv = (cvt<TA>(p.rhs[r * p.ldr + c]) + acc[k]) * inv;
-            xn[k] = cvt<TX>(yv);
-            ch |= fabs(yv - cvt<TA>(xo[k])) > (TA)p.delta;
-          }
-        }
+      for (int k = 0; k < VW; ++k) {
+        const TA yv = (cvt<TA>(rh[k]) + acc[k]) * inv;
+        xn[k] = cvt<TX>(yv);
+        ch |= own && act && cl * VW + k < p.C && fabs(yv - cvt<TA>(xo[k])) > (TA)p.delta;
       }
       const bool any = (__ballot_sync(0xffffffffu, ch) & gmask) != 0;  // the row changed (any of its lanes)
       if (valid && es == 0 && (any || stale)) {
