@@ -45,6 +45,8 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_colreduce": ("iiipqpqpipppzp", ct.c_int),
     "dlp_colreduce_noalloc": ("iiipqpqpippp", ct.c_int),
     "dlp_cc_edges": ("ippqppp", ct.c_int),
+    "dlp_cc_edges_workspace_bytes": ("", ct.c_size_t),
+    "dlp_cc_edges_ws": ("ippqpppzp", ct.c_int),
     "dlp_cc_graph_workspace_bytes": ("", ct.c_size_t),
     "dlp_cc_graph": ("ippppipppppzp", ct.c_int),
     "dlp_cc_graph_warm_workspace_bytes": ("i", ct.c_size_t),

@@ -14,35 +14,47 @@ from . import _lib
 from .backend import code, ptr, stream, workspace
 
 
-def min_vertex_roots(n, rows, cols) -> torch.Tensor:
-    """parent[v] = smallest vertex id in v's component (int32, device)."""
+def _roots(n, rows, cols, err) -> torch.Tensor:
     rows = rows.to(torch.int32).contiguous()
     cols = cols.to(torch.int32).contiguous()
-    dev = rows.device
-    parent = torch.empty(max(n, 1), dtype=torch.int32, device=dev)
-    err = torch.zeros(1, dtype=torch.int32, device=dev)
-    _lib.call("dlp_cc_edges", int(n), ptr(rows), ptr(cols), int(rows.numel()), ptr(parent), ptr(err), stream())
-    if int(err.item()):
-        raise ValueError("connected_components: edge endpoint outside [0, n)")
+    parent = torch.empty(max(n, 1), dtype=torch.int32, device=rows.device)
+    ws = workspace("cc_edges").get(_lib.lib().dlp_cc_edges_workspace_bytes())
+    _lib.call("dlp_cc_edges_ws", int(n), ptr(rows), ptr(cols), int(rows.numel()), ptr(parent), ptr(err), ptr(ws),
+              ws.numel(), stream())
     return parent[:n]
 
 
-def relabel(parent: torch.Tensor, sync: bool = True):
-    """Rank of each root among the roots (unique + inverse); returns (labels, n_comp)."""
+def min_vertex_roots(n, rows, cols) -> torch.Tensor:
+    """parent[v] = smallest vertex id in v's component (int32, device)."""
+    err = torch.zeros(1, dtype=torch.int32, device=rows.device)
+    parent = _roots(n, rows, cols, err)
+    if int(err.item()):
+        raise ValueError("connected_components: edge endpoint outside [0, n)")
+    return parent
+
+
+def relabel(parent: torch.Tensor, sync: bool = True, count=None):
+    """Rank of each root among the roots (unique + inverse); returns (labels, n_comp). count: where the
+    component count goes (device int32[1])."""
     n = int(parent.numel())
     label = torch.empty(max(n, 1), dtype=torch.int32, device=parent.device)
-    nc = torch.empty(1, dtype=torch.int32, device=parent.device)
+    nc = torch.empty(1, dtype=torch.int32, device=parent.device) if count is None else count
     ws = workspace("compact").get(_lib.lib().dlp_compact_workspace_bytes(n))
     _lib.call("dlp_cc_relabel", n, ptr(parent), ptr(label), ptr(nc), ptr(ws), ws.numel(), stream())
     return (label[:n], int(nc.item())) if sync else (label[:n], nc)
 
 
 def connected_components(n, rows, cols):
-    """(labels in [0, n_comp), n_comp) for an undirected edge list (dynlp/cc.py:8-23)."""
+    """(labels in [0, n_comp), n_comp) for an undirected edge list (dynlp/cc.py:8-23). One host read."""
     if n == 0:
         dev = rows.device if torch.is_tensor(rows) else None
         return torch.zeros(0, dtype=torch.int32, device=dev), 0
-    return relabel(min_vertex_roots(n, rows, cols))
+    ec = torch.zeros(2, dtype=torch.int32, device=rows.device)  # [error, count]
+    label, _ = relabel(_roots(n, rows, cols, ec[:1]), sync=False, count=ec[1:])
+    err, nc = ec.tolist()
+    if err:
+        raise ValueError("connected_components: edge endpoint outside [0, n)")
+    return label, nc
 
 
 def graph_components(G, vmask=None, sink=None, w=None):
@@ -102,12 +114,13 @@ def fh_components(m, rows, cols, d, k, ground=None):
     d = d.to(torch.float32).contiguous()
     g = ground.to(torch.float32).contiguous() if ground is not None else None
     root = torch.empty(m, dtype=torch.int32, device=dev)
-    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    ec = torch.zeros(2, dtype=torch.int32, device=dev)  # [a wait ran out, component count]
     ws = workspace("fh").get(_lib.lib().dlp_fh_components_workspace_bytes(m))
     _lib.call("dlp_fh_components", int(m), int(rows.numel()), ptr(rows), ptr(cols), ptr(d), float(k), ptr(g), ptr(root),
-              ptr(err), ptr(ws), ws.numel(), stream())
-    lab, nc = relabel(root)
-    if int(err.item()):
+              ptr(ec), ptr(ws), ws.numel(), stream())
+    lab, _ = relabel(root, sync=False, count=ec[1:])
+    err, nc = ec.tolist()
+    if err:
         raise _lib.DLPError("dlp_fh_components", 8)
     return lab, nc
 

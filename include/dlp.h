@@ -189,6 +189,11 @@ int dlp_colreduce(int kind, int32_t n, int32_t C, const void *X, int64_t ldx, co
  * [0, n) are rejected with DLP_ERR_DEVICE via *err (device int, caller-zeroed; may be NULL). */
 int dlp_cc_edges(int32_t n, const int32_t *rows, const int32_t *cols, int64_t m, int32_t *parent, int32_t *err,
                  dlp_stream_t stream);
+/* The same with scratch (dlp_cc_edges_workspace_bytes; err required): long edge lists run in rounds in one
+ * cooperative launch, same result. *err is also set when a wait on the device ran out. */
+size_t dlp_cc_edges_workspace_bytes(void);
+int dlp_cc_edges_ws(int32_t n, const int32_t *rows, const int32_t *cols, int64_t m, int32_t *parent, int32_t *err,
+                    void *ws, size_t ws_bytes, dlp_stream_t stream);
 
 /* Graph form used by the grounding checks (dynlp/stream.py:150-159, :275-280): vertices 0..n-1
  * plus a sink vertex n. An entry (u, v) of the row ranges joins u and v when vmask[u] and

@@ -319,3 +319,24 @@ def test_fh_components_on_the_device(m, deg, grounds, ties):
     T = lambda x: torch.as_tensor(x).cuda()  # noqa: E731
     lab, n2 = cc.fh_components(m, T(rows), T(cols), T(dd), k, T(g) if g is not None else None)
     assert n2 == nc and np.array_equal(lab.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,m", [(500_000, 500_000), (900_001, 500_001), (1000, 600_000), (1_100_000, 499_999)])
+def test_components_of_long_edge_lists(n, m):
+    """Component labels around the line where the rounds start, a dense graph and one past the giant
+    component, against SciPy; an endpoint outside the range is refused in the rounds too."""
+    import scipy.sparse as ssp
+    from scipy.sparse.csgraph import connected_components
+    from dynlplus_b200 import cc
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, m), rng.integers(0, n, m)
+    _, want = connected_components(ssp.coo_matrix((np.ones(m), (u, v)), (n, n)), directed=False)
+    first = np.full(want.max() + 1, n)
+    np.minimum.at(first, want, np.arange(n))
+    want = np.argsort(np.argsort(first))[want]  # ranks by smallest vertex
+    T = lambda x: torch.as_tensor(x.astype(np.int32)).cuda()  # noqa: E731
+    lab, nc = cc.connected_components(n, T(u), T(v))
+    assert nc == want.max() + 1 and np.array_equal(lab.cpu().numpy(), want)
+    u[m // 2] = n
+    with pytest.raises(ValueError):
+        cc.connected_components(n, T(u), T(v))
