@@ -54,6 +54,9 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_ground_reach_workspace_bytes": ("i", ct.c_size_t),
     "dlp_ground_reach": ("ippppippppppppzp", ct.c_int),
     "dlp_ground_reach_async": ("ippppippppppppzp", ct.c_int),
+    "dlp_build_system_workspace_bytes": ("i", ct.c_size_t),
+    "dlp_build_system_plan": ("ipppppippppppzp", ct.c_int),
+    "dlp_build_system_fill": ("ipppipppiddiippippppipppppppppp" + "p", ct.c_int),
     "dlp_fh_components_workspace_bytes": ("i", ct.c_size_t),
     "dlp_fh_components": ("iqpppdppppzp", ct.c_int),
     "dlp_cc_mask_labels_workspace_bytes": ("i", ct.c_size_t),

@@ -161,31 +161,53 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
     dt = to_dtype(dtype)
     active = active.to(torch.bool)
     labeled = labeled.to(torch.bool)
-    al = active & labeled
-    Bfull = kernels.spmm_axpy(A, _onehot_labels(ds.y, al, K, dev))  # fp64 (fp32 weights x fp64 onehot)
-    vmask = (active & ~labeled).to(torch.uint8)
-    parent, err = cc.graph_components(A, vmask, al.to(torch.uint8))
-    root = parent[n]
-    Um = vmask.bool() & (parent[:n] == root)
-    n_ungrounded = int((vmask.bool() & ~Um).sum().item())
-    U = torch.nonzero(Um, as_tuple=False).flatten()
-    n_u = int(U.numel())
-    loc = torch.full((n,), -1, dtype=torch.int64, device=dev)
-    loc[U] = torch.arange(n_u, device=dev)
-    rows = csr_rows(A).long()
-    cols = A.indices.long()
-    keep = Um[rows] & Um[cols]
-    indptr = torch.zeros(n_u + 1, dtype=torch.int64, device=dev)
-    indptr[1:] = torch.cumsum(torch.bincount(loc[rows[keep]], minlength=n_u), 0)
-    W = CSR(A.data[keep].to(dt), loc[cols[keep]].to(torch.int32), indptr.to(torch.int32), (n_u, n_u))
-    Bm = Bfull[U]
-    s = Bm.sum(dim=1) + eta
-    ones = torch.ones((n_u, 1), dtype=torch.float64, device=dev)
-    rowsum = kernels.spmm_axpy(W if dt != torch.bfloat16 else W.astype(torch.float32), ones)[:, 0] if n_u else \
-        torch.zeros(0, dtype=torch.float64, device=dev)
-    diag = s + rowsum
-    prior = torch.full((1 if K == 2 else K,), 0.5 if K == 2 else 1.0 / K, dtype=torch.float64, device=dev)
-    rhs = (Bm[:, 1:2] if K == 2 else Bm) + eta * prior[None, :]
+    C = 1 if K == 2 else K
+    f64 = torch.float64
+    masks = torch.empty((2, max(n, 1)), dtype=torch.uint8, device=dev)  # U, and the active labelled vertices
+    scans = torch.empty((2, n + 1), dtype=torch.int32, device=dev)      # local ids, entry positions
+    counts = torch.zeros(9, dtype=torch.int32, device=dev)
+    n_u = nnz = n_active = n_ungrounded = 0
+    y = (ds.y if ds.y.dtype == torch.int32 else ds.y.to(torch.int32)).contiguous()
+    if n:
+        ws = workspace("build_system").get(_lib.lib().dlp_build_system_workspace_bytes(n))
+        _lib.call("dlp_build_system_plan", n, ptr(A.indptr), ptr(A.indices), ptr(active.contiguous()),
+                  ptr(labeled.contiguous()), ptr(y), K, ptr(masks[0]), ptr(masks[1]), ptr(scans[0]), ptr(scans[1]),
+                  ptr(counts), ptr(ws), ws.numel(), stream())
+        n_u, nnz, _, bad, n_active, n_ungrounded, _, lost, off = counts.tolist()
+        if off:
+            raise IndexError(f"a labelled vertex's class is outside [0, {K})")
+        if bad:
+            raise ValueError("grounding: entry column outside [0, n)")
+        if lost:
+            raise _lib.DLPError("dlp_build_system_plan", 8)
+        if n_u and not nnz:  # no kernel takes an operator without entries
+            raise _lib.DLPError("dlp_build_system_plan", 1)
+    wdt = dt if dt != torch.bfloat16 else torch.float32
+    U = torch.empty(n_u, dtype=torch.int64, device=dev)
+    ip = torch.zeros(n_u + 1, dtype=torch.int32, device=dev)
+    ci = torch.empty(nnz, dtype=torch.int32, device=dev)
+    wd = torch.empty(nnz, dtype=wdt, device=dev)
+    v64 = torch.empty((2, n_u), dtype=f64, device=dev)
+    s, diag = v64[0], v64[1]
+    Bm = torch.empty((n_u, K), dtype=f64, device=dev)
+    rhs = torch.empty((n_u, C), dtype=f64, device=dev)
+    rhsh = torch.empty((n_u, C + 1), dtype=f64, device=dev)
+    prior_v = 0.5 if K == 2 else 1.0 / K
+    prior = torch.full((C,), prior_v, dtype=f64, device=dev)
+    lo = None
+    if dt == torch.float32:
+        v32 = torch.empty((2, n_u), dtype=dt, device=dev)
+        lo = (torch.empty((n_u, K), dtype=dt, device=dev), v32[0], v32[1], torch.empty((n_u, C), dtype=dt, device=dev),
+              torch.empty((n_u, C + 1), dtype=dt, device=dev))
+    if n_u:
+        if dt == torch.bfloat16:
+            A = CSR(A.data.to(dt).to(torch.float32), A.indices, A.indptr, A.shape)
+        _lib.call("dlp_build_system_fill", n, ptr(A.indptr), ptr(A.indices), ptr(A.data), code(A.data), ptr(masks[0]),
+                  ptr(masks[1]), ptr(y), K, float(eta), prior_v, C, 1 if K == 2 else 0, ptr(scans[0]),
+                  ptr(scans[1]), n_u, ptr(U), ptr(ip), ptr(ci), ptr(wd), code(wd), ptr(Bm), ptr(s), ptr(diag), ptr(rhs),
+                  ptr(rhsh), *([ptr(x) for x in lo] if lo else [None] * 5), stream())
+        A = ds.A
+    W = CSR(wd if dt != torch.bfloat16 else wd.to(dt), ci, ip, (n_u, n_u))
     is_new = torch.ones(n_u, dtype=torch.bool, device=dev) if prev_U is None else ~prev_U[U]
     seed = is_new.clone()
     if ins_ids is not None or del_ids is not None:
@@ -204,15 +226,14 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
         Wd = W.data.to(dt)
         comps = new_components_rows(new, W.indptr[:-1], W.indptr[1:], W.indices, Wd, nl, tau, wmax,
                                Bm[new].to(dt).sum(dim=1))
-    sysd = dict(t=t, U=U, W=W, s=s.to(dt), diag=diag.to(dt), B=Bm.to(dt), rhs=rhs.to(dt).contiguous(),
-                prior=prior.to(dt), is_new=is_new, seed=seed, comps=comps, K=K, C=1 if K == 2 else K, eta=eta,
-                n_inserted=ins, n_deleted=dele, n_active=int(active.sum().item()), n_ungrounded=n_ungrounded)
-    sysd["rhs_h"] = torch.cat([sysd["rhs"], sysd["diag"][:, None]], dim=1).contiguous()
-    S = System(**sysd)
-    if dt != torch.float64:
-        S._conv[torch.float64] = System(**{**sysd, "W": CSR(W.data.to(torch.float32), W.indices, W.indptr, W.shape),
-                                           "s": s, "diag": diag, "B": Bm, "rhs": rhs.contiguous(),
-                                           "prior": prior, "rhs_h": torch.cat([rhs, diag[:, None]], 1).contiguous()})
+    if lo is None:
+        lo = tuple(x.to(dt) for x in (Bm, s, diag, rhs, rhsh))
+    common = dict(t=t, U=U, is_new=is_new, seed=seed, comps=comps, K=K, C=C, eta=eta, n_inserted=ins, n_deleted=dele,
+                  n_active=n_active, n_ungrounded=n_ungrounded)
+    S = System(W=W, B=lo[0], s=lo[1], diag=lo[2], rhs=lo[3], rhs_h=lo[4], prior=prior.to(dt), **common)
+    if dt != f64:
+        S._conv[f64] = System(W=CSR(W.data.to(torch.float32), W.indices, W.indptr, W.shape), B=Bm, s=s, diag=diag, rhs=rhs,
+                              rhs_h=rhsh, prior=prior, **common)
     return S
 
 

@@ -241,6 +241,26 @@ int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, 
                            int32_t *count, int32_t *err, int32_t *info, void *ws, size_t ws_bytes,
                            dlp_stream_t stream);
 
+/* ---- the grounded system of one batch (Stream._build, dynlp/stream.py:142-177) -----------------
+ * plan: from a symmetric CSR and byte masks, umask (the grounded unlabelled vertices U), sink (active
+ * labelled ones), loc[v] = v's row in the system (exclusive scan of umask, n + 1 ints), pos[v] = v's first
+ * entry there (n + 1 ints), and counts (device, nine ints): rows, entries, -, a column out of range,
+ * active vertices, ungrounded vertices, sweeps, a wait ran out, a labelled vertex's class y outside
+ * [-K, K). Asynchronous; the caller reads counts.
+ * fill: U (ids), the CSR of A[U, U] in stored order with weights in w_out_dtype, B (n_u x K label weights
+ * by class y), s = sum B + eta, diag = s + row sum, rhs = B[:, col0 : col0 + C] + eta * prior, rhsh = [rhs,
+ * diag]; fp32 copies where the pointers are not NULL. */
+size_t dlp_build_system_workspace_bytes(int32_t n);
+int dlp_build_system_plan(int32_t n, const int32_t *indptr, const int32_t *col, const uint8_t *active,
+                          const uint8_t *labeled, const int32_t *y, int32_t K, uint8_t *umask, uint8_t *sink, int32_t *loc, int32_t *pos,
+                          int32_t *counts, void *ws, size_t ws_bytes, dlp_stream_t stream);
+int dlp_build_system_fill(int32_t n, const int32_t *indptr, const int32_t *col, const void *w, int w_dtype,
+                          const uint8_t *umask, const uint8_t *sink, const int32_t *y, int32_t K, double eta,
+                          double prior, int32_t C, int32_t col0, const int32_t *loc, const int32_t *pos, int32_t n_u,
+                          int64_t *U, int32_t *indptr_out, int32_t *col_out, void *w_out, int w_out_dtype, double *B,
+                          double *s_, double *diag, double *rhs, double *rhsh, float *B32, float *s32, float *diag32,
+                          float *rhs32, float *rhsh32, dlp_stream_t stream);
+
 /* Felzenszwalb-Huttenlocher merging (dynlp/cc.py:37-73) of m vertices over E weighted edges (both
  * directions stored): Boruvka rounds on the device in one cooperative launch; with ground (m floats,
  * may be NULL) components without any then join their lightest neighbour. root[v] = the smallest vertex

@@ -340,3 +340,35 @@ def test_components_of_long_edge_lists(n, m):
     u[m // 2] = n
     with pytest.raises(ValueError):
         cc.connected_components(n, T(u), T(v))
+
+
+@pytest.mark.parametrize("n,K,dtype,wdtype,eta", [(6, 2, "float32", "float32", 0.0), (33, 3, "float64", "float64", 0.1),
+                                                  (257, 9, "float32", "float64", 0.0), (5000, 2, "float64", "float32", 0.3),
+                                                  (4999, 17, "float32", "float32", 0.0)])
+def test_built_system_equals_the_oracle(n, K, dtype, wdtype, eta):
+    """The system of a graph with inactive vertices and isolated ones: sets, columns and weights equal the
+    oracle's, sums to 1e-12 (1e-6 in fp32), in both precisions it carries."""
+    from oracle import ref_np as O
+    rng = np.random.default_rng(n)
+    ds = graphs.er_graph(n, 5, K, weights="lognormal", seed=n, dtype=wdtype)
+    y = ds.y.cpu().numpy()
+    active, lab = rng.random(n) < 0.9, rng.random(n) < 0.15
+    lab[:2] = active[:2] = True
+    want = O.build_system(ds.A.to_scipy(), y, K, active, lab, eta=eta)
+    S = stream.build_system(ds, torch.as_tensor(active).cuda(), torch.as_tensor(lab).cuda(), dtype=dtype, eta=eta)
+    assert np.array_equal(S.U.cpu().numpy(), want["U"]) and S.n_ungrounded == want["n_ungrounded"]
+    assert S.n_active == int(active.sum()) and S.U.dtype == torch.int64
+    for T in (S, S.astype(torch.float64)):
+        W, Ww = T.W.to_scipy(), want["W"]
+        assert np.array_equal(W.indptr, Ww.indptr) and np.array_equal(W.indices, Ww.indices)
+        assert np.array_equal(W.data.astype(np.float64), Ww.data.astype(W.data.dtype).astype(np.float64))
+        tol = 1e-12 if T.diag.dtype == torch.float64 and (wdtype == "float32" or dtype == "float64") else 1e-6
+        for name in ("s", "diag", "B", "rhs"):
+            np.testing.assert_allclose(getattr(T, name).double().cpu().numpy(), want[name], rtol=tol, atol=tol)
+        h = torch.cat([T.rhs, T.diag[:, None]], 1)
+        assert torch.equal(T.rhs_h, h) and T.rhs.is_contiguous()
+    bad = ds.y.clone()
+    bad[0] = K
+    with pytest.raises(IndexError):
+        stream.build_system(graphs.Dataset("x", ds.A, bad, K, ds.order), torch.as_tensor(active).cuda(),
+                            torch.as_tensor(lab).cuda(), dtype=dtype)
