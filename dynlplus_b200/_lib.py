@@ -107,6 +107,10 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_pcg_amg": ("ppppiippqpqpqpqpqpqippdiiiidpipidipzppppppq", ct.c_int),
     "dlp_dense_spd_inverse_workspace_bytes": ("i", ct.c_size_t),
     "dlp_dense_spd_inverse": ("ippzp", ct.c_int),
+    "dlp_batch_offsets": ("ippiqppp", ct.c_int),
+    "dlp_batch_colstats_workspace_bytes": ("ii", ct.c_size_t),
+    "dlp_batch_colstats": ("ipqiiippppppzp", ct.c_int),
+    "dlp_batch_scale": ("iipqppqiipppp", ct.c_int),
     "dlp_pcg_batched_workspace_bytes": ("iii", ct.c_size_t),
     "dlp_pcg_batched": ("pppiippqpqpqpqpqiiippppppdiiiiiidpzpppp", ct.c_int),
     "dlp_ground_update": ("ipppppp", ct.c_int),

@@ -38,40 +38,66 @@ class BatchedSystems:
         N = int(self.offsets[-1])
         self.N = N
         nnzs = [s.W.nnz for s in systems]
-        ip = [torch.zeros(1, dtype=torch.int64, device=dev)]
-        cols, ws = [], []
-        base_nnz = 0
-        for s, off in zip(systems, self.offsets[:-1]):
-            W = s.W
-            ip.append(W.indptr[1:].long() + base_nnz)
-            cols.append(W.indices.long() + int(off))
-            ws.append(W.data.float())
-            base_nnz += W.nnz
-        self.indptr = torch.cat(ip).to(torch.int32)
-        self.col = torch.cat(cols).to(torch.int32) if cols else torch.zeros(0, dtype=torch.int32, device=dev)
-        self.w = torch.cat(ws) if ws else torch.zeros(0, dtype=torch.float32, device=dev)
         self.nnz = int(sum(nnzs))
+        # concatenated as they are; one kernel then shifts the row pointers and columns of each block
+        self.indptr = torch.cat([torch.zeros(1, dtype=torch.int32, device=dev)] + [s.W.indptr[1:].to(torch.int32) for s in systems])
+        self.col = torch.cat([s.W.indices.to(torch.int32) for s in systems])
+        self.w = torch.cat([s.W.data.float() for s in systems])
+        B = len(systems)
+        offs = np.zeros(2 * (B + 1), dtype=np.int32)
+        offs[: B + 1] = self.offsets
+        offs[B + 2:] = np.cumsum(nnzs)
+        offs = torch.from_numpy(offs).to(dev)
+        _lib.call("dlp_batch_offsets", B, ptr(offs), ptr(offs[B + 1:]), N, self.nnz, ptr(self.indptr), ptr(self.col),
+                  stream())
         s64 = [s.astype(torch.float64) for s in systems]
-        self.diag = torch.cat([s.diag for s in s64]).to(dtype).contiguous()
-        rhs = torch.cat([torch.cat([s.rhs, s.diag[:, None]], 1) if with_h else s.rhs for s in s64])
-        self.rhs = rhs.to(dtype).contiguous()
+        self.diag64 = torch.cat([s.diag for s in s64])
+        self.diag = self.diag64.to(dtype)
+        self.rhs64 = torch.cat([self._rhs(s, with_h) for s in s64])
+        self.rhs = self.rhs64.to(dtype)
         self.set_tiles(tile_rows)
 
+    @staticmethod
+    def _rhs(s, with_h):
+        if not with_h:
+            return s.rhs
+        return s.rhs_h if s.rhs_h is not None else torch.cat([s.rhs, s.diag[:, None]], 1)
+
     def set_tiles(self, tile_rows):
+        """Cut every instance into tiles of up to tile_rows rows, fewer for small instances (at most some 128
+        tiles each, at least 128 rows): the batch then has enough tiles to fill the chip, and the cut depends
+        on the instance alone, so it gets the same sums in every batch."""
         self.tile_rows = tile_rows
-        tinst, tbeg, tend, toff = [], [], [], [0]
-        for i, (a, b) in enumerate(zip(self.offsets[:-1], self.offsets[1:])):
-            starts = np.arange(a, b, tile_rows) if b > a else np.zeros(0, dtype=np.int64)
-            tinst.append(np.full(starts.shape[0], i, dtype=np.int32))
-            tbeg.append(starts)
-            tend.append(np.minimum(starts + tile_rows, b))
-            toff.append(toff[-1] + starts.shape[0])
-        dev = self.dev
-        self.tinst = torch.from_numpy(np.concatenate(tinst).astype(np.int32)).to(dev)
-        self.tbeg = torch.from_numpy(np.concatenate(tbeg).astype(np.int32)).to(dev)
-        self.tend = torch.from_numpy(np.concatenate(tend).astype(np.int32)).to(dev)
-        self.toff = torch.tensor(toff, dtype=torch.int32, device=dev)
-        self.ntiles = int(self.tinst.numel())
+        sizes = np.diff(self.offsets)
+        tr = np.full(sizes.shape[0], int(tile_rows), dtype=np.int64)
+        want = np.maximum(128, 2 ** np.ceil(np.log2(np.maximum(sizes, 1) / 128.0)).astype(np.int64).clip(0, 62))
+        tr = np.minimum(tr, want)
+        count = -(-sizes // tr)
+        toff = np.concatenate([[0], np.cumsum(count)])
+        inst = np.repeat(np.arange(sizes.shape[0]), count)
+        beg = self.offsets[inst] + (np.arange(inst.shape[0]) - toff[inst]) * tr[inst]
+        end = np.minimum(beg + tr[inst], self.offsets[inst + 1])
+        self.ntiles = int(inst.shape[0])
+        m = max(self.ntiles, 1)
+        host = np.zeros(3 * m + toff.shape[0], dtype=np.int32)  # one upload for the four arrays
+        host[: self.ntiles], host[m: m + self.ntiles], host[2 * m: 2 * m + self.ntiles] = inst, beg, end
+        host[3 * m:] = toff
+        t = torch.from_numpy(host).to(self.dev)
+        self.tinst, self.tbeg, self.tend, self.toff = t[: self.ntiles], t[m: m + self.ntiles], t[2 * m: 2 * m + self.ntiles], t[3 * m:]
+
+    def col_stats(self, X):
+        """(sums of squares, largest magnitudes) per instance and column of X (N x C), device B x C each."""
+        B, C = len(self.systems), X.shape[1]
+        out = torch.empty((B, 2, C), dtype=torch.float64, device=self.dev)
+        ws = workspace("batch_stats").get(_lib.lib().dlp_batch_colstats_workspace_bytes(self.ntiles, C))
+        _lib.call("dlp_batch_colstats", C, ptr(X), ld(X), code(X), B, self.ntiles, ptr(self.tinst), ptr(self.tbeg),
+                  ptr(self.tend), ptr(self.toff), ptr(out), ptr(ws), ws.numel(), stream())
+        return out
+
+    def scale_rows(self, mode, X, scale, Y):
+        """mode 0: Y = X / scale (fp32 of fp64); mode 1: Y += X * scale; scale per instance and column, zero: untouched."""
+        _lib.call("dlp_batch_scale", mode, X.shape[1], ptr(X), ld(X), ptr(scale), ptr(Y), ld(Y), len(self.systems), self.ntiles,
+                  ptr(self.tinst), ptr(self.tbeg), ptr(self.tend), stream())
 
     def csr(self) -> CSR:
         return CSR(self.w, self.col, self.indptr, (self.N, self.N))
@@ -111,16 +137,11 @@ class BatchedSystems:
         Z = padded_empty(N, Ch, dt, dev)
         if Z0 is not None:
             Z.copy_(Z0)
-        else:
-            Z.zero_()
         R = torch.empty((N, Ch), dtype=dt, device=dev)
         P = padded_empty(N, Ch, dt, dev, 0.0)
-        AP = torch.empty((N, Ch), dtype=dt, device=dev)
+        AP = padded_empty(N, Ch, dt, dev)  # rows padded like P's: the apply writes them whole
         # per-instance column norms of the right-hand side (fp64); the h column only needs a loose solve
-        rn = torch.empty((B, Ch), dtype=torch.float64, device=dev)
-        for i, (a, b) in enumerate(zip(self.offsets[:-1], self.offsets[1:])):
-            rn[i] = kernels.colreduce(2, self.rhs[a:b]).sqrt() if b > a else torch.ones(Ch, dtype=torch.float64,
-                                                                                        device=dev)
+        rn = self.col_stats(self.rhs)[:, 0].sqrt()
         if Ch > self.C:
             rn[:, self.C:] *= 1e3
         rn = torch.where(rn > 0, rn, torch.ones_like(rn))
@@ -128,10 +149,10 @@ class BatchedSystems:
             t = torch.as_tensor(np.asarray(inst_targets, dtype=np.float64) / target_relres, device=dev)
             rn = rn * t[:, None]
         rn = rn.contiguous()
-        mode = 2
+        mode = 2 if Z0 is not None else 6  # from zero: no residual to compute
         epsd = torch.full((B, Ch), 1e300, dtype=torch.float64, device=dev)
         if eps is not None:
-            mode = 3
+            mode |= 1
             epsd[:] = torch.as_tensor(eps, dtype=torch.float64, device=dev)
         ws = workspace("batched").get(_lib.lib().dlp_pcg_batched_workspace_bytes(B, self.ntiles, Ch))
         iters = (ct.c_int32 * B)()
@@ -189,42 +210,37 @@ def solve_many_mixed(systems, target_relres=1e-6, tile_rows=1024, rounds=6, auto
         bs = BatchedSystems(group, tile_rows=tile_rows, dtype=torch.float32)
         if autotune:
             bs.autotune()
-        dev, N, Ch = bs.dev, bs.N, bs.Ch
-        s64 = [s.astype(torch.float64) for s in group]
-        diag64 = torch.cat([s.diag for s in s64]).contiguous()
-        rhs64 = torch.cat([torch.cat([s.rhs, s.diag[:, None]], 1) for s in s64]).contiguous()
+        dev, N, Ch, B = bs.dev, bs.N, bs.Ch, len(group)
+        diag64, rhs64 = bs.diag64, bs.rhs64
         A = CSR(bs.w, bs.col, bs.indptr, (N, N))
         spans = list(zip(bs.offsets[:-1], bs.offsets[1:]))
-        ones = torch.ones(C, dtype=torch.float64, device=dev)
-        rhs_n = [kernels.colreduce(2, rhs64[a:b, :C]).sqrt() if b > a else ones for a, b in spans]
+        rhs_n = bs.col_stats(rhs64)[:, 0, :C].sqrt()
+        rhs_n = torch.where(rhs_n > 0, rhs_n, torch.ones_like(rhs_n))
         Z64 = padded_empty(N, Ch, torch.float64, dev, 0.0)
         # the fp32 solves aim no lower than `inner`: below their precision floor (about 1e-6 of
         # ||rhs|| on these systems, lower for some) a solve only stalls until its patience runs out
         Zf, it, _, _ = bs.solve(target_relres=max(target_relres, inner))
-        Z64 += Zf.double()
+        Z64.copy_(Zf)
         iters = it.astype(np.int64)
-        rel = np.zeros(len(group))
+        rel = np.zeros(B)
+        rhs32 = torch.empty((N, Ch), dtype=torch.float32, device=dev)
         for rnd in range(rounds + 1):
-            R64 = kernels.spmm_axpy(A, Z64, a=diag64, alpha=-1.0, b=1.0, rhs=rhs64)
-            rn = [kernels.colreduce(2, R64[a:b, :C]).sqrt() if b > a else 0 * ones for a, b in spans]
-            rel = np.array([float((r / torch.where(h > 0, h, torch.ones_like(h))).max()) for r, h in zip(rn, rhs_n)])
+            R64 = kernels.spmm_axpy(A, Z64, a=diag64, alpha=-1.0, b=1.0, rhs=rhs64, out=padded_empty(N, Ch, torch.float64, dev))
+            st = bs.col_stats(R64)
+            rel_d = (st[:, 0, :C].sqrt() / rhs_n).amax(dim=1)
+            rel = rel_d.cpu().numpy()
             if (rel <= target_relres).all() or rnd == rounds:
                 break
-            scales, rhs32 = [], torch.empty((N, Ch), dtype=torch.float32, device=dev)
-            for a, b in spans:
-                sc = kernels.colreduce(3, R64[a:b]) if b > a else torch.ones(Ch, dtype=torch.float64, device=dev)
-                sc = torch.where(sc > 0, sc, torch.ones_like(sc))
-                rhs32[a:b] = (R64[a:b] / sc[None, :]).float()
-                scales.append(sc)
+            sc = torch.where(st[:, 1] > 0, st[:, 1], torch.ones_like(st[:, 1])).contiguous()
+            bs.scale_rows(0, R64, sc, rhs32)
             bs.rhs = rhs32
             # each instance's correction brings its residual to a fifth of the target, or by `inner`
             # when that is further than one fp32 solve safely resolves (another round follows)
             need = [max(0.2 * target_relres / max(r, 1e-300), inner) for r in rel]
             D, it2, _, _ = bs.solve(target_relres=target_relres, inst_targets=need)
-            for k, ((a, b), sc) in enumerate(zip(spans, scales)):
-                if rel[k] > target_relres:  # a converged instance keeps its scores (same as alone)
-                    Z64[a:b] += D[a:b].double() * sc[None, :]
-                    iters[k] += it2[k]
+            # a converged instance keeps its scores (same as alone)
+            bs.scale_rows(1, D, torch.where(rel_d[:, None] > target_relres, sc, torch.zeros_like(sc)).contiguous(), Z64)
+            iters += np.where(rel > target_relres, it2, 0)
         for k, j in enumerate(idx):
             a, b = spans[k]
             out[j] = Z64[a:b, :C]

@@ -615,12 +615,28 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
 
 
 /* The inverse of a dense symmetric positive definite fp64 matrix A (n x n, row-major), in place:
- * Gauss-Jordan elimination without pivoting, two launches per pivot (the coarsest AMG level's solve,
- * dynlp/amg.py:105-108 inverts it with the library's LU). Asynchronous.
+ * Gauss-Jordan elimination without pivoting (the coarsest AMG level's solve, dynlp/amg.py:105-108
+ * inverts it with the library's LU): one cooperative launch that keeps the rows in shared memory up to
+ * some 1,900 rows (synchronises the stream), two launches per pivot beyond.
  * Workspace: dlp_dense_spd_inverse_workspace_bytes(n). */
 size_t dlp_dense_spd_inverse_workspace_bytes(int32_t n);
 int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_stream_t stream);
 
+
+/* ---- the vectors of a batch of systems (concatenated; tiles as below) -------------------------
+ * offsets: CSRs concatenated as they are (indptr: a zero, then each one's row ends) become one block-diagonal
+ * CSR in place; row_off / nnz_off: device, each instance's first row / entry. colstats: out[i] = the
+ * instance's C column sums of squares, then its C largest magnitudes (fp64, fixed order). scale: mode 0
+ * Y (f32) = X (f64) / scale, mode 1 Y (f64) += X (f32) * scale, scale ninst x C, rows of a zero untouched. */
+int dlp_batch_offsets(int32_t ninst, const int32_t *row_off, const int32_t *nnz_off, int32_t N, int64_t nnz,
+                      int32_t *indptr, int32_t *col, dlp_stream_t stream);
+size_t dlp_batch_colstats_workspace_bytes(int32_t ntiles, int32_t C);
+int dlp_batch_colstats(int32_t C, const void *X, int64_t ldx, int dtype, int32_t ninst, int32_t ntiles,
+                       const int32_t *tile_inst, const int32_t *tile_beg, const int32_t *tile_end,
+                       const int32_t *inst_tiles, double *out, void *ws, size_t ws_bytes, dlp_stream_t stream);
+int dlp_batch_scale(int32_t mode, int32_t C, const void *X, int64_t ldx, const double *scale, void *Y, int64_t ldy,
+                    int32_t ninst, int32_t ntiles, const int32_t *tile_inst, const int32_t *tile_beg,
+                    const int32_t *tile_end, dlp_stream_t stream);
 
 /* ---- batched independent solves (config: many instances in one launch sequence) -------------
  * No reference counterpart (the reference solves one system at a time). Block PCG with the Jacobi
@@ -630,8 +646,9 @@ int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_s
  * and instance i owns tiles [inst_tiles[i], inst_tiles[i+1]) (inst_tiles has ninst + 1 entries).
  * Every instance runs its own CG (its own alpha, beta and stop state; reductions per instance in
  * a fixed tile order, so an instance gets the iterates it would get alone) until the stop rule
- * `mode` (as in dlp_pcg; eps_dev and rhs_norm_dev are DEVICE arrays of ninst x C doubles) holds,
- * confirmed on its true residual. Synchronous: per-instance iterations, status (5 converged,
+ * `mode` (bits 0 and 1 as in dlp_pcg; eps_dev and rhs_norm_dev are DEVICE arrays of ninst x C doubles;
+ * bit 2: every solve starts from Z = 0, whatever Z holds) holds, confirmed on its true residual. The host
+ * queues check_every iterations between reads (use_graph is accepted and has no effect). Synchronous: per-instance iterations, status (5 converged,
  * 2 stalled, 3 cap, 4 breakdown) and relative residuals are written to HOST arrays of ninst. */
 size_t dlp_pcg_batched_workspace_bytes(int32_t ninst, int32_t ntiles, int32_t C);
 int dlp_pcg_batched(const int32_t *indptr, const int32_t *col, const float *w, int32_t N, int32_t C, const void *diag,

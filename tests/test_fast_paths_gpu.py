@@ -372,3 +372,28 @@ def test_built_system_equals_the_oracle(n, K, dtype, wdtype, eta):
     with pytest.raises(IndexError):
         stream.build_system(graphs.Dataset("x", ds.A, bad, K, ds.order), torch.as_tensor(active).cuda(),
                             torch.as_tensor(lab).cuda(), dtype=dtype)
+
+
+@pytest.mark.parametrize("K,dtype", [(2, "float64"), (4, "float64"), (8, "float64"), (4, "float32"), (8, "float32"),
+                                     (16, "float64")])
+def test_uneven_batch_equals_each_system_alone(K, dtype):
+    """Systems of very different sizes in one batch: bit for bit the scores, iterations and status each has
+    alone, the target met on the fp64 residual (or the precision's floor), from zero and from a start."""
+    from dynlplus_b200 import batched
+    dt = getattr(torch, dtype)
+    systems = [grounded(n, K, seed=n, deg=(6, 4))[2] for n in (60, 127, 130, 1000, 5000, 20_000)]
+    target = 1e-8 if dt == torch.float64 else 1e-4
+    for start in (False, True):
+        bs = batched.BatchedSystems(systems, dtype=dt)
+        Z0 = torch.full((bs.N, bs.Ch), 0.3, dtype=dt, device="cuda") if start else None
+        Z, it, status, rel = bs.solve(target_relres=target, Z0=Z0)
+        assert (status == 5).all() and (rel <= target).all()
+        for k, s in enumerate(systems):
+            one = batched.BatchedSystems([s], dtype=dt)
+            a, b = bs.offsets[k], bs.offsets[k + 1]
+            Z1, it1, st1, rel1 = one.solve(target_relres=target, Z0=Z0[a:b] if start else None)
+            assert torch.equal(Z[a:b], Z1) and it[k] == it1[0] and rel[k] == rel1[0]
+            S64 = s.astype(torch.float64)
+            R = solvers.residual(S64, Z[a:b, : s.C].double().contiguous(), S64.rhs.contiguous())
+            bn = S64.rhs.norm(dim=0)  # a zero right-hand side (a class without a label) counts as one, as in the solver
+            assert bool((R.norm(dim=0) <= 1.01 * target * torch.where(bn > 0, bn, torch.ones_like(bn))).all())
