@@ -121,17 +121,19 @@ __global__ void __launch_bounds__(kAT) k_sort_members(int32_t nc, const int32_t 
   if (lane < L) members[b + rank] = x;
 }
 
-// The aggregates of more than `more` members among this block's share (blockDim.x at a time), one after
+// The aggregates of more than `more` members among this block's share (at most kAT at a time), one after
 // another: fn(a) is called by the whole block.
 template <class Fn>
 __device__ __forceinline__ void for_long_aggregates(int32_t nc, const int32_t *off, int more, Fn fn) {
   __shared__ int32_t s_list[kAT];
   __shared__ int s_n;
-  for (long long a0 = (long long)blockIdx.x * kAT; a0 < nc; a0 += (long long)gridDim.x * kAT) {
+  // equal shares of at most kAT: the few long aggregates of a coarse level go to as many blocks
+  const int per = min(kAT, (int)((nc + gridDim.x - 1) / gridDim.x));
+  for (long long a0 = (long long)blockIdx.x * per; a0 < nc; a0 += (long long)gridDim.x * per) {
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     const long long a = a0 + threadIdx.x;
-    if (a < nc && off[a + 1] - off[a] > more) s_list[atomicAdd(&s_n, 1)] = (int32_t)a;
+    if ((int)threadIdx.x < per && a < nc && off[a + 1] - off[a] > more) s_list[atomicAdd(&s_n, 1)] = (int32_t)a;
     __syncthreads();
     const int m = s_n;
     for (int i = 0; i < m; ++i) fn(s_list[i]);
@@ -199,7 +201,7 @@ static int sort_members(int32_t n, int32_t nc, const int32_t *off, int32_t *memb
                                          v) == cudaSuccess ? (size_t)v : (size_t)0;
   }();
   if (bits <= most)
-    k_sort_members_long<<<std::min(sm_count(), g1(nc)), kAT, bits, s>>>(n, nc, off, members);
+    k_sort_members_long<<<std::min(sm_count(), nc), kAT, bits, s>>>(n, nc, off, members);
   else
     k_sort_members_serial<<<g1(nc), kAT, 0, s>>>(nc, off, members);
   return check_launch();
@@ -364,11 +366,13 @@ __global__ void k_run_emit(long long m, const long long *__restrict__ key, const
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
     if (lane == src) acc += part;
   }
+  const int32_t a = mine ? (int32_t)(k / nc) : -1;
+  const unsigned row = __match_any_sync(0xffffffffu, a);
   if (!mine) return;
-  const int32_t a = (int32_t)(k / nc);
   col_c[pos[i]] = (int32_t)(k - (long long)a * nc);
   w_c[pos[i]] = (float)acc;
-  atomicAdd(rowcnt + a, 1);
+  // keys are sorted, so a warp's runs lie in few rows: one count per row and warp
+  if (lane == __ffs(row) - 1) atomicAdd(rowcnt + a, __popc(row));
 }
 
 // s_c[a] = sum of s over the members of aggregate a, in member order
@@ -406,11 +410,11 @@ __global__ void k_restrict(int32_t nc, int32_t C, const int32_t *__restrict__ of
   Rc[a * ldc + c] = s;
 }
 
-// The aggregates of more than kShortSum members: the block brings tiles of member rows to shared memory (all
-// rows of a tile in flight) and one thread per column adds them in member order, as k_restrict does, up to
-// 64 columns a pass. The longest list in one thread's dependent loads bounded the restriction (the
-// 120,000-row hierarchy, 51 launches: 1,390 us).
-constexpr int kSumTile = 4096;
+// The aggregates of more than kShortSum members: the block brings tiles of member rows to shared memory and
+// one thread per column adds them in member order, as k_restrict does, up to 64 columns a pass. The longest
+// list in dependent loads bounds the launch, so a thread keeps kSumFly members' rows in flight, the next
+// tile's while the column threads add this one's, sixteen values at a time.
+constexpr int kSumTile = 4096, kSumFly = kSumTile / kAT;
 template <typename T>
 __global__ void __launch_bounds__(kAT) k_restrict_long(int32_t nc, int32_t C, const int32_t *__restrict__ off,
                                                        const int32_t *__restrict__ members, const T *__restrict__ R,
@@ -420,18 +424,46 @@ __global__ void __launch_bounds__(kAT) k_restrict_long(int32_t nc, int32_t C, co
   for_long_aggregates(nc, off, kShortSum, [&](int32_t a) {
     const int b = off[a], e = off[a + 1];
     for (int c0 = 0; c0 < C; c0 += 64) {
+      // value t of a tile: column t % cw of its member t / cw; a thread's values lie kAT apart, so its member
+      // and column advance by fixed steps
       const int cw = min(64, C - c0), tile = kSumTile / cw;
-      T s = T(0);
-      for (int i0 = b; i0 < e; i0 += tile) {
-        const int m = min(tile, e - i0) * cw;
-        for (int t = tid; t < m; t += kAT) {
-          const int i = t / cw;
-          s_row[t] = R[(long long)members[i0 + i] * ldr + c0 + (t - i * cw)];
+      const int di = kAT / cw, dc = kAT - di * cw, i_first = tid / cw, c_first = tid - i_first * cw;
+      T s = T(0), v[kSumFly];
+      auto fetch = [&](int i0) {
+        const int rows = min(tile, e - i0);
+        int i = i_first, c = c_first, at[kSumFly];
+#pragma unroll
+        for (int u = 0; u < kSumFly; ++u) {
+          at[u] = i < rows ? members[i0 + i] : -1;
+          i += di;
+          c += dc;
+          if (c >= cw) { c -= cw; ++i; }
         }
+        c = c_first;
+#pragma unroll
+        for (int u = 0; u < kSumFly; ++u) {
+          v[u] = at[u] >= 0 ? R[(long long)at[u] * ldr + c0 + c] : T(0);
+          c += dc;
+          if (c >= cw) c -= cw;
+        }
+      };
+      fetch(b);
+      for (int i0 = b; i0 < e; i0 += tile) {
+#pragma unroll
+        for (int u = 0; u < kSumFly; ++u) s_row[u * kAT + tid] = v[u];
         __syncthreads();
+        if (i0 + tile < e) fetch(i0 + tile);
         if (tid < cw) {
-#pragma unroll 8
-          for (int t = tid; t < m; t += cw) s += s_row[t];
+          const int rows = min(tile, e - i0);
+          int i = 0;
+          for (; i + 16 <= rows; i += 16) {
+            T q[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) q[u] = s_row[(i + u) * cw + tid];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) s += q[u];
+          }
+          for (; i < rows; ++i) s += s_row[i * cw + tid];
         }
         __syncthreads();
       }
@@ -626,7 +658,7 @@ int dlp_amg_restrict(int32_t nc, int32_t C, const int32_t *off, const int32_t *m
   if (nc == 0) return DLP_OK;
   cudaStream_t s = (cudaStream_t)stream;
   const long long t = (long long)nc * C;
-  const int gl = std::min(2 * sm_count(), g1(nc));
+  const int gl = std::min(2 * sm_count(), nc);
   if (dtype == DLP_F32) {
     k_restrict<float><<<g1(t), kAT, 0, s>>>(nc, C, off, members, (const float *)R, ldr, (float *)Rc, ldc);
     k_restrict_long<float><<<gl, kAT, 0, s>>>(nc, C, off, members, (const float *)R, ldr, (float *)Rc, ldc);

@@ -174,9 +174,9 @@ int exclusive_scan_i32(const int32_t *in, int32_t n, int32_t *out, void *ws, siz
 // Stable LSD radix sort of (int64 key, fp64 value) pairs, 8 bits per pass (the AMG coarsening's
 // sort by coarse entry). Keys above max_key order as max_key (the "no entry" marker sorts last).
 // Per pass: tile histograms stored digit-major, one exclusive scan of them (each (digit, tile) gets
-// its first output slot), then a stable scatter: a tile is taken in chunks of 256 elements in input
-// order; inside a chunk equal digits are ranked by __match_any_sync per warp and per-warp counts in
-// shared memory, and a running count per digit carries over to the next chunk.
+// its first output slot), then a stable scatter: each warp ranks its own run of the tile against its
+// running digit counts (__match_any_sync, no block barrier), the tile is put in digit order in shared
+// memory and leaves it in runs of neighbouring addresses. Its bound is the 32 bytes an entry moves.
 // ------------------------------------------------------------------------------------------------
 constexpr int kRsItems = 8;
 constexpr int kRsTile = kScanThreads * kRsItems;
@@ -204,45 +204,74 @@ __global__ void __launch_bounds__(kScanThreads) k_rs_hist(long long m, const lon
 __global__ void __launch_bounds__(kScanThreads)
     k_rs_scatter(long long m, const long long *__restrict__ keys, const double *__restrict__ vals, long long maxk,
                  int shift, const int32_t *__restrict__ offs, int ntiles, long long *keys_out, double *vals_out) {
-  __shared__ int32_t s_base[256];
-  __shared__ int32_t s_cnt[kScanThreads / 32][256];
+  constexpr int kWarps = kScanThreads / 32;
+  static_assert(kScanThreads == 256, "one thread per digit");
+  __shared__ int32_t s_cnt[kWarps][256];  // digits of a warp's run so far; then its first place in the tile
+  __shared__ int32_t s_out[256], s_warp[kWarps];
+  __shared__ long long s_key[kRsTile];
+  __shared__ double s_val[kRsTile];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  s_base[tid] = offs[(long long)tid * ntiles + blockIdx.x];
-#pragma unroll
-  for (int w = 0; w < kScanThreads / 32; ++w) s_cnt[w][tid] = 0;
-  __syncthreads();
   const long long base = (long long)blockIdx.x * kRsTile;
-  for (int i = 0; i < kRsItems; ++i) {
-    const long long e = base + (long long)i * kScanThreads + tid;
-    const bool valid = e < m;
-    long long k = 0;
-    double v = 0.0;
-    int d = 256;  // no digit: past the end
-    if (valid) {
-      k = keys[e];
-      v = vals[e];
-      d = rs_digit(k, maxk, shift);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int wrank = __popc(peers & ((1u << lane) - 1u));
-    if (valid && wrank == 0) s_cnt[wid][d] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      int pre = 0;
-      for (int w = 0; w < wid; ++w) pre += s_cnt[w][d];
-      const int dest = s_base[d] + pre + wrank;
-      keys_out[dest] = k;
-      vals_out[dest] = v;
-    }
-    __syncthreads();
-    int tot = 0;
+  const int count = (int)min((long long)kRsTile, m - base);
+  const int at = wid * 32 * kRsItems + lane;
+  long long k[kRsItems];
+  double v[kRsItems];
+  int rank[kRsItems];
 #pragma unroll
-    for (int w = 0; w < kScanThreads / 32; ++w) {
-      tot += s_cnt[w][tid];
-      s_cnt[w][tid] = 0;
+  for (int u = 0; u < kRsItems; ++u) {
+    const int e = at + 32 * u;
+    k[u] = e < count ? keys[base + e] : 0;
+    v[u] = e < count ? vals[base + e] : 0.0;
+  }
+  for (int d = lane; d < 256; d += 32) s_cnt[wid][d] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < kRsItems; ++u) {
+    const bool valid = at + 32 * u < count;
+    const int d = valid ? rs_digit(k[u], maxk, shift) : 256;  // 256: past the end
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const int before = __popc(peers & ((1u << lane) - 1u));
+    rank[u] = (valid ? s_cnt[wid][d] : 0) + before;
+    __syncwarp();
+    if (valid && before == 0) s_cnt[wid][d] += __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  int tot = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) tot += s_cnt[w][tid];
+  int incl = tot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  int first = incl - tot;
+  for (int w = 0; w < wid; ++w) first += s_warp[w];
+  s_out[tid] = offs[(long long)tid * ntiles + blockIdx.x] - first;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    const int t = s_cnt[w][tid];
+    s_cnt[w][tid] = first;
+    first += t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kRsItems; ++u) {
+    if (at + 32 * u < count) {
+      const int q = s_cnt[wid][rs_digit(k[u], maxk, shift)] + rank[u];
+      s_key[q] = k[u];
+      s_val[q] = v[u];
     }
-    s_base[tid] += tot;
-    __syncthreads();
+  }
+  __syncthreads();
+  for (int q = tid; q < count; q += kScanThreads) {
+    const long long kq = s_key[q];
+    const int dest = s_out[rs_digit(kq, maxk, shift)] + q;
+    keys_out[dest] = kq;
+    vals_out[dest] = s_val[q];
   }
 }
 
