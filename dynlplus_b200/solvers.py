@@ -841,16 +841,18 @@ class IncrementalLP(DynLPPlus):
         st.edges += s64.nnz
         self.since_full = 0
 
-    def _push(self, s64, eps, st):
-        """Repair the violating rows of R (dynlp/solvers.py:375-389): the fused asynchronous push
+    def _violating_rows(self, s64, eps):
+        eps_d = torch.as_tensor(eps, dtype=F64, device=self.Z.device)
+        return kernels.flatnonzero(kernels.violating(self.R, s64.diag, eps_d))
+
+    def _push(self, s64, eps, st, cand):
+        """Repair the violating rows `cand` of R (dynlp/solvers.py:375-389): the fused asynchronous push
         for up to 33 columns, the synchronous vectorised push beyond."""
         Z, R = self.Z, self.R
-        eps_d = torch.as_tensor(eps, dtype=F64, device=Z.device)
         if Z.shape[1] <= 33:
             if getattr(self, "_fused", None) is None or self._fused.W is not s64.W:
                 self._fused = kernels.FusedPush(s64.W, Z.shape[1], self.group)
-            cand = kernels.flatnonzero(kernels.violating(R, s64.diag, eps_d))
-            rounds, ok, edges = self._fused.run(Z, R, s64.diag, eps_d, cand, self.max_rounds)
+            rounds, ok, edges = self._fused.run(Z, R, s64.diag, eps, cand, self.max_rounds)
             st.iters, st.edges = st.iters + rounds, st.edges + edges
             return ok
         ops = FrontierOps(s64.W, Z.shape[1], self.group)
@@ -906,18 +908,18 @@ class IncrementalLP(DynLPPlus):
                     small = False
                     if self.target_relres is None and self.method in ("auto", "push"):
                         eps = [tol / (1.25 * (self.hmax or 1.0))] * C + [self.eps_h]
-                        eps_d = torch.as_tensor(eps, dtype=F64, device=self.Z.device)
-                        nviol = int(kernels.violating(self.R, s64.diag, eps_d).sum().item())
-                        small = nviol / max(s64.n_solved, 1) <= self.push_frac
+                        cand = self._violating_rows(s64, eps)
+                        small = cand.numel() / max(s64.n_solved, 1) <= self.push_frac
                     if small:
                         st.path = "inc-push"
                         for _ in range(4):
-                            ok = self._push(s64, eps, st)
+                            ok = self._push(s64, eps, st, cand)
                             rc2, _, _, h2 = residual_stats(s64, self.R, H=self.Z[:, C:])
                             hmax, bound = self._bound(rc2, h2)
                             if ok and bound <= tol:
                                 break
                             eps = [tol / (1.25 * hmax)] * C + [self.eps_h]
+                            cand = self._violating_rows(s64, eps)
                         rel = float("nan")
                         stats = None
                     if not (bound <= tol and small):

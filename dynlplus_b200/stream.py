@@ -49,6 +49,7 @@ class System:
     changed: object = None   # global-index systems: rows whose equation changed
     moved: object = None     # global-index systems: rows that entered or left U this batch
     rhs_h: object = None     # (n, C+1) [rhs | diag], the DynLP+ right-hand side with the h column
+    solved_count: object = None  # global-index systems: the number of solved rows, where it is known
     _conv: dict = field(default_factory=dict, repr=False, compare=False)
 
     n_u = property(lambda self: int(self.U.numel()))
@@ -56,7 +57,9 @@ class System:
 
     @property
     def n_solved(self) -> int:
-        return self.n_u if self.solved is None else int(self.solved.sum().item())
+        if self.solved is None:
+            return self.n_u
+        return int(self.solved.sum().item()) if self.solved_count is None else self.solved_count
 
     def label_cols(self, M):
         """Columns of a (., K) class matrix that are solved (class 1 if binary)."""
@@ -642,7 +645,7 @@ class EdgeStream:
             wd = G.data if self.dtype == torch.float32 else G.data.to(self.dtype)
             comps = new_components_rows(new, G.rbeg, G.rend, G.indices, wd, nl, tau, wmax, self.B[new].sum(dim=1))
         self._vertex_batch = {"is_new": is_new, "seed": seed, "comps": comps}
-        self._counts = None
+        self._counts = self._n_labeled = None
         return self.system
 
     def solver_csr(self) -> CSR:
@@ -687,6 +690,8 @@ class EdgeStream:
         if getattr(self, "_counts", None) is None:
             self._counts = torch.stack([self.vmask.sum() + self.labeled.sum(), (self.vmask.bool() & ~um).sum()]).tolist()
         n_active, n_ungrounded = self._counts
+        if getattr(self, "_n_labeled", None) is None:  # changes with vertex batches only
+            self._n_labeled = int(self.labeled.sum().item())
         vx = getattr(self, "_vertex_batch", None)
         common = dict(t=self.t, U=self._ids, W=self.solver_csr(),
                       is_new=vx["is_new"] if vx else self._no_new,
@@ -695,6 +700,7 @@ class EdgeStream:
                       eta=self.eta,
                       n_inserted=self.n_ins, n_deleted=self.n_del, n_active=int(n_active),
                       n_ungrounded=int(n_ungrounded), solved=um,
+                      solved_count=int(n_active) - self._n_labeled - int(n_ungrounded),
                       changed=self.last_changed, moved=self.last_moved)
         ch = C + (1 if self.with_h else 0)
         # the grounding stays fp64 in every precision (its one reader, the AMG setup, works in fp64)

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from dynlplus_b200 import graphs, solvers, stream
+from dynlplus_b200 import graphs, kernels, solvers, stream
 
 pytestmark = pytest.mark.gpu
 
@@ -397,3 +397,39 @@ def test_uneven_batch_equals_each_system_alone(K, dtype):
             R = solvers.residual(S64, Z[a:b, : s.C].double().contiguous(), S64.rhs.contiguous())
             bn = S64.rhs.norm(dim=0)  # a zero right-hand side (a class without a label) counts as one, as in the solver
             assert bool((R.norm(dim=0) <= 1.01 * target * torch.where(bn > 0, bn, torch.ones_like(bn))).all())
+
+
+@pytest.mark.parametrize("dt", ["float32", "float64"])
+@pytest.mark.parametrize("C", [1, 4, 5, 8, 9, 16, 17, 32, 33])
+def test_push_in_one_launch_equals_the_launched_rounds(C, dt):
+    """One cooperative launch against the rounds launched by the host. fp64: the same frontiers (rounds and
+    edge visits), Z and R equal up to the order of the atomic sums. Both types: R stays the residual of Z, no
+    row violates at the end, and columns beyond C keep their values."""
+    n, tdt = 3001, getattr(torch, dt)
+    ds = graphs.er_graph(n, 11, 4, seed=C)
+    es = stream.EdgeStream(ds, graphs.label_mask(n, 0.05, seed=C), dtype="float32")
+    S = es.system.astype(torch.float64)
+    W, diag = es.G, S.diag.to(tdt)
+    g = torch.Generator().manual_seed(C)
+    base = (torch.rand((n, C), generator=g, dtype=torch.float64).to("cuda") * S.solved[:, None]).to(tdt)
+    eps = [1e-2] * C
+    cand = torch.nonzero(S.solved).flatten().to(torch.int32)
+    out = []
+    for whole in (True, False):
+        Z, R = torch.zeros((n, C + 3), dtype=tdt, device="cuda"), torch.full((n, C + 3), 7.0, dtype=tdt, device="cuda")
+        R[:, :C] = base
+        rounds, ok, edges = kernels.FusedPush(W, C).run(Z[:, :C], R[:, :C], diag, eps, cand, 10_000, use_graph=whole)
+        assert ok and float((R[:, C:] - 7.0).abs().max()) == 0.0 and float(Z[:, C:].abs().max()) == 0.0
+        z, x = Z[:, :C].double().contiguous(), R[:, :C].double()
+        assert bool((x.abs() <= eps[0] * diag.double()[:, None] * (1 + 1e-6)).all())
+        # a value of R takes at most one rounded add per round and entry of its row (degree < 64), each of a
+        # residual no larger than diag * max Z; Z one per round
+        u = 2.0 ** (-24 if dt == "float32" else -53)
+        lim = u * 66 * rounds * float(diag.max()) * max(float(z.abs().max()), 1.0)
+        true = base.double() - kernels.spmm_axpy(W, z, a=S.diag, b=-1.0)
+        assert float((true - x).abs().max()) <= lim
+        out.append((rounds, edges, z, x, lim))
+    (r0, e0, z0, x0, lim), (r1, e1, z1, x1, _) = out
+    if dt == "float64":
+        assert (r0, e0) == (r1, e1)
+        assert float((x0 - x1).abs().max()) <= 2 * lim and float((z0 - z1).abs().max()) <= 2 * lim
