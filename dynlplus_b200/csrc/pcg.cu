@@ -1817,7 +1817,11 @@ int dlp_residual_stats(int32_t n, int32_t C, const void *R, int64_t ldr, const v
   cudaStream_t s = (cudaStream_t)stream;
   static const int per32 = resident_per_sm(k_resid_stats<float>, kSweepThreads);
   static const int per64 = resident_per_sm(k_resid_stats<double>, kSweepThreads);
-  const int nb = sm_count() * (dtype == DLP_F32 ? per32 : per64);  // one wave, <= upd_blocks()
+  // one wave (<= upd_blocks()), and no more blocks than have kSweepUnroll values for each thread: the final
+  // reduction reads every block's
+  const long long most = std::max(((long long)n * ldr + kSweepThreads * kSweepUnroll - 1) / (kSweepThreads * kSweepUnroll),
+                                  (long long)((ldr + kSweepThreads - 1) / kSweepThreads));
+  const int nb = (int)std::min((long long)sm_count() * (dtype == DLP_F32 ? per32 : per64), most);
   double *part = (double *)ws;
   auto rows10 = [](const void *a, int64_t lda) { return (uintptr_t)a % 16 == 0 && lda >= 10 && lda % 2 == 0; };
   int nbu = nb;
@@ -1825,7 +1829,8 @@ int dlp_residual_stats(int32_t n, int32_t C, const void *R, int64_t ldr, const v
     // whole fp64 rows, one per thread (the decision rests on R alone, so calls with and without rhs
     // sum R in the same order)
     static const int per_rows = resident_per_sm(k_resid_stats_rows10, kSweepThreads);
-    nbu = std::min(sm_count() * per_rows, nb);
+    nbu = (int)std::min((long long)std::min(sm_count() * per_rows, nb),
+                        std::max(1LL, ((long long)n + kSweepThreads - 1) / kSweepThreads));
     k_resid_stats_rows10<<<nbu, kSweepThreads, 0, s>>>(n, C, (const double *)R, ldr, (const double *)rhs, ldrhs,
                                                         (const double *)diag, (const double *)H, ldh, part);
   } else if (dtype == DLP_F32) {

@@ -133,7 +133,18 @@ class FrontierOps:
         self.gs = _group(W, group)
         self.real = torch.float64 if W.data.dtype == torch.float64 else torch.float32
         self.use_kernel = True  # there is no fallback: the kernels are the implementation
-        self.edges = torch.zeros((), dtype=torch.int64, device=W.indices.device)  # device edge-visit counter
+        self._edges = None
+
+    @property
+    def edges(self):
+        """Device edge-visit counter (made when first asked for)."""
+        if self._edges is None:
+            self._edges = torch.zeros((), dtype=torch.int64, device=self.W.indices.device)
+        return self._edges
+
+    @edges.setter
+    def edges(self, value):
+        self._edges = value
 
     def _rows(self, rows):
         rbeg, rend = _rows_of(self.W)

@@ -130,7 +130,7 @@ def residual_stats(sys: System, R, rhs=None, H=None):
     (dynlp/solvers.py:52-54, :295-301)."""
     n, C = R.shape
     dt = R.dtype
-    out = torch.zeros(3 * C + 1, dtype=F64, device=R.device)
+    out = (torch.empty if n else torch.zeros)(3 * C + 1, dtype=F64, device=R.device)  # written whole
     if n:
         if rhs is not None:
             rhs = rhs.to(dt)
@@ -682,7 +682,7 @@ class DynLPPlus(Solver):
             scale = [r if r > 0 else 1.0 for r in rc]
             dv = getattr(stats, "dev", None)
             if dv is not None and dv.device == dev and dv.numel() >= C + 1:
-                sc = torch.where(dv[: C + 1] > 0, dv[: C + 1], torch.ones_like(dv[: C + 1]))  # = scale, on device
+                sc = dv[: C + 1] if all(r > 0 for r in rc) else torch.where(dv[: C + 1] > 0, dv[: C + 1], torch.ones_like(dv[: C + 1]))  # = scale, on device
             else:
                 sc = torch.tensor(scale, dtype=F64, device=dev)
             eps_c = [min(max(e / s, self._floor(h_est)), 1.0) for e, s in
