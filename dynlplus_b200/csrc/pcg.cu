@@ -665,6 +665,97 @@ __global__ void __launch_bounds__(kSweepThreads, (sweep_min_blocks<T>())) k_pcg_
     finish_sweep(phase, C, B, false);
 }
 
+// K2 on fp32 rows of a multiple of four columns, four columns a thread: one 16-byte load per array and the
+// diagonal's fp64 reciprocal once per four values, whose cost per value bounded the scalar form (n = 250,000,
+// 32 columns: 38.6 -> 28.6 us, of which the 96 MB are 15 and the last block's decision most of the rest; two or
+// four rows in flight, three or four blocks per SM: the same). The threads' columns repeat every C / 4.
+template <int U>
+__global__ void __launch_bounds__(kSweepThreads, 3)
+    k_pcg_update_v4(int phase, int32_t n, int32_t C, float *__restrict__ R, int64_t ldr, const float *__restrict__ AP,
+                    int64_t ldap, const float *__restrict__ diag, PcgBufs B) {
+  PcgCtl *ctl = B.ctl;
+  if (phase == 0 && !ctl->go) {
+    if (B.has_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(B.cond, 0u);  // loop ends
+    return;
+  }
+  if (B.has_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(B.cond, 0u);
+  __shared__ double s_rz[4][kSweepThreads], s_ss[4][kSweepThreads], s_v[kSweepThreads / 32];
+  const int NV = C / 4;
+  const SweepIdx ix = sweep_index(NV, NV);
+  double rz[4] = {0.0, 0.0, 0.0, 0.0}, ss[4] = {0.0, 0.0, 0.0, 0.0}, rmax[4] = {0.0, 0.0, 0.0, 0.0}, vmax = 0.0;
+  if (ix.on) {
+    const int c0 = ix.c * 4;
+    float al[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) al[i] = phase == 0 ? (float)B.alpha[c0 + i] : 0.f;
+    for (long long r = ix.r0; r < n; r += U * ix.RS) {
+      float4 rv[U], av[U];
+      float dv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long q = r + u * ix.RS;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        rv[u] = q >= n ? zero : *reinterpret_cast<const float4 *>(phase == 3 ? AP + q * ldap + c0 : R + q * ldr + c0);
+        av[u] = q < n && phase == 0 ? *reinterpret_cast<const float4 *>(AP + q * ldap + c0) : zero;
+        dv[u] = q < n ? diag[q] : 1.f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long q = r + u * ix.RS;
+        if (q >= n) break;
+        float x[4] = {rv[u].x, rv[u].y, rv[u].z, rv[u].w};
+        const float y[4] = {av[u].x, av[u].y, av[u].z, av[u].w};
+        if (phase == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i] = x[i] - al[i] * y[i];
+        }
+        if (phase == 0 || phase == 3)
+          *reinterpret_cast<float4 *>(R + q * ldr + c0) = make_float4(x[0], x[1], x[2], x[3]);
+        const double dinv = __drcp_rn((double)dv[u]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double r64 = (double)x[i], r2 = r64 * r64;
+          rz[i] += r2 * dinv;
+          ss[i] += r2;
+          rmax[i] = fmax(rmax[i], fabs(r64) * dinv);
+        }
+      }
+    }
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bad |= !isfinite(ss[i]);
+      vmax = fmax(vmax, rmax[i] * B.epsinv[c0 + i]);
+    }
+    if (bad) ctl->bad = 1;
+  }
+  const int tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    s_rz[i][tid] = rz[i];
+    s_ss[i][tid] = ss[i];
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
+  if (lane == 0) s_v[wid] = vmax;
+  __syncthreads();
+  for (int c = wid; c < C; c += kSweepThreads / 32) {
+    const double a = block_column_sum(s_rz[c & 3], c >> 2, NV);
+    const double b = block_column_sum(s_ss[c & 3], c >> 2, NV);
+    if (lane == 0) {
+      B.part2[(long long)c * B.nbmax + blockIdx.x] = a;
+      B.part2[(long long)(C + c) * B.nbmax + blockIdx.x] = b;
+    }
+  }
+  if (tid == 0) {
+    double v = 0.0;
+    for (int w = 0; w < kSweepThreads / 32; ++w) v = fmax(v, s_v[w]);
+    B.part2[(long long)(2 * C) * B.nbmax + blockIdx.x] = v;
+  }
+  if (last_block_grouped<kSweepThreads>(B.part2, B.nbmax, 2 * C + 1, 2 * C, ctl->gcnt2, &ctl->cnt2, B.gpart2))
+    finish_sweep(phase, C, B, false);
+}
+
 // K2 of the two-kernel iteration: the residual update, the solution update and the next direction
 // in one sweep, with the beta the apply predicted (k_pcg_apply, FUSE):
 //   R -= alpha AP; Z += alpha P; P_next = R / diag + beta P; rz_c, ss_c, violation of the new R
@@ -1033,6 +1124,58 @@ __global__ void __launch_bounds__(kSweepThreads, (sweep_min_blocks<T>())) k_pcg_
   }
 }
 
+// K3 on fp32 rows of a multiple of four columns, four columns a thread (as k_pcg_update_v4; n = 250,000, 32
+// columns, us: 31.7 -> 20.5, 160 MB a launch).
+template <int U>
+__global__ void __launch_bounds__(kSweepThreads, 3)
+    k_pcg_dir_v4(int mode, int32_t n, int32_t C, float *__restrict__ Z, int64_t ldz, float *__restrict__ P, int64_t ldp,
+                 const float *__restrict__ R, int64_t ldr, const float *__restrict__ diag, PcgBufs B) {
+  PcgCtl *ctl = B.ctl;
+  if (mode == 0 && !ctl->go) return;
+  const bool upd_p = mode != 0 || ctl->done == 0;
+  const int NV = C / 4;
+  const SweepIdx ix = sweep_index(NV, NV);
+  if (!ix.on) return;
+  const int c0 = ix.c * 4;
+  const bool init = mode == 2 || mode == 4;  // P = R/diag: the old P is not read
+  float al[4], be[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    al[i] = mode == 0 ? (float)B.alpha[c0 + i] : 0.f;
+    be[i] = init ? 0.f : (float)B.beta[c0 + i];
+  }
+  for (long long r = ix.r0; r < n; r += U * ix.RS) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 pv[U], rv[U], zv[U];
+    float dv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long q = r + u * ix.RS;
+      const bool ok = q < n;
+      pv[u] = ok && !init ? *reinterpret_cast<const float4 *>(P + q * ldp + c0) : zero;
+      zv[u] = ok && mode == 0 ? *reinterpret_cast<const float4 *>(Z + q * ldz + c0) : zero;
+      rv[u] = ok && upd_p ? *reinterpret_cast<const float4 *>(R + q * ldr + c0) : zero;
+      dv[u] = ok && upd_p ? diag[q] : 1.f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long q = r + u * ix.RS;
+      if (q >= n) break;
+      const float4 p = pv[u], x = rv[u];
+      if (mode == 0)
+        *reinterpret_cast<float4 *>(Z + q * ldz + c0) = make_float4(zv[u].x + al[0] * p.x, zv[u].y + al[1] * p.y,
+                                                                    zv[u].z + al[2] * p.z, zv[u].w + al[3] * p.w);
+      if (mode == 4) *reinterpret_cast<float4 *>(Z + q * ldz + c0) = zero;
+      if (upd_p) {
+        float4 y = make_float4(x.x / dv[u], x.y / dv[u], x.z / dv[u], x.w / dv[u]);
+        if (!init)
+          y = make_float4(y.x + be[0] * p.x, y.y + be[1] * p.y, y.z + be[2] * p.z, y.w + be[3] * p.w);
+        *reinterpret_cast<float4 *>(P + q * ldp + c0) = y;
+      }
+    }
+  }
+}
+
 // Blocks per SM of a grid-stride kernel that are resident at once: its grid is that many blocks per
 // SM (one wave), since a second, partial wave leaves most SMs idle while it drains. Computed once
 // per kernel instantiation from the occupancy calculator (first called before any stream capture),
@@ -1303,12 +1446,24 @@ static int launch_apply(const PcgProblem &q, const PcgBufs &B, cudaStream_t s, b
   return launch ? check_launch() : DLP_OK;
 }
 
+// The sweeps four columns a thread: from 16 columns on (fewer run the two-kernel iteration).
+static bool rows16(const void *x, int64_t ld) { return (uintptr_t)x % 16 == 0 && ld % 4 == 0; }
+static bool wide_rows(const PcgProblem &q) { return q.C >= 16 && q.C % 4 == 0 && rows16(q.R, q.ldr); }
+
 // src (phase 3 only): the array the initial residual is copied from, in place of AP
 template <typename TS>
 static int launch_update(int phase, const PcgProblem &q, const PcgBufs &B, cudaStream_t s,
                          const void *src = nullptr, int64_t ldsrc = 0) {
   const TS *ap = phase == 3 ? (const TS *)src : (const TS *)q.AP;
   const int64_t ldap = phase == 3 ? ldsrc : q.ldap;
+  if constexpr (std::is_same<TS, float>::value) {
+    if (wide_rows(q) && rows16(ap, ldap)) {
+      static const int per = resident_per_sm(k_pcg_update_v4<2>, kSweepThreads);
+      k_pcg_update_v4<2><<<sm_count() * per, kSweepThreads, 0, s>>>(phase, q.n, q.C, (float *)q.R, q.ldr, ap, ldap,
+                                                                 (const float *)q.diag, B);
+      return check_launch();
+    }
+  }
   k_pcg_update<TS><<<update_grid<TS>(), kSweepThreads, 0, s>>>(phase, q.n, q.C, (TS *)q.R, q.ldr, ap, ldap,
                                                             (const TS *)q.diag, B);
   return check_launch();
@@ -1316,6 +1471,14 @@ static int launch_update(int phase, const PcgProblem &q, const PcgBufs &B, cudaS
 
 template <typename TS>
 static int launch_dir(int mode, const PcgProblem &q, const PcgBufs &B, cudaStream_t s) {
+  if constexpr (std::is_same<TS, float>::value) {
+    if (wide_rows(q) && rows16(q.Z, q.ldz) && rows16(q.P, q.ldp) && !q.P_lo && !q.fused) {
+      static const int per = resident_per_sm(k_pcg_dir_v4<2>, kSweepThreads);
+      k_pcg_dir_v4<2><<<sm_count() * per, kSweepThreads, 0, s>>>(mode, q.n, q.C, (float *)q.Z, q.ldz, (float *)q.P, q.ldp,
+                                                              (const float *)q.R, q.ldr, (const float *)q.diag, B);
+      return check_launch();
+    }
+  }
   k_pcg_dir<TS><<<dir_grid<TS>(), kSweepThreads, 0, s>>>(mode, q.n, q.C, (TS *)q.Z, q.ldz, (TS *)q.P, q.ldp,
                                                          (const TS *)q.R, q.ldr, (const TS *)q.diag, B,
                                                          (bf16 *)q.P_lo, q.ld_lo, q.fused ? (TS *)q.AP : nullptr);

@@ -433,3 +433,30 @@ def test_push_in_one_launch_equals_the_launched_rounds(C, dt):
     if dt == "float64":
         assert (r0, e0) == (r1, e1)
         assert float((x0 - x1).abs().max()) <= 2 * lim and float((z0 - z1).abs().max()) <= 2 * lim
+
+
+@pytest.mark.parametrize("n", [35, 257, 5001])
+@pytest.mark.parametrize("C", [15, 16, 20, 32, 36])
+def test_pcg_sweeps_four_columns_a_thread(C, n):
+    """The wide-row sweeps (C of at least 16, a multiple of four, aligned rows) against the scalar ones (a Z on
+    an odd pitch keeps the direction sweep scalar; C = 15 both): the true residual meets the target from a
+    warm and a zero start, and columns beyond C keep their values."""
+    ds = graphs.er_graph(n, 8, 4, seed=n)
+    lab = torch.as_tensor(graphs.label_mask(n, 0.2, seed=n)).cuda()
+    S = stream.build_system(ds, torch.ones(n, dtype=torch.bool, device="cuda"), lab, eta=1e-3, dtype="float32")
+    m = S.n_u
+    g = torch.Generator().manual_seed(C * n)
+    rhs = torch.rand((m, C), generator=g).cuda()
+    rn = rhs.double().norm(dim=0)
+    target = 1e-4  # far above the fp32 floor of these systems
+    for odd in (False, True):
+        for zero in (False, True):
+            Z = solvers.padded_empty(m, C, torch.float32, "cuda", fill=0.5) if not odd else \
+                torch.full((m, C + 5 - C % 2), 0.5, device="cuda")[:, :C]
+            st = solvers.Stats()
+            solvers.pcg(S, Z, rhs, None, solvers.jacobi_M(S), 3000, st, target_relres=target, use_graph=False,
+                        zero_start=zero)
+            R = rhs.double() - kernels.spmm_axpy(S.W, Z.double().contiguous(), a=S.diag.double(), b=-1.0)
+            assert float((R.norm(dim=0) / rn).max()) <= 1.05 * target and 1 < st.iters < 3000
+            if odd:
+                assert float((Z.as_strided((m, 1), (Z.stride(0), 1), Z.storage_offset() + C) - 0.5).abs().max()) == 0.0
