@@ -82,6 +82,7 @@ SIGNATURES: dict[str, tuple[str, object]] = {
     "dlp_system_rows": ("pippipdpiiippqppqp", ct.c_int),
     "dlp_park_rows": ("pipiipdpqpqp", ct.c_int),
     "dlp_cols_scale": ("iipqipipqip", ct.c_int),
+    "dlp_rows_take": ("qiqpqippqip", ct.c_int),
     "dlp_fused_push_workspace_bytes": ("ii", ct.c_size_t),
     "dlp_fused_push": ("ppppiiippqpqippiiiipzpppp", ct.c_int),
     "dlp_fused_push_counts": ("ppp", ct.c_int),

@@ -146,6 +146,10 @@ class FrontierOps:
     def edges(self, value):
         self._edges = value
 
+    def edge_count(self) -> int:
+        """The counter's value; no host read where nothing was counted."""
+        return 0 if self._edges is None else int(self._edges)
+
     def _rows(self, rows):
         rbeg, rend = _rows_of(self.W)
         rows = rows.to(torch.int32)
@@ -204,6 +208,22 @@ class FrontierOps:
         rbeg, rend = _rows_of(self.W)
         _lib.call("dlp_mark_neighbors", ptr(rbeg), ptr(rend), ptr(self.W.indices), ptr(r), int(r.numel()),
                   ptr(mark), stream())
+
+
+def rows_take(X, idx, dtype, out=None):
+    """X[idx] (row ids) in `dtype`, into `out` when given."""
+    floats = (torch.float32, torch.float64)
+    if not X.is_cuda or idx.dtype != torch.int64 or X.dtype not in floats or dtype not in floats or X.stride(1) != 1:
+        Y = X[idx].to(dtype)
+        return Y if out is None else out.copy_(Y)
+    n = int(idx.numel())
+    if out is None:
+        out = torch.empty((n, X.shape[1]), dtype=dtype, device=X.device)
+    idx = idx.contiguous()
+    if n and X.shape[1]:
+        _lib.call("dlp_rows_take", n, X.shape[1], X.shape[0], ptr(X), ld(X), code(X), ptr(idx), ptr(out), ld(out),
+                  code(out), stream())
+    return out
 
 
 def flatnonzero(flag: torch.Tensor, idx: torch.Tensor | None = None, out: torch.Tensor | None = None,

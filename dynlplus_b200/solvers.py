@@ -395,7 +395,7 @@ def push(sys: System, Z, R, eps, ops: FrontierOps, st: Stats, budget_edges=None,
     flags = torch.empty(max(n, 1), dtype=torch.uint8, device=dev)
     mark = torch.zeros(max(n, 1), dtype=torch.uint8, device=dev)
     cand = kernels.flatnonzero(kernels.violating(R, diag, eps_d, out=flags))
-    e0, it, best, stall = int(ops.edges), 0, float("inf"), 0
+    e0, it, best, stall = ops.edge_count(), 0, float("inf"), 0
     D = torch.empty((max(n, 1), Z.shape[1]), dtype=dt, device=dev)
     while cand.numel() and it < max_iter:
         kernels.push_take(cand, Z, R, diag, D[: cand.numel()], mark)
@@ -407,7 +407,7 @@ def push(sys: System, Z, R, eps, ops: FrontierOps, st: Stats, budget_edges=None,
         cand = kernels.flatnonzero(viol, idx=touched)
         it += 1
         if it % 32 == 0:
-            if budget_edges is not None and int(ops.edges) - e0 > budget_edges:
+            if budget_edges is not None and ops.edge_count() - e0 > budget_edges:
                 break
             v = violation(sys, R, eps_d)
             best, stall = (v, 0) if v < 0.99 * best else (best, stall + 1)
@@ -444,8 +444,10 @@ def supernode_init(sys: System, X, known=None, cols=None, comp="tau"):
     dynlp/solvers.py:138-153): with known=None the share of the component's weight to each
     labelled class (DynLP's rule); with a known mask the weighted average over labelled and known
     neighbours. Writes X[new, cols] in place and returns X."""
+    if comp not in sys.comps:  # asked first: the rows' number is a host read
+        return X
     new = torch.nonzero(sys.is_new, as_tuple=False).flatten()
-    if not new.numel() or comp not in sys.comps:
+    if not new.numel():
         return X
     cols = slice(0, sys.C) if cols is None else cols
     B = sys.B.to(X.dtype)
@@ -462,8 +464,8 @@ def supernode_init(sys: System, X, known=None, cols=None, comp="tau"):
 def init_h(sys: System, H, known, fallback, comp="fh"):
     """New rows: h = 1 + the component's weighted average h over known neighbours, labelled ones
     counting with h = 0 (dynlp/solvers.py:156-163). Writes H[new, 0] in place and returns H."""
-    new = torch.nonzero(sys.is_new, as_tuple=False).flatten()
-    if new.numel() and comp in sys.comps:
+    new = torch.nonzero(sys.is_new, as_tuple=False).flatten() if comp in sys.comps else None
+    if new is not None and new.numel():
         kf = known.to(H.dtype)
         lab, nc = sys.comps[comp]
         a = _rows_spmm(sys, new, (H[:, 0] * kf)[:, None])[:, 0]
@@ -485,17 +487,17 @@ class Solver:
         self.n_total, self.K, self.dtype = n_total, K, to_dtype(dtype)
         self.store_dtype, self.C, self.F = to_dtype(store_dtype or dtype), 1 if K == 2 else K, None
 
-    def _warm(self, sys: System):
+    def _warm(self, sys: System, out=None):
         if self.F is None:
             self.F = torch.empty((self.n_total, self.C), dtype=self.store_dtype, device=sys.diag.device)
             self.F[:] = sys.prior.to(self.store_dtype)
-        return self.F[sys.U].to(self.dtype)
+        return kernels.rows_take(self.F, sys.U, self.dtype, out=out)
 
     def _store(self, sys: System, X):
         self.F[sys.U] = X.to(self.store_dtype)
 
     def scores(self, sys: System):
-        return self.F[sys.U]
+        return kernels.rows_take(self.F, sys.U, self.F.dtype)
 
 
 class ItLP(Solver):
@@ -564,7 +566,7 @@ class DynLP(Solver):
                 ops.mark_neighbors(upd, mark)
                 frontier = kernels.flatnonzero(mark)
             self._store(sys, X)
-        st.edges, st.ms = int(ops.edges), tm.ms
+        st.edges, st.ms = ops.edge_count(), tm.ms
         return st
 
 
@@ -768,11 +770,9 @@ class DynLPPlus(Solver):
             if self.H is None:
                 self.H = torch.zeros((self.n_total, 1), dtype=self.store_dtype, device=dev)
             known = ~sw.is_new
-            X = supernode_init(sw, self._warm(sw), known, comp="fh")
-            Hc = init_h(sw, self.H[sw.U].to(self.dtype), known, self.hmax or 1.0)
             Z = padded_empty(n, C + 1, self.dtype, dev)
-            Z[:, :C] = X
-            Z[:, C:] = Hc
+            supernode_init(sw, self._warm(sw, out=Z[:, :C]), known, comp="fh")
+            init_h(sw, kernels.rows_take(self.H, sw.U, self.dtype, out=Z[:, C:]), known, self.hmax or 1.0)
             rhs = self._rhs_h(sw)
             ops, amg_box, hmax = FrontierOps(sw.W, C + 1, self.group), [None], self.hmax
             if hmax is None and n:  # first batch: get h before choosing the label tolerance
@@ -809,7 +809,7 @@ class DynLPPlus(Solver):
             self._store(sw, Z64[:, :C])
             self.H[sw.U] = Z64[:, C:]
             self._Z64, self._R64 = Z64, R64
-        st.edges += int(ops.edges)
+        st.edges += ops.edge_count()
         st.ms = tm.ms
         return st
 
@@ -857,7 +857,7 @@ class IncrementalLP(DynLPPlus):
             return ok
         ops = FrontierOps(s64.W, Z.shape[1], self.group)
         ok = push(s64, Z, R, eps, ops, st, max_iter=self.max_rounds)[2]
-        st.edges += int(ops.edges)
+        st.edges += ops.edge_count()
         return ok
 
     def _park(self, s64, rows):

@@ -424,6 +424,11 @@ int dlp_park_rows(const int32_t *rows, int32_t nr, const uint8_t *umask, int32_t
 int dlp_cols_scale(int32_t n, int32_t C, const void *X, int64_t ldx, int x_dtype, const double *scale, int32_t op,
                    void *Y, int64_t ldy, int y_dtype, dlp_stream_t stream);
 
+/* dst[i, 0..C) = src[idx[i], 0..C) (a solver's rows U of its resident scores), converted between f32 and
+ * f64; an index outside [0, n_src) gives NaN. src and dst must not overlap. */
+int dlp_rows_take(int64_t n, int32_t C, int64_t n_src, const void *src, int64_t lds, int src_dtype, const int64_t *idx,
+                  void *dst, int64_t ldd, int dst_dtype, dlp_stream_t stream);
+
 /* Class-sum elimination for the refinement's corrections (no reference counterpart: the reference
  * solves every class column). On a grounded row the class right-hand sides sum to the grounding
  * (dynlp/stream.py:163-165: s = sum_c B_c + eta, rhs = B + eta * prior, sum_c prior_c = 1), so the

@@ -460,3 +460,25 @@ def test_pcg_sweeps_four_columns_a_thread(C, n):
             assert float((R.norm(dim=0) / rn).max()) <= 1.05 * target and 1 < st.iters < 3000
             if odd:
                 assert float((Z.as_strided((m, 1), (Z.stride(0), 1), Z.storage_offset() + C) - 0.5).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("src,dst", [("float32", "float32"), ("float32", "float64"), ("float64", "float32"),
+                                     ("float64", "float64")])
+@pytest.mark.parametrize("n,C", [(0, 3), (1, 1), (257, 5), (4099, 33)])
+def test_rows_take_equals_indexing(n, C, src, dst):
+    """Rows by id against tensor indexing, every value the same: from and into rows on a pitch of their own,
+    other id types and layouts on the general path, and an id outside the source gives NaN."""
+    g = torch.Generator().manual_seed(n + C)
+    X = torch.randn((5000, C + 2), generator=g, dtype=torch.float64).to("cuda").to(getattr(torch, src))[:, :C]
+    idx = torch.randint(0, 5000, (n,), generator=g).cuda()
+    want = X[idx].to(getattr(torch, dst))
+    out = torch.full((n, C + 3), 3.0, dtype=want.dtype, device="cuda")
+    kernels.rows_take(X, idx, want.dtype, out=out[:, :C])
+    assert torch.equal(out[:, :C], want) and bool((out[:, C:] == 3.0).all())
+    assert torch.equal(kernels.rows_take(X, idx, want.dtype), want)
+    assert torch.equal(kernels.rows_take(X, idx.to(torch.int32), want.dtype), want)
+    assert torch.equal(kernels.rows_take(X.t().contiguous().t(), idx, want.dtype), want)
+    if n > 1:
+        bad = idx.clone()
+        bad[1] = 5000
+        assert bool(kernels.rows_take(X, bad, want.dtype)[1].isnan().all())
