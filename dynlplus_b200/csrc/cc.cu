@@ -302,8 +302,10 @@ __global__ void k_cc_gather_rank(const int32_t *__restrict__ parent, int32_t n, 
 // kReachMaxSweeps), the union-find over every live edge where they do not settle (long chains), and the
 // membership update, with a grid barrier where a launch boundary or a host read was. A settled graph takes
 // four sweeps; launch by launch, each batch of sweeps ended in a host read in the middle of the patch.
-// Bound by the first sweep's row scans (n = 1M, degree 10: 114 us of 160); at n = 3,000 by the barriers
-// (four launches, the read and two clears, 90 us of host time -> one launch of 15 us).
+// Bound by the first sweep's row scans (n = 1M, degree 10: 183 us in all) and, below, by the sweeps' number
+// and barriers (n = 3,000: 26 us, in place of four launches, two clears and a host read; 60,000: 33). One
+// thread per row: 4 or 8 lanes a row, or several entries in flight, scan sooner than the marks spread in place
+// and need more sweeps (60,000: 41 to 68 us; 250,000: 61 -> 67 to 134).
 // info: [0] vertices of vmask or sink, [1] vertices of vmask left ungrounded, [2] sweeps run (negative:
 // the union-find finished), [3] a barrier's wait ran out.
 constexpr int kGroundThreads = 1024;

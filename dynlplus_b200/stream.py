@@ -22,7 +22,7 @@ import torch
 
 from . import _lib, cc, kernels
 from .backend import CSR, code, ld, ptr, stream, sync, to_dtype, workspace
-from .graphs import Dataset, csr_rows
+from .graphs import Dataset
 
 
 @dataclass

@@ -598,8 +598,8 @@ int dlp_amg_vcycle(const dlp_amg_level *levels, int32_t nlev, const double *coar
  * is the operator rbeg/rend/col/w of the solve). Per iteration: AP = A P, pAp, alpha, Z += alpha P,
  * R -= alpha AP, the stop metric (mode bit 0: max_uc |R_uc| / (eps_c diag_u) <= 1; bit 1:
  * max_c ||R_c|| / rhs_norm[c] <= target_relres), Y = M(R), rz = R.Y, beta, P = Y + beta P; inner
- * products in fp64 with a fixed reduction order. With use_graph != 0 the iterations run on the device
- * as one CUDA graph with a conditional WHILE node (cached per problem), stopping at a proposed stop,
+ * products in fp64 with a fixed reduction order. The host launches the iterations and reads the
+ * device's decision after each (use_graph is accepted and changes nothing), stopping at a proposed stop,
  * the patience rule (no 10% improvement in `patience` iterations), the cap or the cancel word; a
  * proposed stop is confirmed on the true residual as the reference does (solvers.py:85-89), and a
  * failed confirmation resumes from the true residual. Y is an n x C scratch like R, P and AP.
