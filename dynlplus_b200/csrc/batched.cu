@@ -273,7 +273,7 @@ constexpr int kBUnroll = 4;
 // order; its first tile's block keeps it, and whether the instance is in this iteration, for the direction
 // sweep), R -= alpha AP; then, as phase 1 (a true residual after a proposed stop) and phase 2 (the start), the
 // tile's sums of R^2 / diag and R^2 and the largest violation. Phase 3: as 2, R copied from AP (the
-// right-hand side of a zero start). Measured with the direction sweep on the same systems: 57 -> 27 us.
+// right-hand side of a zero start). Measured with the direction sweep on the same systems: 57 -> 20 us.
 template <typename TS>
 __global__ void __launch_bounds__(kBThreads) k_b_update(int phase, int32_t C, TS *R, int64_t ldr,
                                                         const TS *__restrict__ AP, int64_t ldap,

@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(kPushThreads) k_push_seed(PushArgs<T> a, const
 
 // The whole run in one cooperative launch: the seed's take, then rounds of scatter, barrier, sift, barrier
 // until the frontier is empty or the run stops. As two launches a round in a graph's loop, 17 rounds took
-// 320 us at n = 60,000 (3 fp64 columns, mean degree 16); in one launch, with both phases as they are now, the whole call takes 280.
+// 320 us at n = 60,000 (2 fp64 columns, mean degree 16); in one launch, with both phases as they are now, the
+// whole call of 15 rounds takes 280.
 template <typename TW, typename T, int CMAX>
 __global__ void __launch_bounds__(kPushThreads) k_push_whole(PushArgs<T> a, const int32_t *__restrict__ cand, int nc,
                                                              int words) {
