@@ -295,6 +295,14 @@ __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, cons
   for (int k = 0; k < VPL; ++k)
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[k][i] = TA(0);
+  // fp32 lanes of one vector (several lanes per row, then with few entry slots) keep two sums, of every other
+  // entry: the rounding of two slots, whose chains of additions are half as long
+  constexpr bool kTwo = VPL == 1 && ROW == kRowVec && sizeof(TA) == 4 && U % 2 == 0;
+  TA odd[kTwo ? VW : 1];
+  if constexpr (kTwo) {
+#pragma unroll
+    for (int i = 0; i < VW; ++i) odd[i] = TA(0);
+  }
   for (int j0 = beg + es; j0 < end; j0 += U * ES) {
     int v[U];
     TA wv[U];
@@ -376,9 +384,16 @@ __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, cons
 #pragma unroll
         for (int k = 0; k < VPL; ++k)
 #pragma unroll
-          for (int i = 0; i < VW; ++i) acc[k][i] = fmaa(wv[u], t[u][k][i], acc[k][i]);
+          for (int i = 0; i < VW; ++i) {
+            if (kTwo && (u & 1)) odd[kTwo ? i : 0] = fmaa(wv[u], t[u][k][i], odd[kTwo ? i : 0]);
+            else acc[k][i] = fmaa(wv[u], t[u][k][i], acc[k][i]);
+          }
       }
     }
+  }
+  if constexpr (kTwo) {
+#pragma unroll
+    for (int i = 0; i < VW; ++i) acc[0][i] += odd[i];
   }
   for (int off = LV; off < G; off <<= 1) {
 #pragma unroll

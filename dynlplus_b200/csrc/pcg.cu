@@ -1887,7 +1887,11 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
     DLP_CUDA(cudaEventRecord(hs->up, s));
   }
   WholePlan whole;
-  if (use_graph && !(mode & 8) && whole_fits(q, &whole)) {
+  // A recheck at the fp32 floor keeps the two-kernel iteration: its predicted beta recovers from a failed one where
+  // the three-kernel arithmetic of the whole solve drifts off (10,000 x 8 and 60,000 x 8 to 1e-6: 27 and 31
+  // iterations against 426 and a lost iterate).
+  const bool floor_recheck = q.fused && !(mode & 16) && (mode & 2);
+  if (use_graph && !(mode & 8) && !floor_recheck && whole_fits(q, &whole)) {
     DLP_TRY(whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s));
     PcgCtl cur{};
     DLP_TRY(read_ctl(B, hs, s, &cur));

@@ -69,8 +69,12 @@ template <class TW, class TX, int VW>
 __device__ __forceinline__ void whole_gather(const int32_t *col, const TW *w, const TX *X, int64_t ldx, int beg, int end,
                                              int es, int ES, int LV, int G, TX (&acc)[VW]) {
   constexpr int U = VW * (int)sizeof(TX) <= 16 ? 8 : 4;
+  // two sums per lane, of every other entry: shorter chains of rounded additions (the fp32 residual of a recheck
+  // is no coarser than the launched kernels', which have more entry slots: with one sum a solve of 8 columns to
+  // 1e-6, n = 60,000, failed its rechecks that theirs passed)
+  TX odd[VW];
 #pragma unroll
-  for (int i = 0; i < VW; ++i) acc[i] = TX(0);
+  for (int i = 0; i < VW; ++i) acc[i] = odd[i] = TX(0);
   for (int j0 = beg + es; j0 < end; j0 += U * ES) {
     TX t[U][VW], wv[U];
     int v[U];
@@ -89,8 +93,13 @@ __device__ __forceinline__ void whole_gather(const int32_t *col, const TW *w, co
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < VW; ++i) acc[i] = fmaa(wv[u], t[u][i], acc[i]);
+      for (int i = 0; i < VW; ++i) {
+        if (u & 1) odd[i] = fmaa(wv[u], t[u][i], odd[i]);
+        else acc[i] = fmaa(wv[u], t[u][i], acc[i]);
+      }
   }
+#pragma unroll
+  for (int i = 0; i < VW; ++i) acc[i] += odd[i];
   for (int off = LV; off < G; off <<= 1) {
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);

@@ -482,3 +482,18 @@ def test_rows_take_equals_indexing(n, C, src, dst):
         bad = idx.clone()
         bad[1] = 5000
         assert bool(kernels.rows_take(X, bad, want.dtype)[1].isnan().all())
+
+
+@pytest.mark.parametrize("n,K", [(10_000, 8), (20_000, 8), (10_000, 10)])
+def test_plain_fp32_solve_to_its_floor_in_the_device_loop(n, K):
+    """fp32 solves to 1e-6 with their own rechecks, at the floor of fp32: the device-side loop takes the host
+    loop's iterations (a failed recheck may not cost it the iterate)."""
+    ds = graphs.sbm(n, K=K, deg=16.0, seed=3)
+    lab = torch.as_tensor(graphs.label_mask(n, 0.01, seed=3)).cuda()
+    S = stream.build_system(ds, torch.ones(n, dtype=torch.bool, device="cuda"), lab, dtype="float32")
+    its = []
+    for graph in (True, False):
+        Z, st = solvers.padded_empty(S.n_u, K, torch.float32, "cuda", fill=0.0), solvers.Stats()
+        solvers.pcg(S, Z, S.rhs, None, solvers.jacobi_M(S), 10_000, st, target_relres=1e-6, use_graph=graph)
+        its.append(st.iters)
+    assert its[0] == its[1]
