@@ -275,7 +275,7 @@ enum RowPath : int { kRowVec = 0, kRow12F = 1, kRow10D = 2, kRow16H = 3, kRow8F 
 
 // COH (kRowVec only): X is read through L2, for kernels that write X in the same launch.
 template <typename TW, typename TX, typename TA, int VW, int VPL, int U = gather_batch_wide<TA, VW, VPL>(),
-          int ROW = kRowVec, bool COH = false>
+          int ROW = kRowVec, bool COH = false, bool TWO = false>
 __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, const TW *__restrict__ w,
                                            const TX *__restrict__ X, int64_t ldx, int beg, int end, int es,
                                            int ES, int cl, int LV, int NV, int G, TA (&acc)[VPL][VW]) {
@@ -295,9 +295,9 @@ __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, cons
   for (int k = 0; k < VPL; ++k)
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[k][i] = TA(0);
-  // fp32 lanes of one vector (several lanes per row, then with few entry slots) keep two sums, of every other
-  // entry: the rounding of two slots, whose chains of additions are half as long
-  constexpr bool kTwo = VPL == 1 && ROW == kRowVec && sizeof(TA) == 4 && U % 2 == 0;
+  // TWO (the SpMM and the PCG apply): fp32 lanes of one vector (several lanes per row, then with few entry slots)
+  // keep two sums, of every other entry: the rounding of two slots, whose chains of additions are half as long
+  constexpr bool kTwo = TWO && VPL == 1 && ROW == kRowVec && sizeof(TA) == 4 && U % 2 == 0;
   TA odd[kTwo ? VW : 1];
   if constexpr (kTwo) {
 #pragma unroll

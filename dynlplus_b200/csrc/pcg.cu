@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, (apply_min_blocks<T, VW, VPL>())) k_
     // per iteration at n = 1M against two), two 12-float rows
     gather_row<typename T::TW, typename T::TX, TA, VW, VPL,
                (ROWP == kRow8F ? 4 : WHOLE ? 2 : gather_batch_lean<TA, VW, VPL>()),
-               (WHOLE ? ROWP : kRowVec)>(
+               (WHOLE ? ROWP : kRowVec), false, true>(
         p.col, p.w, p.P, p.ldp, beg, end, es, ES, cl, LV, NV, G, acc);
     // FUSE: this row's P . AP and AP^2 / diag per column (0 past C and on invalid lanes)
     float pv_[FUSE ? 12 : 1], qv[FUSE ? 12 : 1];

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kThreads) k_spmm(SpmmArgs<T> p) {
     // rows (the fp64 residual 278 -> 267 us against two), two 12-float rows (three: 121 -> 133 us)
     gather_row<typename T::TW, TX, TA, VW, VPL,
                (ROW == kRow12F ? 2 : ROW == kRow16H ? 4 : ROW == kRow10D ? 4 : gather_batch_wide<TA, VW, VPL>()),
-               ROW>(
+               ROW, false, true>(
         p.col, p.w, p.X, p.ldx, beg, end, es, ES, cl, LV, NV, G, acc);
     if constexpr (ROW == kRow10D) {
       if (valid && es == 0) {  // same arithmetic, in the same order, as the per-column epilogue below
