@@ -162,8 +162,8 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
     dev = A.indices.device
     n = A.shape[0]
     dt = to_dtype(dtype)
-    active = active.to(torch.bool)
-    labeled = labeled.to(torch.bool)
+    active = active.to(torch.bool).contiguous()  # bound to their names: the kernels get bare addresses
+    labeled = labeled.to(torch.bool).contiguous()
     C = 1 if K == 2 else K
     f64 = torch.float64
     masks = torch.empty((2, max(n, 1)), dtype=torch.uint8, device=dev)  # U, and the active labelled vertices
@@ -173,8 +173,8 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
     y = (ds.y if ds.y.dtype == torch.int32 else ds.y.to(torch.int32)).contiguous()
     if n:
         ws = workspace("build_system").get(_lib.lib().dlp_build_system_workspace_bytes(n))
-        _lib.call("dlp_build_system_plan", n, ptr(A.indptr), ptr(A.indices), ptr(active.contiguous()),
-                  ptr(labeled.contiguous()), ptr(y), K, ptr(masks[0]), ptr(masks[1]), ptr(scans[0]), ptr(scans[1]),
+        _lib.call("dlp_build_system_plan", n, ptr(A.indptr), ptr(A.indices), ptr(active),
+                  ptr(labeled), ptr(y), K, ptr(masks[0]), ptr(masks[1]), ptr(scans[0]), ptr(scans[1]),
                   ptr(counts), ptr(ws), ws.numel(), stream())
         n_u, nnz, _, bad, n_active, n_ungrounded, _, lost, off = counts.tolist()
         if off:
