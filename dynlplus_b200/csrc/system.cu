@@ -6,6 +6,8 @@
 // Bound by that pass (columns, weights and marks of every entry, 16 bytes with the outputs) at large sizes and
 // by launches at small ones: some fifteen instead of about a hundred tensor operations with eleven host reads
 // (degree 16, the whole call: n = 100,000 1.61 -> 0.28 ms; n = 5,000 1.21 -> 0.26 ms).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace dlp {
@@ -61,8 +63,16 @@ struct SysOut {
   float *B32, *s32, *diag32, *rhs32, *rhsh32;  // fp32 copies (NULL: none)
 };
 
+// A kept weight as it is stored: bf16 by way of fp32, as the tensor library rounds fp64.
+template <typename TO, typename TW>
+__device__ __forceinline__ TO stored_weight(TW x) {
+  if constexpr (std::is_same<TO, bf16>::value) return __float2bfloat16_rn((float)x);
+  else return (TO)x;
+}
+
 // Eight lanes per row of U: kept entries in stored order (ranked by ballot), the row sum of the stored weights,
-// label weights added in stored order by the group's first lane (few neighbours are labelled).
+// label weights, which stay as they come, added in stored order by the group's first lane (few neighbours are
+// labelled).
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(kSysThreads)
     k_sys_fill(int32_t n, const int32_t *__restrict__ indptr, const int32_t *__restrict__ col, const TW *__restrict__ w,
@@ -99,9 +109,9 @@ __global__ void __launch_bounds__(kSysThreads)
     if (keep) {
       const int q = at + __popc(kb & ((1u << l) - 1u));
       o.col[q] = loc[v];
-      const TO x = (TO)w[j];
+      const TO x = stored_weight<TO>(w[j]);
       ((TO *)o.w)[q] = x;
-      sum += (double)x;
+      sum += cvt<double>(x);
     }
     at += __popc(kb);
     // labelled neighbours one after another (warp-uniform trip count)
@@ -197,7 +207,8 @@ int dlp_build_system_fill(int32_t n, const int32_t *indptr, const int32_t *col, 
                           float *rhs32, float *rhsh32, dlp_stream_t stream) {
   if (n <= 0 || n_u < 0 || K <= 0 || C <= 0 || col0 < 0 || col0 + C > K) return DLP_ERR_INVALID;
   if (!indptr || !col || !w || !umask || !sink || !y || !loc || !pos || !indptr_out) return DLP_ERR_INVALID;
-  if ((w_dtype != DLP_F32 && w_dtype != DLP_F64) || (w_out_dtype != DLP_F32 && w_out_dtype != DLP_F64))
+  if ((w_dtype != DLP_F32 && w_dtype != DLP_F64) ||
+      (w_out_dtype != DLP_F32 && w_out_dtype != DLP_F64 && w_out_dtype != DLP_BF16))
     return DLP_ERR_DTYPE;
   cudaStream_t s = (cudaStream_t)stream;
   // the last row pointer (the scan's total)
@@ -209,10 +220,15 @@ int dlp_build_system_fill(int32_t n, const int32_t *indptr, const int32_t *col, 
 #define DLP_SYS_FILL(TW, TO)                                                                                        \
   k_sys_fill<TW, TO><<<grid, kSysThreads, 0, s>>>(n, indptr, col, (const TW *)w, umask, sink, y, K, eta, prior, C, col0, \
                                                   loc, pos, o)
-  if (w_dtype == DLP_F32 && w_out_dtype == DLP_F32) DLP_SYS_FILL(float, float);
-  else if (w_dtype == DLP_F32) DLP_SYS_FILL(float, double);
-  else if (w_out_dtype == DLP_F32) DLP_SYS_FILL(double, float);
-  else DLP_SYS_FILL(double, double);
+  if (w_dtype == DLP_F32) {
+    if (w_out_dtype == DLP_F32) DLP_SYS_FILL(float, float);
+    else if (w_out_dtype == DLP_F64) DLP_SYS_FILL(float, double);
+    else DLP_SYS_FILL(float, bf16);
+  } else {
+    if (w_out_dtype == DLP_F32) DLP_SYS_FILL(double, float);
+    else if (w_out_dtype == DLP_F64) DLP_SYS_FILL(double, double);
+    else DLP_SYS_FILL(double, bf16);
+  }
 #undef DLP_SYS_FILL
   return check_launch();
 }

@@ -185,11 +185,10 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
             raise _lib.DLPError("dlp_build_system_plan", 8)
         if n_u and not nnz:  # no kernel takes an operator without entries
             raise _lib.DLPError("dlp_build_system_plan", 1)
-    wdt = dt if dt != torch.bfloat16 else torch.float32
     U = torch.empty(n_u, dtype=torch.int64, device=dev)
     ip = torch.zeros(n_u + 1, dtype=torch.int32, device=dev)
     ci = torch.empty(nnz, dtype=torch.int32, device=dev)
-    wd = torch.empty(nnz, dtype=wdt, device=dev)
+    wd = torch.empty(nnz, dtype=dt, device=dev)
     v64 = torch.empty((2, n_u), dtype=f64, device=dev)
     s, diag = v64[0], v64[1]
     Bm = torch.empty((n_u, K), dtype=f64, device=dev)
@@ -203,14 +202,11 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
         lo = (torch.empty((n_u, K), dtype=dt, device=dev), v32[0], v32[1], torch.empty((n_u, C), dtype=dt, device=dev),
               torch.empty((n_u, C + 1), dtype=dt, device=dev))
     if n_u:
-        if dt == torch.bfloat16:
-            A = CSR(A.data.to(dt).to(torch.float32), A.indices, A.indptr, A.shape)
         _lib.call("dlp_build_system_fill", n, ptr(A.indptr), ptr(A.indices), ptr(A.data), code(A.data), ptr(masks[0]),
                   ptr(masks[1]), ptr(y), K, float(eta), prior_v, C, 1 if K == 2 else 0, ptr(scans[0]),
                   ptr(scans[1]), n_u, ptr(U), ptr(ip), ptr(ci), ptr(wd), code(wd), ptr(Bm), ptr(s), ptr(diag), ptr(rhs),
                   ptr(rhsh), *([ptr(x) for x in lo] if lo else [None] * 5), stream())
-        A = ds.A
-    W = CSR(wd if dt != torch.bfloat16 else wd.to(dt), ci, ip, (n_u, n_u))
+    W = CSR(wd, ci, ip, (n_u, n_u))
     is_new = torch.ones(n_u, dtype=torch.bool, device=dev) if prev_U is None else ~prev_U[U]
     seed = is_new.clone()
     if ins_ids is not None or del_ids is not None:

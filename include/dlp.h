@@ -247,8 +247,8 @@ int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, 
  * entry there (n + 1 ints), and counts (device, nine ints): rows, entries, -, a column out of range,
  * active vertices, ungrounded vertices, sweeps, a wait ran out, a labelled vertex's class y outside
  * [-K, K). Asynchronous; the caller reads counts.
- * fill: U (ids), the CSR of A[U, U] in stored order with weights in w_out_dtype, B (n_u x K label weights
- * by class y), s = sum B + eta, diag = s + row sum, rhs = B[:, col0 : col0 + C] + eta * prior, rhsh = [rhs,
+ * fill: U (ids), the CSR of A[U, U] in stored order with weights in w_out_dtype (f32, f64 or bf16; the row
+ * sums are those of the stored weights), B (n_u x K label weights by class y, from w as it is), s = sum B + eta, diag = s + row sum, rhs = B[:, col0 : col0 + C] + eta * prior, rhsh = [rhs,
  * diag]; fp32 copies where the pointers are not NULL. */
 size_t dlp_build_system_workspace_bytes(int32_t n);
 int dlp_build_system_plan(int32_t n, const int32_t *indptr, const int32_t *col, const uint8_t *active,

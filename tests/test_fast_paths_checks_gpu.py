@@ -36,3 +36,27 @@ def test_build_system_takes_masks_of_any_layout(layout):
     else:
         a, b = on.to(torch.int64), torch.stack([lab, lab], 1).to(torch.float32)[:, 0]
     same_system(stream.build_system(ds, a, b), want)
+
+
+@pytest.mark.parametrize("wdtype", ["float32", "float64"])
+@pytest.mark.parametrize("K,eta", [(2, 0.0), (5, 0.3)])
+def test_bf16_system_rounds_its_operator_only(K, eta, wdtype):
+    """The label weights (B, s, rhs) of a bf16 system come from the weights as they are, in its fp64 twin to
+    fp64 rounding; the operator's entries are the rounded ones and the diagonal has their row sums."""
+    from oracle import ref_np as O
+    n = 1003
+    ds = graphs.er_graph(n, 9, K, weights="lognormal", seed=K, dtype=wdtype)
+    lab = np.random.default_rng(K).random(n) < 0.2
+    on = torch.ones(n, dtype=torch.bool, device="cuda")
+    S = stream.build_system(ds, on, torch.as_tensor(lab).cuda(), dtype="bfloat16", eta=eta)
+    want = O.build_system(ds.A.to_scipy(), ds.y.cpu().numpy(), K, np.ones(n, bool), lab, eta=eta)
+    T = S.astype(torch.float64)
+    assert np.array_equal(S.U.cpu().numpy(), want["U"])
+    w = torch.as_tensor(want["W"].data).to(torch.bfloat16)
+    assert torch.equal(S.W.data.cpu(), w) and np.array_equal(S.W.indices.cpu().numpy(), want["W"].indices)
+    rowsum = np.add.reduceat(np.append(w.double().numpy(), 0.0), want["W"].indptr[:-1]) * (np.diff(want["W"].indptr) > 0)
+    for name, ref in (("s", want["s"]), ("B", want["B"]), ("rhs", want["rhs"]), ("diag", want["s"] + rowsum)):
+        got = getattr(T, name).cpu().numpy()
+        np.testing.assert_allclose(got, ref, rtol=1e-13, atol=1e-13)
+        low = getattr(S, name)
+        assert low.dtype == torch.bfloat16 and torch.equal(low, getattr(T, name).to(torch.bfloat16))
