@@ -53,15 +53,13 @@ class BatchedSystems:
         s64 = [s.astype(torch.float64) for s in systems]
         self.diag64 = torch.cat([s.diag for s in s64])
         self.diag = self.diag64.to(dtype)
-        self.rhs64 = torch.cat([self._rhs(s, with_h) for s in s64])
+        # from each system's own rhs and diag (its [rhs | diag] copy does not follow a replaced right-hand side)
+        self.rhs64 = torch.empty((N, self.Ch), dtype=torch.float64, device=dev)
+        torch.cat([s.rhs for s in s64], out=self.rhs64[:, :self.C])
+        if with_h:
+            self.rhs64[:, self.C] = self.diag64
         self.rhs = self.rhs64.to(dtype)
         self.set_tiles(tile_rows)
-
-    @staticmethod
-    def _rhs(s, with_h):
-        if not with_h:
-            return s.rhs
-        return s.rhs_h if s.rhs_h is not None else torch.cat([s.rhs, s.diag[:, None]], 1)
 
     def set_tiles(self, tile_rows):
         """Cut every instance into tiles of up to tile_rows rows, fewer for small instances (at most some 128

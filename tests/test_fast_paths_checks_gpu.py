@@ -1,9 +1,11 @@
 """What the fast paths take besides plain calls: layouts, types, limits and inputs that are refused."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
 
-from dynlplus_b200 import graphs, stream
+from dynlplus_b200 import batched, graphs, solvers, stream
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +62,20 @@ def test_bf16_system_rounds_its_operator_only(K, eta, wdtype):
         np.testing.assert_allclose(got, ref, rtol=1e-13, atol=1e-13)
         low = getattr(S, name)
         assert low.dtype == torch.bfloat16 and torch.equal(low, getattr(T, name).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("with_h", [True, False])
+def test_batch_takes_each_systems_own_right_hand_side(with_h):
+    """Systems whose right-hand side was replaced (their [rhs | diag] copy was not) are solved for the new one:
+    the batch holds it, and the scores are those of the scaled system."""
+    ds, lab = labelled_graph()
+    S = stream.build_system(ds, torch.ones_like(lab), lab, dtype="float64")
+    T = dataclasses.replace(S, rhs=2 * S.rhs, _conv={})
+    bs = batched.BatchedSystems([S, T, S], with_h=with_h)
+    h = [S.diag[:, None]] if with_h else []
+    assert torch.equal(bs.rhs, torch.cat([torch.cat([x.rhs, *h], 1) for x in (S, T, S)]))
+    for solve in (batched.solve_many, batched.solve_many_mixed):
+        (a, b), _ = solve([S, T], target_relres=1e-8)
+        for sys, F in ((S, a), (T, b)):
+            R = solvers.residual(sys, F.contiguous(), sys.rhs)
+            assert float((R.norm(dim=0) / sys.rhs.norm(dim=0)).max()) <= 1.01e-8
