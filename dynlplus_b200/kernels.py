@@ -70,12 +70,13 @@ def spmm_axpy(W, X, a=None, b=1.0, group="auto", *, rhs=None, cr=1.0, alpha=1.0,
     if rhs is not None and rhs.dtype != (torch.float32 if out.dtype == torch.bfloat16 else out.dtype):
         rhs = rhs.to(torch.float32 if out.dtype == torch.bfloat16 else out.dtype)
     # rows that cannot be gathered as vectors may be copied to scratch that can (decided by the library;
-    # the test here spares small calls the question)
+    # the test here spares small calls the question). The scratch belongs to this call: a captured graph
+    # replays into it, so it may not be a buffer that a later call grows and frees
     if rows is None and C > 2 and X.dtype != torch.float64 and W.nnz * C >= 12_000_000 and X.shape[0] == n:
         avg = W.nnz / n
         need = _lib.lib().dlp_spmm_workspace_bytes(n, C, ptr(X), ld(X), code(X), avg)
         if need:
-            ws = workspace("spmm_rows").get(need)
+            ws = torch.empty(need, dtype=torch.uint8, device=X.device)
             _lib.call("dlp_spmm_ws", ptr(rbeg), ptr(rend), ptr(W.indices), ptr(W.data), code(W.data), n, C, ptr(X), ld(X),
                       code(X), ptr(a), float(alpha), float(b), ptr(rhs), ld(rhs) if rhs is not None else C, float(cr),
                       ptr(out), ld(out), code(out), _group(W, group), avg, ptr(ws), ws.numel(), stream())

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 import torch
 
-from dynlplus_b200 import batched, graphs, solvers, stream
+from dynlplus_b200 import batched, graphs, kernels, solvers, stream
+from dynlplus_b200.backend import CSR
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +80,32 @@ def test_batch_takes_each_systems_own_right_hand_side(with_h):
         for sys, F in ((S, a), (T, b)):
             R = solvers.residual(sys, F.contiguous(), sys.rhs)
             assert float((R.norm(dim=0) / sys.rhs.norm(dim=0)).max()) <= 1.01e-8
+
+
+def random_csr(n, deg, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    col = torch.randint(0, n, (n * deg,), generator=g, device="cuda").to(torch.int32)
+    ip = torch.arange(0, n * deg + 1, deg, device="cuda").to(torch.int32)
+    return CSR(torch.rand(n * deg, generator=g, device="cuda"), col, ip, (n, n))
+
+
+def test_captured_product_keeps_its_scratch():
+    """A product whose odd rows go through scratch, captured into a graph: replayed after a larger one has run and
+    the memory it left was taken, it gives the product of the values X then holds and writes nothing else."""
+    n, C = 60_000, 17
+    W, X = random_csr(n, 16, 0), torch.rand((n, C), device="cuda")
+    Y = torch.empty_like(X)
+    kernels.spmm_axpy(W, X, out=Y)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        kernels.spmm_axpy(W, X, out=Y)
+    V, U = random_csr(2 * n, 16, 1), torch.rand((2 * n, C), device="cuda")
+    kernels.spmm_axpy(V, U)
+    taken = [torch.full((1 << 20,), 7.0, device="cuda") for _ in range(16)]
+    X.uniform_(0, 1)
+    want = kernels.spmm_axpy(W, X)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(Y, want)
+    assert all(bool((t == 7.0).all()) for t in taken)
