@@ -76,7 +76,11 @@ def spmm_axpy(W, X, a=None, b=1.0, group="auto", *, rhs=None, cr=1.0, alpha=1.0,
         avg = W.nnz / n
         need = _lib.lib().dlp_spmm_workspace_bytes(n, C, ptr(X), ld(X), code(X), avg)
         if need:
-            ws = torch.empty(need, dtype=torch.uint8, device=X.device)
+            try:
+                ws = torch.empty(need, dtype=torch.uint8, device=X.device)
+            except torch.OutOfMemoryError:
+                need = 0  # no room: the rows are gathered as they are
+        if need:
             _lib.call("dlp_spmm_ws", ptr(rbeg), ptr(rend), ptr(W.indices), ptr(W.data), code(W.data), n, C, ptr(X), ld(X),
                       code(X), ptr(a), float(alpha), float(b), ptr(rhs), ld(rhs) if rhs is not None else C, float(cr),
                       ptr(out), ld(out), code(out), _group(W, group), avg, ptr(ws), ws.numel(), stream())

@@ -109,3 +109,21 @@ def test_captured_product_keeps_its_scratch():
     torch.cuda.synchronize()
     assert torch.equal(Y, want)
     assert all(bool((t == 7.0).all()) for t in taken)
+
+
+def test_product_without_room_for_its_scratch(monkeypatch):
+    """Where the scratch for odd rows cannot be allocated the product gathers them as they are: fp64 product of
+    the same values within the roundoff of 16 terms in [0, 1)."""
+    n, C = 60_000, 17
+    W, X, Y = random_csr(n, 16, 0), torch.rand((n, C), device="cuda"), torch.empty((n, C), device="cuda")
+    empty = torch.empty
+
+    def full(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    kernels.spmm_axpy(W, X, out=Y)
+    monkeypatch.undo()
+    want = kernels.spmm_axpy(CSR(W.data.double(), W.indices, W.indptr, W.shape), X.double())
+    assert float((Y.double() - want).abs().max()) <= 16 * 16 * 2.0 ** -24
