@@ -8,6 +8,8 @@ leading dimensions so score matrices may be padded for 16-byte vector gathers.
 """
 from __future__ import annotations
 
+import math
+
 import torch
 
 from . import _lib
@@ -191,9 +193,11 @@ class FrontierOps:
         diag, rhs = diag.to(X.dtype).contiguous(), rhs.to(X.dtype)
         ws = workspace("frontier").get(_lib.lib().dlp_frontier_solve_workspace_bytes(W.shape[0], self.C, code(X)))
         rounds, edges = ct.c_int32(0), ct.c_ulonglong(0)
+        # any number is a cap, as in a loop `while rounds < max_rounds`; the kernel's is an int32
+        cap = math.ceil(min(max(max_rounds, 0), 2**31 - 1))
         _lib.call("dlp_frontier_solve", ptr(rbeg), ptr(rend), ptr(W.indices), ptr(W.data), code(W.data), W.shape[0],
                   self.C, ptr(X), ld(X), ptr(rhs), ld(rhs), ptr(diag), code(X), float(delta), ptr(f), int(f.numel()),
-                  int(max_rounds), self.gs, W.nnz / max(W.shape[0], 1), ptr(ws), ws.numel(), ct.byref(rounds),
+                  cap, self.gs, W.nnz / max(W.shape[0], 1), ptr(ws), ws.numel(), ct.byref(rounds),
                   ct.byref(edges), stream())
         self.edges += int(edges.value)
         return int(rounds.value)

@@ -127,3 +127,15 @@ def test_product_without_room_for_its_scratch(monkeypatch):
     monkeypatch.undo()
     want = kernels.spmm_axpy(CSR(W.data.double(), W.indices, W.indptr, W.shape), X.double())
     assert float((Y.double() - want).abs().max()) <= 16 * 16 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("cap", [0, 2.5, 2**31 - 1, 2**31, 2**33 + 5, float("inf")])
+def test_frontier_solve_takes_any_cap(cap):
+    """The number of rounds of the device loop under caps beyond an int32, infinite and fractional, against the host
+    loop's."""
+    n = 3000
+    ds, lab = labelled_graph(n)
+    S = stream.build_system(ds, torch.ones_like(lab), lab)
+    a, b = (solvers.DynLP(n, 3, max_iter=cap) for _ in range(2))
+    sa, sb = a.solve(S), b.solve(S, record=[])
+    assert sa.iters == sb.iters and torch.equal(a.F, b.F) and (sa.iters > 100 or cap < 3)
