@@ -162,8 +162,11 @@ def build_system(ds: Dataset, active, labeled, *, eta=0.0, dtype="float32", t=0,
     dev = A.indices.device
     n = A.shape[0]
     dt = to_dtype(dtype)
-    active = active.to(torch.bool).contiguous()  # bound to their names: the kernels get bare addresses
-    labeled = labeled.to(torch.bool).contiguous()
+    # n flags each (any other length raises), bound to their names: the kernels get bare addresses
+    active = active.to(torch.bool).expand(n).contiguous()
+    labeled = labeled.to(torch.bool).expand(n).contiguous()
+    if ds.y.numel() < n:
+        raise IndexError(f"{ds.y.numel()} labels for {n} vertices")
     C = 1 if K == 2 else K
     f64 = torch.float64
     masks = torch.empty((2, max(n, 1)), dtype=torch.uint8, device=dev)  # U, and the active labelled vertices

@@ -139,3 +139,23 @@ def test_frontier_solve_takes_any_cap(cap):
     a, b = (solvers.DynLP(n, 3, max_iter=cap) for _ in range(2))
     sa, sb = a.solve(S), b.solve(S, record=[])
     assert sa.iters == sb.iters and torch.equal(a.F, b.F) and (sa.iters > 100 or cap < 3)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_build_system_refuses_masks_and_labels_of_another_length(dtype):
+    ds, lab = labelled_graph(1000)
+    on = torch.ones_like(lab)
+    for m in (0, 2, 999, 1001):
+        long = torch.ones(m, dtype=torch.bool, device="cuda")
+        for a, b in ((long, lab), (on, long), (long, long)):
+            with pytest.raises(RuntimeError):
+                stream.build_system(ds, a, b, dtype=dtype)
+    with pytest.raises(RuntimeError):
+        stream.build_system(ds, on[:, None], lab, dtype=dtype)
+    short = graphs.Dataset("x", ds.A, ds.y[:999], ds.K, ds.order)
+    with pytest.raises(IndexError):
+        stream.build_system(short, on, lab, dtype=dtype)
+    # one flag for all, and labels beyond the graph's vertices, are taken as before
+    want = stream.build_system(ds, on, lab, dtype=dtype)
+    more = graphs.Dataset("x", ds.A, torch.cat([ds.y, ds.y[:5]]), ds.K, ds.order)
+    same_system(stream.build_system(more, on[:1], lab, dtype=dtype), want)
