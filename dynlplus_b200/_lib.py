@@ -156,7 +156,7 @@ class Cancelled(DLPError):
     """A device-side loop stopped because the registered cancel word was set (DLP_ERR_CANCELLED)."""
 
 
-DLP_ERR_CAP, DLP_ERR_CANCELLED = 4, 5
+DLP_ERR_INVALID, DLP_ERR_CAP, DLP_ERR_CANCELLED = 1, 4, 5
 
 
 def call(name: str, *args, allow: tuple = ()) -> int:

@@ -110,18 +110,24 @@ def fh_components(m, rows, cols, d, k, ground=None):
     dev = rows.device
     if m == 0 or not rows.numel():
         return torch.arange(m, dtype=torch.int32, device=dev), m
+    if cols.shape != rows.shape or d.shape != rows.shape or rows.dim() != 1:
+        raise IndexError(f"{tuple(rows.shape)}, {tuple(cols.shape)} and {tuple(d.shape)} edge ends and weights")
+    if ground is not None and ground.shape != (m,):
+        raise IndexError(f"ground of shape {tuple(ground.shape)} for {m} vertices")
     rows, cols = rows.to(torch.int32).contiguous(), cols.to(torch.int32).contiguous()
     d = d.to(torch.float32).contiguous()
     g = ground.to(torch.float32).contiguous() if ground is not None else None
     root = torch.empty(m, dtype=torch.int32, device=dev)
-    ec = torch.zeros(2, dtype=torch.int32, device=dev)  # [a wait ran out, component count]
+    ec = torch.zeros(2, dtype=torch.int32, device=dev)  # [error, component count]
     ws = workspace("fh").get(_lib.lib().dlp_fh_components_workspace_bytes(m))
     _lib.call("dlp_fh_components", int(m), int(rows.numel()), ptr(rows), ptr(cols), ptr(d), float(k), ptr(g), ptr(root),
               ptr(ec), ptr(ws), ws.numel(), stream())
     lab, _ = relabel(root, sync=False, count=ec[1:])
     err, nc = ec.tolist()
+    if err == _lib.DLP_ERR_INVALID:
+        raise IndexError(f"fh_components: edge end outside [0, {m})")
     if err:
-        raise _lib.DLPError("dlp_fh_components", 8)
+        raise _lib.DLPError("dlp_fh_components", err)
     return lab, nc
 
 

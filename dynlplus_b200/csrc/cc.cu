@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
 struct FhCtl {
   GridBar bar;
   int32_t ext[2], ok[2];  // this round saw an outgoing edge / a permitted merge, by the round's parity
+  int32_t bad;            // an edge's end outside [-m, m): nothing is merged
 };
 
 __device__ __forceinline__ uint32_t float_order(float x) {  // monotone in the float's order
@@ -436,14 +437,24 @@ __global__ void __launch_bounds__(kFhThreads, 1)
     best[v] = 0xffffffffu;
     nb[v] = m;
   }
+  bool wrong = false;
+  for (long long e = t0; e < E; e += step)
+    wrong |= rows[e] < -m || rows[e] >= m || cols[e] < -m || cols[e] >= m;
+  if (wrong) {
+    atomicExch(err, DLP_ERR_INVALID);
+    atomicExch(&ctl->bad, 1);
+  }
   if (!barrier()) return;
+  if (__ldcg(&ctl->bad)) return;
+  // the component of an edge's end (a negative one counts from the last vertex, as an index does)
+  auto component = [&](int32_t v) { return __ldcg(lab + (v < 0 ? v + m : v)); };
   bool fh = true;
   for (int round = 0;; ++round) {
     const int p = round & 1;
     // the lightest outgoing edge of every component (of the ungrounded ones once fh is over)
     bool any = false;
     for (long long e = t0; e < E; e += step) {
-      const int32_t cu = __ldcg(lab + rows[e]), cv = __ldcg(lab + cols[e]);
+      const int32_t cu = component(rows[e]), cv = component(cols[e]);
       if (cu == cv || (!fh && __ldcg(grounded + cu))) continue;
       any = true;
       atomicMin(best + cu, float_order(d[e]));
@@ -453,7 +464,7 @@ __global__ void __launch_bounds__(kFhThreads, 1)
     if (!barrier()) return;
     if (__ldcg(&ctl->ext[p]) == 0) break;
     for (long long e = t0; e < E; e += step) {
-      const int32_t cu = __ldcg(lab + rows[e]), cv = __ldcg(lab + cols[e]);
+      const int32_t cu = component(rows[e]), cv = component(cols[e]);
       if (cu == cv || (!fh && __ldcg(grounded + cu))) continue;
       if (float_order(d[e]) == __ldcg(best + cu)) {
         atomicMin(nb + cu, cv);

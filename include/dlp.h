@@ -264,8 +264,9 @@ int dlp_build_system_fill(int32_t n, const int32_t *indptr, const int32_t *col, 
 /* Felzenszwalb-Huttenlocher merging (dynlp/cc.py:37-73) of m vertices over E weighted edges (both
  * directions stored): Boruvka rounds on the device in one cooperative launch; with ground (m floats,
  * may be NULL) components without any then join their lightest neighbour. root[v] = the smallest vertex
- * of v's component (dlp_cc_relabel numbers them). *err (device int, caller-zeroed) is set when a wait on
- * the device ran out. Asynchronous. */
+ * of v's component (dlp_cc_relabel numbers them). Ends in [-m, 0) count from the last vertex. *err (device
+ * int, caller-zeroed) becomes DLP_ERR_INVALID when an end lies outside [-m, m) (no vertices are merged then),
+ * DLP_ERR_DEVICE when a wait on the device ran out. Asynchronous. */
 size_t dlp_fh_components_workspace_bytes(int32_t m);
 int dlp_fh_components(int32_t m, int64_t E, const int32_t *rows, const int32_t *cols, const float *d, double k,
                       const float *ground, int32_t *root, int32_t *err, void *ws, size_t ws_bytes, dlp_stream_t stream);

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from dynlplus_b200 import batched, graphs, kernels, solvers, stream
+from dynlplus_b200 import batched, cc, graphs, kernels, solvers, stream
 from dynlplus_b200.backend import CSR
 
 pytestmark = pytest.mark.gpu
@@ -159,3 +159,28 @@ def test_build_system_refuses_masks_and_labels_of_another_length(dtype):
     want = stream.build_system(ds, on, lab, dtype=dtype)
     more = graphs.Dataset("x", ds.A, torch.cat([ds.y, ds.y[:5]]), ds.K, ds.order)
     same_system(stream.build_system(more, on[:1], lab, dtype=dtype), want)
+
+
+@pytest.mark.parametrize("m", [3, 2000])
+def test_fh_components_checks_its_edges(m):
+    """Edge ends, weights and grounding of other lengths and ends outside [0, m) are refused; ends counted from the
+    last vertex are taken as indices are."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    u = torch.randint(0, m - 1, (4 * m,), generator=g, device="cuda")
+    v = (u + 1 + torch.randint(0, m - 1, (4 * m,), generator=g, device="cuda")) % m
+    rows, cols = torch.cat([u, v]), torch.cat([v, u])
+    d = torch.rand(4 * m, generator=g, device="cuda").repeat(2)
+    ground = (torch.arange(m, device="cuda") % 7 == 0).float()
+    want, nc = cc.fh_components(m, rows, cols, d, 0.3, ground)
+    lab, n2 = cc.fh_components(m, rows - m, torch.where(cols % 2 == 0, cols - m, cols), d, 0.3, ground)
+    assert n2 == nc and torch.equal(lab, want)
+    for a, b, c, gr in ((rows, cols[:-1], d, ground), (rows, cols, d[:1], ground), (rows, cols, d, ground[:-1]),
+                        (rows, cols, torch.cat([d, d]), None), (rows, cols, d, torch.cat([ground, ground]))):
+        with pytest.raises(IndexError):
+            cc.fh_components(m, a, b, c, 0.3, gr)
+    for side in (0, 1):
+        for value in (m, -m - 1, 2**31 - 1):
+            ends = [rows.clone(), cols.clone()]
+            ends[side][-1] = value
+            with pytest.raises(IndexError):
+                cc.fh_components(m, *ends, d, 0.3, ground)
