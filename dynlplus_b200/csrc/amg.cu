@@ -192,15 +192,9 @@ static int sort_members(int32_t n, int32_t nc, const int32_t *off, int32_t *memb
   k_sort_members<<<g1(32LL * nc), kAT, 0, s>>>(nc, off, members);
   DLP_TRY(check_launch());
   const size_t bits = ((size_t)n + 31) / 32 * 4;
-  static const size_t most = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    v -= 4096;  // the kernel's own arrays
-    return v > 0 && cudaFuncSetAttribute((const void *)k_sort_members_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         v) == cudaSuccess ? (size_t)v : (size_t)0;
-  }();
-  if (bits <= most)
+  static std::atomic<uint64_t> allowed{0};
+  const int most = most_smem(4096);  // 4096: the kernel's own arrays
+  if (bits <= (size_t)most && allow_smem(allowed, (const void *)k_sort_members_long, most))
     k_sort_members_long<<<std::min(sm_count(), nc), kAT, bits, s>>>(n, nc, off, members);
   else
     k_sort_members_serial<<<g1(nc), kAT, 0, s>>>(nc, off, members);

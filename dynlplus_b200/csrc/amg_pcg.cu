@@ -639,14 +639,9 @@ int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_s
     // one launch where the blocks' rows and the pivot row fit shared memory (up to some 1,900 rows)
     const int rows = (n + sm_count() - 1) / sm_count();
     const size_t smem = ((size_t)rows + 1) * n * sizeof(double);
-    static const int most = [] {
-      int dev = 0, v = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-      v -= 1024;
-      return cudaFuncSetAttribute((const void *)k_gj_whole, cudaFuncAttributeMaxDynamicSharedMemorySize, v) == cudaSuccess ? v : 0;
-    }();
-    if (smem <= (size_t)most) {
+    static std::atomic<uint64_t> allowed{0};
+    const int most = most_smem(1024);
+    if (smem <= (size_t)most && allow_smem(allowed, (const void *)k_gj_whole, most)) {
       GridBar *bar = (GridBar *)((char *)ws + 2 * al256a(sizeof(double) * (size_t)n));
       DLP_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), s));
       int32_t nn = n, rr = rows;

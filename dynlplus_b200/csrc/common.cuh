@@ -8,6 +8,7 @@
 #include <memory>
 
 #include "dlp.h"
+#include "per_device.h"
 
 namespace dlp {
 
@@ -54,6 +55,27 @@ struct GraphExec {
   }
 };
 using GraphRef = std::shared_ptr<GraphExec>;
+
+// Whether `kernel` may be launched on the current device with up to `bytes` of dynamic shared memory: an attribute of
+// the kernel on one device, so `done` (one per kernel) remembers the devices it was raised on.
+inline bool allow_smem(std::atomic<uint64_t> &done, const void *kernel, int bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return once_per_device(done, dev, [&] {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e == cudaSuccess;
+  });
+}
+
+// The most dynamic shared memory a block of the current device can have beside `own` bytes of static memory.
+inline int most_smem(int own) {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    (void)cudaGetLastError();
+  return v > own ? v - own : 0;
+}
 
 inline size_t dtype_size(int dt) { return dt == DLP_F64 ? 8 : dt == DLP_F32 ? 4 : dt == DLP_BF16 ? 2 : 0; }
 

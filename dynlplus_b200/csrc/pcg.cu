@@ -1769,12 +1769,13 @@ static size_t whole_state(const PcgProblem &q, int rows) {
   return (size_t)rows * (4 * es * q.C + es + 8 + 8) + 64;
 }
 
+// kNotLaunched: this device does not give the kernel its shared memory; the launched loop takes the solve.
+constexpr int kNotLaunched = -1;
 template <class T, int VW>
 static int launch_whole_t(WholeArgs<T> &a, cudaStream_t s) {
   auto *kern = k_pcg_whole<T, VW>;
-  static const cudaError_t set =
-      cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSmem);
-  DLP_CUDA(set);
+  static std::atomic<uint64_t> allowed{0};
+  if (!allow_smem(allowed, (const void *)kern, kWholeSmem)) return kNotLaunched;
   void *argv[] = {(void *)&a};
   const int grid = (a.n + a.rows - 1) / a.rows;
   DLP_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kWholeThreads), argv, kWholeSmem, s));
@@ -1892,17 +1893,20 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
   // iterations against 426 and a lost iterate).
   const bool floor_recheck = q.fused && !(mode & 16) && (mode & 2);
   if (use_graph && !(mode & 8) && !floor_recheck && whole_fits(q, &whole)) {
-    DLP_TRY(whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s));
-    PcgCtl cur{};
-    DLP_TRY(read_ctl(B, hs, s, &cur));
-    if (cur.done == 0) return DLP_ERR_DEVICE;  // a barrier's wait ran out
-    if (iters_out) *iters_out = cur.iters;
-    if (viol_out) *viol_out = cur.viol;
-    if (relres_out) *relres_out = cur.relres;
-    if (status_out) *status_out = cur.done;
-    if (cur.done == 3) return DLP_ERR_CAP;
-    if (cur.done == 6) return DLP_ERR_CANCELLED;
-    return DLP_OK;
+    const int st = whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s);
+    if (st != DLP_OK && st != kNotLaunched) return st;
+    if (st == DLP_OK) {
+      PcgCtl cur{};
+      DLP_TRY(read_ctl(B, hs, s, &cur));
+      if (cur.done == 0) return DLP_ERR_DEVICE;  // a barrier's wait ran out
+      if (iters_out) *iters_out = cur.iters;
+      if (viol_out) *viol_out = cur.viol;
+      if (relres_out) *relres_out = cur.relres;
+      if (status_out) *status_out = cur.done;
+      if (cur.done == 3) return DLP_ERR_CAP;
+      if (cur.done == 6) return DLP_ERR_CANCELLED;
+      return DLP_OK;
+    }
   }
   // R = rhs - A Z, best = violation, rz = R.(R/diag), P = R/diag; a zero start takes R = rhs in the
   // update sweep itself and sets Z = 0 in the direction sweep (no SpMM, no separate copy)
