@@ -24,12 +24,18 @@ def _roots(n, rows, cols, err) -> torch.Tensor:
     return parent[:n]
 
 
+def _raise_on(err):
+    if err < 0:
+        raise _lib.DLPError("dlp_cc_edges_ws", -err)
+    if err:
+        raise ValueError("connected_components: edge endpoint outside [0, n)")
+
+
 def min_vertex_roots(n, rows, cols) -> torch.Tensor:
     """parent[v] = smallest vertex id in v's component (int32, device)."""
     err = torch.zeros(1, dtype=torch.int32, device=rows.device)
     parent = _roots(n, rows, cols, err)
-    if int(err.item()):
-        raise ValueError("connected_components: edge endpoint outside [0, n)")
+    _raise_on(int(err.item()))
     return parent
 
 
@@ -52,8 +58,7 @@ def connected_components(n, rows, cols):
     ec = torch.zeros(2, dtype=torch.int32, device=rows.device)  # [error, count]
     label, _ = relabel(_roots(n, rows, cols, ec[:1]), sync=False, count=ec[1:])
     err, nc = ec.tolist()
-    if err:
-        raise ValueError("connected_components: edge endpoint outside [0, n)")
+    _raise_on(err)
     return label, nc
 
 

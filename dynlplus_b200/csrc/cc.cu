@@ -98,6 +98,7 @@ __device__ __forceinline__ int32_t ld_l1(const int32_t *p) {
   return v;
 }
 constexpr int kCcRounds = 64;
+constexpr int32_t kCcLost = -DLP_ERR_DEVICE;  // *err of a lost wait (an edge's end out of range: DLP_ERR_DEVICE)
 // Where the rounds are used: half a million edges on, and a mean degree above one, where a giant component
 // can form. Below, the unions meet on no common root and are done sooner (whole calls, us, unions / rounds:
 // n = 2M, degree 0.8, 148 / 218; n = 400,000, degree 1.2, 153 / 169; n = 2M, degree 1.5, 1,136 / 298).
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(kCcRoundThreads, 2)
   uint32_t target = 0;
   auto barrier = [&]() -> bool {
     if (grid_barrier(&ctl->bar, target)) return true;
-    if (t0 == 0) atomicExch(err, DLP_ERR_DEVICE);
+    if (threadIdx.x == 0) atomicExch(err, kCcLost);
     return false;
   };
   for (long long v = t0; v < n; v += step) parent[v] = (int32_t)v;
@@ -319,6 +320,11 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   const bool first = t0 == 0;
   uint32_t target = 0;
+  auto barrier = [&]() -> bool {
+    if (grid_barrier(bar, target)) return true;
+    if (threadIdx.x == 0) atomicExch(info + 3, 1);
+    return false;
+  };
   int sweeps = 0;
   bool settled = false;
   while (!settled && sweeps < kReachMaxSweeps) {  // flags and reached were cleared before the launch
@@ -342,19 +348,13 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
       }
     }
     if (__syncthreads_or(any) && threadIdx.x == 0) atomicAdd(flags + sweeps, 1);
-    if (!grid_barrier(bar, target)) {
-      if (first) info[3] = 1;
-      return;
-    }
+    if (!barrier()) return;
     settled = __ldcg(flags + sweeps) == 0;
     ++sweeps;
   }
   if (!settled) {
     for (long long v = t0; v <= n; v += step) parent[v] = (int32_t)v;
-    if (!grid_barrier(bar, target)) {
-      if (first) info[3] = 1;
-      return;
-    }
+    if (!barrier()) return;
     for (long long u = t0; u < n; u += step) {
       if (vmask && !vmask[u]) continue;
       for (int j = rbeg[u]; j < rend[u]; ++j) {
@@ -365,10 +365,7 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
         else if (sink && sink[v]) unite(parent, (int32_t)u, n, err);
       }
     }
-    if (!grid_barrier(bar, target)) {
-      if (first) info[3] = 1;
-      return;
-    }
+    if (!barrier()) return;
   }
   const int32_t root = settled ? 0 : find_root(parent, n, err);
   int changes = 0, active = 0, lost = 0;
@@ -426,7 +423,7 @@ __global__ void __launch_bounds__(kFhThreads, 1)
   uint32_t target = 0;
   auto barrier = [&]() -> bool {
     if (grid_barrier(&ctl->bar, target)) return true;
-    if (t0 == 0) atomicExch(err, DLP_ERR_DEVICE);
+    if (threadIdx.x == 0) atomicExch(err, DLP_ERR_DEVICE);
     return false;
   };
   for (long long v = t0; v < m; v += step) {

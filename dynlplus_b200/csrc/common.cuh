@@ -134,8 +134,10 @@ __device__ __forceinline__ void atomic_add(double *p, double v) { atomicAdd(p, v
 // A monotone arrival counter (zeroed by the host before the launch): barrier k is passed when
 // k * gridDim.x blocks have arrived. Every block of the launch is resident (cooperative launch), so a
 // wait ends with the slowest block; the spin is bounded all the same (kBarSpins polls, seconds), and a
-// block that gives up sets `abort`, which ends every other block's wait. Data written by other blocks
-// before the barrier is read through L2 (__ldcg) after it.
+// block that gives up sets `abort`, which ends every other block's wait. A block may give up where the others
+// pass (the last arrival comes between its last poll and its limit), so a caller learns of a lost wait from
+// `abort` or from a word that every block which gives up writes, never from one block's return alone. Data
+// written by other blocks before the barrier is read through L2 (__ldcg) after it.
 struct GridBar {
   uint32_t count;
   int32_t abort;

@@ -36,7 +36,8 @@ struct PcgCtl {
   uint32_t cnt1, cnt2;
   int32_t mode, patience;
   int32_t max_iter, bad;  // bad: non-finite residual entries seen (breakdown)
-  int32_t par, pad;       // two-kernel iteration: which of P / AP holds the current direction
+  int32_t par;            // two-kernel iteration: which of P / AP holds the current direction
+  int32_t lost;           // the one-launch solve: a block's wait ran out (its rows may be missing)
   double best, viol, relres, target;
   // first-level counters of the grid reductions (last_block_grouped), one per group of blocks;
   // zero between launches. The host reads only the fields above them (kCtlHead).
@@ -1898,7 +1899,7 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
     if (st == DLP_OK) {
       PcgCtl cur{};
       DLP_TRY(read_ctl(B, hs, s, &cur));
-      if (cur.done == 0) return DLP_ERR_DEVICE;  // a barrier's wait ran out
+      if (cur.lost || cur.done == 0) return DLP_ERR_DEVICE;  // a barrier's wait ran out
       if (iters_out) *iters_out = cur.iters;
       if (viol_out) *viol_out = cur.viol;
       if (relres_out) *relres_out = cur.relres;

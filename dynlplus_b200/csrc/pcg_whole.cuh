@@ -192,7 +192,11 @@ __global__ void __launch_bounds__(kWholeThreads, 1) k_pcg_whole(WholeArgs<T> p) 
   uint32_t target = 0;
 
   // Every block's stores before the barrier are visible through L2 after it; false when a wait ran out.
-  auto barrier = [&]() -> bool { return grid_barrier(p.bar, target); };
+  auto barrier = [&]() -> bool {
+    if (grid_barrier(p.bar, target)) return true;
+    if (tid == 0) atomicExch(&B.ctl->lost, 1);
+    return false;
+  };
   // Sum over all blocks of NO outputs, per-thread values in s_v: outputs 0..C-1 from s_v[0], C..2C-1 from
   // s_v[1], 2C the maximum of s_v[2], 2C + 1 block 0's read of the cancel word. One warp per output, block
   // sums and then the blocks in fixed orders; the results are in s_red (alpha: rz / sum instead of the sum).

@@ -499,12 +499,13 @@ int dlp_fused_push(const int32_t *rbeg, const int32_t *rend, const int32_t *col,
   }
   DLP_CUDA(cudaMemcpyAsync(&out, W.ctl, sizeof(out), cudaMemcpyDeviceToHost, s));
   DLP_CUDA(cudaStreamSynchronize(s));
+  // a wait ran out in a block, or the loop ended without a decision
+  if (out.bar.abort || out.status == kRunning) return DLP_ERR_DEVICE;
   if (rounds_out) *rounds_out = out.rounds;
   if (converged_out) *converged_out = out.status == kConverged ? 1 : 0;
   if (edges_out) *edges_out = out.edges;
   if (out.status == kCapped) return DLP_ERR_CAP;
   if (out.status == kCancelled) return DLP_ERR_CANCELLED;
-  if (out.status != kConverged) return DLP_ERR_DEVICE;  // the loop ended without a decision
   return DLP_OK;
 }
 

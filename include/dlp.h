@@ -190,7 +190,7 @@ int dlp_colreduce(int kind, int32_t n, int32_t C, const void *X, int64_t ldx, co
 int dlp_cc_edges(int32_t n, const int32_t *rows, const int32_t *cols, int64_t m, int32_t *parent, int32_t *err,
                  dlp_stream_t stream);
 /* The same with scratch (dlp_cc_edges_workspace_bytes; err required): long edge lists run in rounds in one
- * cooperative launch, same result. *err is also set when a wait on the device ran out. */
+ * cooperative launch, same result. *err becomes -DLP_ERR_DEVICE when a wait on the device ran out. */
 size_t dlp_cc_edges_workspace_bytes(void);
 int dlp_cc_edges_ws(int32_t n, const int32_t *rows, const int32_t *cols, int64_t m, int32_t *parent, int32_t *err,
                     void *ws, size_t ws_bytes, dlp_stream_t stream);

@@ -184,3 +184,50 @@ def test_fh_components_checks_its_edges(m):
             ends[side][-1] = value
             with pytest.raises(IndexError):
                 cc.fh_components(m, *ends, d, 0.3, ground)
+
+
+LOST_WAIT = r"""
+#include "cc.cu"
+// The grounding kernel as it is launched, on two blocks, with its barrier's `abort` set beforehand: a block that has to
+// wait gives up after its first 1,024 polls, the block that arrives last finds every arrival and passes.
+extern "C" int lost_wait(int32_t n, const int32_t *rbeg, const int32_t *rend, const int32_t *col, const float *w,
+                         const uint8_t *vmask, const uint8_t *sink, uint8_t *umask, uint8_t *in_t, int32_t *count,
+                         int32_t *err, int32_t *info, uint8_t *reached, int32_t *flags, int32_t *parent, GridBar *bar) {
+  GridBar b{};
+  b.abort = 1;
+  cudaMemcpy(bar, &b, sizeof(b), cudaMemcpyHostToDevice);
+  void *args[] = {&n,     &rbeg, &rend,  &col, &w,    &vmask,   &sink,  &reached,
+                  &flags, &parent, &umask, &in_t, &count, &err, &info, &bar};
+  const void *kern = (const void *)k_ground_whole<float>;
+  cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(2), dim3(kGroundThreads), args, 0, nullptr);
+  return e != cudaSuccess ? (int)e : (int)cudaDeviceSynchronize();
+}
+"""
+
+
+def test_a_wait_lost_in_any_block_is_reported(tmp_path):
+    """Block 1 of the grounding gives up at the only barrier of a run, block 0 (it has one long row) passes and
+    writes its rows: the run says that a wait was lost, since block 1's rows are missing."""
+    import ctypes as ct
+    import subprocess
+    from dynlplus_b200 import _lib, build
+    from dynlplus_b200.backend import ptr
+    _lib.lib()
+    src, so = tmp_path / "lost_wait.cu", tmp_path / "lost_wait.so"
+    src.write_text(LOST_WAIT)
+    subprocess.run([build.nvcc(), *build.ARCH, *build.FLAGS, "-shared", "-cudart", "static", str(src), "-o", str(so),
+                    build.LIB], check=True)
+    n, m = 2048, 200_000
+    rend = torch.full((n,), m, dtype=torch.int32, device="cuda")
+    rbeg = rend.clone()
+    rbeg[0] = 0  # row 0 has all the entries, none of them to a reached vertex
+    col = torch.full((m,), 5, dtype=torch.int32, device="cuda")
+    i32, u8 = (lambda k: torch.zeros(k, dtype=torch.int32, device="cuda")), (lambda k: torch.zeros(k, dtype=torch.uint8, device="cuda"))
+    vmask, sink, umask, in_t, w = u8(n) + 1, u8(n), u8(n) + 1, u8(n), torch.ones(m, device="cuda")
+    count, err, info, reached, flags, parent, bar = i32(1), i32(1), i32(4), u8(n), i32(64), i32(n + 1), i32(64)
+    torch.cuda.synchronize()
+    args = [ct.c_void_p(ptr(t)) for t in (rbeg, rend, col, w, vmask, sink, umask, in_t, count, err, info, reached, flags,
+                                          parent, bar)]
+    assert ct.CDLL(str(so)).lost_wait(ct.c_int32(n), *args) == 0
+    assert int(umask[:1024].sum()) == 0 and int(umask[1024:].sum()) == 1024  # block 0 finished, block 1 did not
+    assert int(info[3]) == 1
