@@ -326,13 +326,15 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
     return false;
   };
   int sweeps = 0;
+  uint32_t walked = 0;
   bool settled = false;
   while (!settled && sweeps < kReachMaxSweeps) {  // flags and reached were cleared before the launch
     bool any = false;
     for (long long u = t0; u < n; u += step) {
       if ((vmask && !vmask[u]) || reached[u]) continue;
-      const int end = rend[u];
-      for (int j = rbeg[u]; j < end; ++j) {
+      const int beg = rbeg[u], end = rend[u];
+      bar_announce(bar, end - beg, walked);
+      for (int j = beg; j < end; ++j) {
         if (!live(w, j)) continue;
         const int32_t v = col[j];
         if ((unsigned)v >= (unsigned)n) {
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
     if (!barrier()) return;
     for (long long u = t0; u < n; u += step) {
       if (vmask && !vmask[u]) continue;
+      bar_announce(bar, rend[u] - rbeg[u], walked);
       for (int j = rbeg[u]; j < rend[u]; ++j) {
         if (!live(w, j)) continue;
         const int32_t v = col[j];

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int r0 = __ldcg(&ctl->round);
-  uint32_t bar = 0;
+  uint32_t bar = 0, walked = 0;
   unsigned long long edges = 0;
   int done = 0, status = 0;
   for (; done < p.max_rounds; ++done) {
@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
       const int r = valid ? __ldcg(front + gi) : 0;
       const int beg = valid ? p.rbeg[r] : 0;
       const int end = valid ? p.rend[r] : 0;
+      bar_announce(&ctl->bar, end - beg, walked);
       TA acc[VPL][VW];
       gather_row<typename T::TW, TX, TA, VW, VPL, gather_batch_wide<TA, VW, VPL>(), kRowVec, true>(
           p.col, p.w, p.X, p.ldx, beg, end, es, ES, cl, LV, NV, G, acc);
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
       const int gi = valid ? __ldcg(p.upd + i) : 0;
       const int r = valid ? __ldcg(front + gi) : 0;
       const int beg = valid ? p.rbeg[r] : 0, end = valid ? p.rend[r] : 0;
+      bar_announce(&ctl->bar, end - beg, walked);
       if (valid)
         for (int c = lane & 7; c < p.C; c += 8)
           p.X[(long long)r * p.ldx + c] = __ldcg(p.Y + (long long)gi * p.C + c);

@@ -92,6 +92,7 @@ __device__ __forceinline__ void push_scatter(const PushArgs<T> &a, int p, int nf
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long stride = (((long long)gridDim.x * blockDim.x) >> 5) * kGroups;
   unsigned long long my_edges = 0;
+  uint32_t walked = 0;
   for (long long base = warp * kGroups; base < nf; base += stride) {  // warp-uniform bounds
     const long long g = base + lane / G;
     const bool valid = g < nf;
@@ -103,6 +104,7 @@ __device__ __forceinline__ void push_scatter(const PushArgs<T> &a, int p, int nf
       const int u = __ldcg(a.front + g);
       beg = a.rbeg[u];
       end = a.rend[u];
+      bar_announce(&ctl->bar, end - beg, walked);
       const T *dr = a.D + g * a.C;
 #pragma unroll
       for (int k = 0; k < DC; ++k)

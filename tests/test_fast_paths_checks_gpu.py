@@ -231,3 +231,33 @@ def test_a_wait_lost_in_any_block_is_reported(tmp_path):
     assert ct.CDLL(str(so)).lost_wait(ct.c_int32(n), *args) == 0
     assert int(umask[:1024].sum()) == 0 and int(umask[1024:].sum()) == 1024  # block 0 finished, block 1 did not
     assert int(info[3]) == 1
+
+
+@pytest.mark.parametrize("call", ["grounding", "frontier", "push"])
+def test_a_hub_keeps_the_other_blocks_waiting(call):
+    """A vertex of 8 million neighbours, whose row one thread or lane group walks for seconds while every other block
+    waits at the barrier: the wait is as long as the row, and the result is the star graph's."""
+    n = 8_000_000
+    ip = torch.cat([torch.zeros(1, dtype=torch.int32, device="cuda"), torch.arange(n - 1, 2 * n - 1, device="cuda").to(torch.int32)])
+    col = torch.cat([torch.arange(1, n, device="cuda"), torch.zeros(n - 1, dtype=torch.int64, device="cuda")]).to(torch.int32)
+    A = CSR(torch.ones(2 * n - 2, device="cuda"), col, ip, (n, n))
+    hub = torch.zeros(1, dtype=torch.int32, device="cuda")
+    diag = torch.full((n,), 2.0, dtype=torch.float64, device="cuda")
+    diag[0] = n
+    if call == "grounding":  # the hub's last neighbour is the only labelled vertex
+        sink = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        sink[-1] = 1
+        umask, in_t = torch.zeros_like(sink), torch.zeros_like(sink)
+        assert cc.ground_reach(A, 1 - sink, sink, umask, in_t)[0] == n - 1
+        assert torch.equal(umask, 1 - sink)
+    elif call == "frontier":  # the hub moves to (n - 1) / 2 / n, then the leaves to half of it
+        X = torch.full((n, 1), 0.5, dtype=torch.float64, device="cuda")
+        rounds = kernels.FrontierOps(A, 1).solve(hub, X, torch.zeros_like(X), diag, 1e-9, 2)
+        assert rounds == 2 and abs(float(X[0, 0]) - 0.5 * (n - 1) / n) <= 1e-9
+        assert float((X[1:] - 0.25).abs().max()) <= 1e-6
+    else:  # the hub's residual n becomes a score of 1 and a residual of 1 at every leaf
+        Z, R = torch.zeros((n, 1), dtype=torch.float64, device="cuda"), torch.zeros((n, 1), dtype=torch.float64, device="cuda")
+        R[0] = float(n)
+        rounds, ok, edges = kernels.FusedPush(A, 1).run(Z, R, diag, [0.9], hub, 5)
+        assert (rounds, ok, edges) == (1, True, n - 1) and float(Z[0, 0]) == 1.0
+        assert bool((R[1:] == 1.0).all()) and float(R[0, 0]) == 0.0
