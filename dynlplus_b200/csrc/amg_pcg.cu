@@ -646,13 +646,14 @@ int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_s
       DLP_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), s));
       int32_t nn = n, rr = rows;
       void *args[] = {(void *)&nn, (void *)&rr, (void *)&A, (void *)&fcol, (void *)&bar};
-      DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_gj_whole, dim3((n + rows - 1) / rows), dim3(kGjThreads), args,
-                                           smem, s));
-      DLP_TRY(check_launch());
-      int32_t lost = 0;  // setup reads back anyway; a wait that ran out must not pass as an inverse
-      DLP_CUDA(cudaMemcpyAsync(&lost, &bar->abort, sizeof(lost), cudaMemcpyDeviceToHost, s));
-      DLP_CUDA(cudaStreamSynchronize(s));
-      return lost ? DLP_ERR_DEVICE : DLP_OK;
+      const int st = launch_cooperative((const void *)k_gj_whole, (n + rows - 1) / rows, kGjThreads, args, smem, s);
+      if (st != DLP_OK && st != kNotLaunched) return st;
+      if (st == DLP_OK) {
+        int32_t lost = 0;  // setup reads back anyway; a wait that ran out must not pass as an inverse
+        DLP_CUDA(cudaMemcpyAsync(&lost, &bar->abort, sizeof(lost), cudaMemcpyDeviceToHost, s));
+        DLP_CUDA(cudaStreamSynchronize(s));
+        return lost ? DLP_ERR_DEVICE : DLP_OK;
+      }
     }
   }
   const int g1 = ceil_div_i(n, 256);

@@ -699,8 +699,7 @@ int dlp_cc_edges_ws(int32_t n, const int32_t *rows, const int32_t *cols, int64_t
   long long mm = m;
   void *args[] = {(void *)&n, (void *)&rows, (void *)&cols, (void *)&mm, (void *)&parent, (void *)&err, (void *)&ctl};
   const int grid = (int)std::min((long long)sm_count() * per, (std::max((long long)n, mm) + kCcRoundThreads - 1) / kCcRoundThreads);
-  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_cc_rounds, dim3(grid), dim3(kCcRoundThreads), args, 0, s));
-  return check_launch();
+  return launch_any_grid((const void *)k_cc_rounds, grid, kCcRoundThreads, args, 0, s);
 }
 
 size_t dlp_cc_graph_workspace_bytes(void) { return 256; }
@@ -848,8 +847,7 @@ int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, 
     void *args[] = {(void *)&n,     (void *)&rbeg,  (void *)&rend,   (void *)&col,   (void *)&wp,   (void *)&vmask,
                     (void *)&sink,  (void *)&reached, (void *)&flags, (void *)&parent, (void *)&umask, (void *)&in_t,
                     (void *)&count, (void *)&err,   (void *)&info,   (void *)&bar};
-    DLP_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kGroundThreads), args, 0, s));
-    return check_launch();
+    return launch_any_grid((const void *)kern, grid, kGroundThreads, args, 0, s);
   };
   if (!w || w_dtype == DLP_F32) return launch(k_ground_whole<float>, (const float *)w);
   if (w_dtype == DLP_F64) return launch(k_ground_whole<double>, (const double *)w);
@@ -903,8 +901,7 @@ int dlp_fh_components(int32_t m, int64_t E, const int32_t *rows, const int32_t *
                   (void *)&ground,   (void *)&root, (void *)&lab,      (void *)&internal, (void *)&size,
                   (void *)&grounded, (void *)&best, (void *)&bestd,    (void *)&nb,   (void *)&err,   (void *)&ctl};
   const int grid = (int)std::max(1LL, std::min((long long)sm_count(), (std::max((long long)m, EE) + kFhThreads - 1) / kFhThreads));
-  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_fh_components, dim3(grid), dim3(kFhThreads), args, 0, s));
-  DLP_TRY(check_launch());
+  DLP_TRY(launch_any_grid((const void *)k_fh_components, grid, kFhThreads, args, 0, s));
   // root[v] is the parent after the last unions: relabelled to the component's smallest vertex
   DLP_CUDA(cudaMemcpyAsync(root, lab, sizeof(int32_t) * (size_t)m, cudaMemcpyDeviceToDevice, s));
   return DLP_OK;

@@ -9,6 +9,7 @@
 
 #include "dlp.h"
 #include "per_device.h"
+#include "resident.h"
 
 namespace dlp {
 
@@ -75,6 +76,39 @@ inline int most_smem(int own) {
       cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     (void)cudaGetLastError();
   return v > own ? v - own : 0;
+}
+
+// Cooperative launches (blocks that wait for one another). kNotLaunched: this device, or the part of it the process
+// has, does not hold the grid; nothing ran and another form of the work can be launched.
+constexpr int kNotLaunched = -1;
+inline Launch try_cooperative(const void *kernel, int grid, int threads, void **args, size_t smem, cudaStream_t s) {
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, s);
+  if (e == cudaSuccess) return Launch::ok;
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorNotPermitted) {
+    (void)cudaGetLastError();
+    return e == cudaErrorCooperativeLaunchTooLarge ? Launch::too_large : Launch::refused;
+  }
+  set_cuda_error(e);
+  return Launch::failed;
+}
+inline int launch_status(Launch r) {
+  return r == Launch::ok ? check_launch() : r == Launch::failed ? (int)DLP_ERR_CUDA : kNotLaunched;
+}
+// A kernel whose blocks own their rows: exactly `grid` blocks, else kNotLaunched.
+inline int launch_cooperative(const void *kernel, int grid, int threads, void **args, size_t smem, cudaStream_t s) {
+  return launch_status(try_cooperative(kernel, grid, threads, args, smem, s));
+}
+// A kernel that takes any number of blocks: at most `grid` (launch_resident).
+inline int launch_any_grid(const void *kernel, int grid, int threads, void **args, size_t smem, cudaStream_t s) {
+  const int st = launch_status(launch_resident(
+      grid, [&](int g) { return try_cooperative(kernel, g, threads, args, smem, s); },
+      [&] {
+        const cudaError_t e = cudaLaunchKernel(kernel, dim3(1), dim3(threads), args, smem, s);
+        if (e == cudaSuccess) return Launch::ok;
+        set_cuda_error(e);
+        return Launch::failed;
+      }));
+  return st == kNotLaunched ? (int)DLP_ERR_CUDA : st;
 }
 
 inline size_t dtype_size(int dt) { return dt == DLP_F64 ? 8 : dt == DLP_F32 ? 4 : dt == DLP_BF16 ? 2 : 0; }

@@ -382,9 +382,7 @@ struct FrRun {
     const int cap = sm_count() * std::min(per, 2);
     const int grid = (int)std::max(1LL, std::min(want, (long long)cap));
     void *args[] = {(void *)&a};
-    DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_frontier_rounds<T, VW, VPL>, dim3(grid), dim3(kFrThreads), args,
-                                         0, s));
-    return check_launch();
+    return launch_any_grid((const void *)k_frontier_rounds<T, VW, VPL>, grid, kFrThreads, args, 0, s);
   }
   template <int VW>
   int launch_vpl(int VPL) {
@@ -407,9 +405,7 @@ template <class T, int VW>
 static int launch_dense(FrDense<T> &a, cudaStream_t s) {
   void *args[] = {(void *)&a};
   const int grid = (a.n + a.rows - 1) / a.rows;
-  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_frontier_dense<T, VW>, dim3(grid), dim3(kFrDenseThreads), args,
-                                       (size_t)a.rows, s));
-  return check_launch();
+  return launch_cooperative((const void *)k_frontier_dense<T, VW>, grid, kFrDenseThreads, args, (size_t)a.rows, s);
 }
 
 template <class T>
@@ -482,7 +478,9 @@ static int run_frontier(const int32_t *rbeg, const int32_t *rend, const int32_t 
       d.ldx[0] = ldx;
       d.X[1] = (TX *)take(sizeof(TX) * nn * (size_t)(C + 3));
       d.ldx[1] = (int64_t)L.NV * L.VW;
-      return run_dense<T>(d, L.VW, seed, nseed, max_rounds, marks, rounds_out, edges_out, s);
+      const int st = run_dense<T>(d, L.VW, seed, nseed, max_rounds, marks, rounds_out, edges_out, s);
+      if (st != kNotLaunched) return st;  // else the lists, on as many blocks as the device holds
+      q = (char *)ws;
     }
   }
   FrRun<T> R;

@@ -1770,8 +1770,7 @@ static size_t whole_state(const PcgProblem &q, int rows) {
   return (size_t)rows * (4 * es * q.C + es + 8 + 8) + 64;
 }
 
-// kNotLaunched: this device does not give the kernel its shared memory; the launched loop takes the solve.
-constexpr int kNotLaunched = -1;
+// kNotLaunched: the launched loop takes the solve.
 template <class T, int VW>
 static int launch_whole_t(WholeArgs<T> &a, cudaStream_t s) {
   auto *kern = k_pcg_whole<T, VW>;
@@ -1779,8 +1778,7 @@ static int launch_whole_t(WholeArgs<T> &a, cudaStream_t s) {
   if (!allow_smem(allowed, (const void *)kern, kWholeSmem)) return kNotLaunched;
   void *argv[] = {(void *)&a};
   const int grid = (a.n + a.rows - 1) / a.rows;
-  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(kWholeThreads), argv, kWholeSmem, s));
-  return check_launch();
+  return launch_cooperative((const void *)kern, grid, kWholeThreads, argv, kWholeSmem, s);
 }
 
 template <class T>

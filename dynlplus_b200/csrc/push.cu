@@ -415,9 +415,8 @@ static int launch_push_t(const PushArgs<T> &a, const PushLaunch &l) {
   const int32_t *cand = l.cand;
   int nc = l.ncand, words = l.words;
   void *args[] = {(void *)&args_a, (void *)&cand, (void *)&nc, (void *)&words};
-  DLP_CUDA(cudaLaunchCooperativeKernel((const void *)k_push_whole<TW, T, CMAX>,
-                                       dim3(sm_count() * std::min(per, kPushPerSm)), dim3(kPushThreads), args, 0, l.s));
-  return check_launch();
+  return launch_any_grid((const void *)k_push_whole<TW, T, CMAX>, sm_count() * std::min(per, kPushPerSm), kPushThreads, args,
+                         0, l.s);
 }
 
 template <typename TW, typename T>

@@ -49,3 +49,34 @@ def test_no_kernel_attribute_is_set_once_per_process():
     where = [(os.path.basename(f), n) for f in glob.glob(os.path.join(CSRC, "*.cu*"))
              for n in [len(re.findall(r"cudaFuncSetAttribute\(", open(f).read()))] if n]
     assert where == [("common.cuh", 1)]
+
+
+def test_resident_kernels_run_on_as_many_blocks_as_the_device_holds(tmp_path):
+    run_cpp(tmp_path, r"""
+#include <cassert>
+#include <vector>
+#include "resident.h"
+using dlp::Launch;
+int main() {
+  std::vector<int> grids;
+  int plain = 0;
+  auto on = [&](int holds, Launch beyond) {  // a device that holds `holds` blocks
+    return [&grids, holds, beyond](int g) { grids.push_back(g); return g <= holds ? Launch::ok : beyond; };
+  };
+  auto one = [&] { ++plain; return Launch::ok; };
+  auto run = [&](int grid, int holds, Launch beyond) { grids.clear(); plain = 0; return dlp::launch_resident(grid, on(holds, beyond), one); };
+  assert(run(296, 296, Launch::too_large) == Launch::ok && grids == std::vector<int>{296} && plain == 0);
+  assert(run(296, 40, Launch::too_large) == Launch::ok && (grids == std::vector<int>{296, 148, 74, 37}) && plain == 0);
+  assert(run(3, 0, Launch::too_large) == Launch::ok && (grids == std::vector<int>{3, 1}) && plain == 1);
+  assert(run(296, 0, Launch::refused) == Launch::ok && grids == std::vector<int>{296} && plain == 1);
+  assert(run(296, 0, Launch::failed) == Launch::failed && grids == std::vector<int>{296} && plain == 0);
+}
+""")
+
+
+def test_every_cooperative_launch_has_another_form():
+    """cudaLaunchCooperativeKernel is called in one place, which tells a refusal from an error; its callers launch
+    another form of the work or a smaller grid then."""
+    where = [(os.path.basename(f), n) for f in sorted(glob.glob(os.path.join(CSRC, "*.cu*")))
+             for n in [len(re.findall(r"cudaLaunchCooperativeKernel\(", open(f).read()))] if n]
+    assert where == [("common.cuh", 1)]
