@@ -1887,10 +1887,11 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
     DLP_CUDA(cudaEventRecord(hs->up, s));
   }
   WholePlan whole;
-  // A recheck at the fp32 floor keeps the two-kernel iteration: its predicted beta recovers from a failed one where
-  // the three-kernel arithmetic of the whole solve drifts off (10,000 x 8 and 60,000 x 8 to 1e-6: 27 and 31
-  // iterations against 426 and a lost iterate).
-  const bool floor_recheck = q.fused && !(mode & 16) && (mode & 2);
+  // A solve that rechecks its own stops keeps the two-kernel iteration, whichever rule stops it: near the fp32 floor
+  // its predicted beta recovers from a failed recheck where the three-kernel arithmetic of the whole solve drifts
+  // off (relative residual 1e-6 on 10,000 x 8 and 60,000 x 8: 27 and 31 iterations against 426 and a lost iterate;
+  // violation 6e-8 there: 22 and 21 against 419 and 420, violations of 30 and 1e8 times the bound).
+  const bool floor_recheck = q.fused && !(mode & 16);
   if (use_graph && !(mode & 8) && !floor_recheck && whole_fits(q, &whole)) {
     const int st = whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s);
     if (st != DLP_OK && st != kNotLaunched) return st;

@@ -261,3 +261,22 @@ def test_a_hub_keeps_the_other_blocks_waiting(call):
         rounds, ok, edges = kernels.FusedPush(A, 1).run(Z, R, diag, [0.9], hub, 5)
         assert (rounds, ok, edges) == (1, True, n - 1) and float(Z[0, 0]) == 1.0
         assert bool((R[1:] == 1.0).all()) and float(R[0, 0]) == 0.0
+
+
+@pytest.mark.parametrize("n,K,weights", [(10_000, 8, "unit"), (60_000, 8, "unit"), (20_000, 8, "lognormal"), (30_000, 12, "lognormal"),
+                                         (50_000, 5, "lognormal")])
+def test_violation_stops_near_the_fp32_floor(n, K, weights):
+    """fp32 solves that stop by the violation rule alone and recheck themselves, down to 6e-8: the device-side loop
+    takes the host loop's iterations and its iterate has the same violation (a failed recheck does not cost it)."""
+    ds = graphs.planted_partition(n, K, 12, 4, weights=weights, seed=3)
+    lab = torch.as_tensor(graphs.label_mask(n, 0.01, seed=3)).cuda()
+    S = stream.build_system(ds, torch.ones_like(lab), lab)
+    S64 = S.astype(torch.float64)
+    for eps in (1e-5, 1.2e-7, 6e-8):
+        out = []
+        for graph in (True, False):
+            Z, st = solvers.padded_empty(S.n_u, K, torch.float32, "cuda", fill=0.0), solvers.Stats()
+            solvers.pcg(S, Z, S.rhs, [eps] * K, solvers.jacobi_M(S), 3000, st, use_graph=graph)
+            R = solvers.residual(S64, Z.double().contiguous(), S64.rhs)
+            out.append((st.iters, float(solvers.rho_cols(S64, R).max()) / eps))
+        assert out[0] == out[1] and out[0][1] <= 2.0
