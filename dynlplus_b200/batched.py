@@ -62,9 +62,9 @@ class BatchedSystems:
         self.set_tiles(tile_rows)
 
     def set_tiles(self, tile_rows):
-        """Cut every instance into tiles of up to tile_rows rows, fewer for small instances (at most some 128
-        tiles each, at least 128 rows): the batch then has enough tiles to fill the chip, and the cut depends
-        on the instance alone, so it gets the same sums in every batch."""
+        """Cut every instance into tiles of up to tile_rows rows, fewer for small instances (some 128 tiles of at
+        least 128 rows, up to 128 * tile_rows rows; beyond, the tiles' number grows): the batch then has enough
+        tiles to fill the chip, and the cut depends on the instance alone, so it gets the same sums in every batch."""
         self.tile_rows = tile_rows
         sizes = np.diff(self.offsets)
         tr = np.full(sizes.shape[0], int(tile_rows), dtype=np.int64)

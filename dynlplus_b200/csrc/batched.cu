@@ -8,7 +8,7 @@
 // (relative residual and/or the reference's violation rule, a true-residual recheck, patience,
 // iteration cap) and stopped instances are skipped by the next iterations. Per iteration four launches: apply
 // (SpMM + pAp), update (alpha from the instance's tiles, R, rz, norms), instance reduce (beta, stop),
-// direction (Z, P). The host queues check_every iterations between reads: the launches cost less than
+// direction (Z, P); a fifth for alpha where an instance may have many tiles. The host queues check_every iterations between reads: the launches cost less than
 // the kernels take, and a graph of them had to be captured again for every new batch (a millisecond each).
 #include <algorithm>
 
@@ -269,9 +269,30 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kBThreads = 256;
 constexpr int kBUnroll = 4;
 
+// pAp over an instance's tiles (a fixed order) and its alpha, for one column, by a warp
+__device__ __forceinline__ double b_fold_alpha(const BCtl &c, int t0, int nt, int C, int x, double rz) {
+  const double s = warp_strided_reduce(c.tp1 + (long long)t0 * C + x, C, nt, false);
+  const double al = s > 0.0 ? rz / s : 0.0;
+  return isfinite(al) && fabs(al) < 1e30 ? al : 0.0;
+}
+
+// Up to kBFoldTiles tiles every block of an instance folds its tiles' pAp for itself, which spares a launch; beyond,
+// where those reads grow with the tiles squared, a block per instance does it once (one system, fp32, a solve in us,
+// folded by all / once: 5 columns, 957 tiles 2,901 / 2,960, 1,914: 5,309 / 5,304, 7,654: 33,179 / 31,183; 9 columns
+// 4,853 / 4,908, 10,027 / 9,850, 52,857 / 46,829).
+constexpr int kBFoldTiles = 1024;
+__global__ void k_b_alpha(int32_t C, BTiles tl, BCtl c) {
+  const int inst = blockIdx.x, t0 = tl.toff[inst], nt = tl.toff[inst + 1] - t0;
+  if (nt <= kBFoldTiles || !b_on(0, c.done[inst])) return;
+  for (int x = threadIdx.x >> 5; x < C; x += blockDim.x >> 5) {
+    const double al = b_fold_alpha(c, t0, nt, C, x, c.rz[(long long)inst * C + x]);
+    if (lane_id() == 0) c.alpha[(long long)inst * C + x] = al;
+  }
+}
+
 // Phase 0: alpha of the tile's instance from its tiles' pAp (every block of the instance folds them in the same
-// order; its first tile's block keeps it, and whether the instance is in this iteration, for the direction
-// sweep), R -= alpha AP; then, as phase 1 (a true residual after a proposed stop) and phase 2 (the start), the
+// order, or k_b_alpha has; its first tile's block keeps it, and whether the instance is in this iteration, for the
+// direction sweep), R -= alpha AP; then, as phase 1 (a true residual after a proposed stop) and phase 2 (the start), the
 // tile's sums of R^2 / diag and R^2 and the largest violation. Phase 3: as 2, R copied from AP (the
 // right-hand side of a zero start). Measured with the direction sweep on the same systems: 57 -> 20 us.
 template <typename TS>
@@ -289,13 +310,11 @@ __global__ void __launch_bounds__(kBThreads) k_b_update(int phase, int32_t C, TS
     if (!act) continue;
     if (phase == 0) {
       for (int x = wid; x < C; x += kBThreads / 32) {
-        const double s = warp_strided_reduce(c.tp1 + (long long)t0 * C + x, C, nt, false);
+        const long long k = (long long)inst * C + x;
+        const double al = nt > kBFoldTiles ? c.alpha[k] : b_fold_alpha(c, t0, nt, C, x, c.rz[k]);
         if (lane == 0) {
-          const long long k = (long long)inst * C + x;
-          double al = s > 0.0 ? c.rz[k] / s : 0.0;
-          al = isfinite(al) && fabs(al) < 1e30 ? al : 0.0;
           s_al[x] = al;
-          if (t == t0) c.alpha[k] = al;
+          if (t == t0 && nt <= kBFoldTiles) c.alpha[k] = al;
         }
       }
       __syncthreads();
@@ -589,6 +608,10 @@ template <typename TS>
 static int b_iteration(const BProblem &q, const BTiles &tl, const BCtl &c, const BParams &bp, cudaStream_t s) {
   if (q.dtype == DLP_F32) DLP_TRY(b_launch_apply<T_F32>(q, tl, c, s));
   else DLP_TRY(b_launch_apply<T_W32X64>(q, tl, c, s));
+  if (tl.ntiles > kBFoldTiles) {
+    k_b_alpha<<<tl.ninst, 256, 0, s>>>(q.C, tl, c);
+    DLP_TRY(check_launch());
+  }
   DLP_TRY(b_update<TS>(0, q, tl, c, s));
   k_b_beta<<<tl.ninst, 256, 0, s>>>(0, q.C, tl, c, bp);
   DLP_TRY(check_launch());

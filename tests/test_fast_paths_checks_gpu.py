@@ -280,3 +280,30 @@ def test_violation_stops_near_the_fp32_floor(n, K, weights):
             R = solvers.residual(S64, Z.double().contiguous(), S64.rhs)
             out.append((st.iters, float(solvers.rho_cols(S64, R).max()) / eps))
         assert out[0] == out[1] and out[0][1] <= 2.0
+
+
+@pytest.mark.parametrize("K,dtype", [(3, "float32"), (8, "float64")])
+def test_batched_alpha_is_folded_once_for_many_tiles(K, dtype):
+    """Instances of 1,024 and 1,025 tiles (where the alphas change from a fold in every tile's block to one of their
+    own): each beside a small instance is bit for bit what it is alone, and from 1,025 tiles on an iteration has one
+    more launch, so that no block but one reads all tiles' sums."""
+    from dynlplus_b200 import _lib
+    dt = getattr(torch, dtype)
+
+    def system(n):  # n rows, all grounded: degree 24 leaves no vertex alone
+        ds = graphs.er_graph(n + 1, 24, K, seed=n)
+        return stream.build_system(ds, torch.ones(n + 1, dtype=torch.bool, device="cuda"),
+                                   torch.arange(n + 1, device="cuda") == n, dtype="float64", eta=0.5)
+    small, launches = system(500), []
+    for n in (1024, 1025):
+        S = system(n)
+        alone = batched.BatchedSystems([S], tile_rows=1, dtype=dt)
+        both = batched.BatchedSystems([small, S], tile_rows=1, dtype=dt)
+        assert alone.ntiles == n
+        before = _lib.lib().dlp_launch_count()
+        Z, it, status, _ = alone.solve(target_relres=1e-5, check_every=64)  # one chunk of 64 iterations, then a recheck
+        launches.append(_lib.lib().dlp_launch_count() - before)
+        Z2, it2, status2, _ = both.solve(target_relres=1e-5, check_every=64)
+        assert status[0] == 5 and (status2 == 5).all() and it[0] == it2[1] < 64
+        assert torch.equal(Z2[both.offsets[1]:], Z)
+    assert launches[1] - launches[0] == 64
