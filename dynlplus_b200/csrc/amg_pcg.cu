@@ -591,11 +591,16 @@ __global__ void __launch_bounds__(kGjThreads, 1) k_gj_whole(int32_t n, int32_t r
   const int tid = threadIdx.x, row0 = blockIdx.x * rows;
   const int nr = max(0, min(rows, n - row0));
   uint32_t target = 0;
+  auto barrier = [&]() -> bool {  // a block whose wait ran out leaves NaN: its rows must not pass as an inverse's
+    if (grid_barrier(bar, target)) return true;
+    for (int i = tid; i < nr * n; i += kGjThreads) A[(long long)row0 * n + i] = __longlong_as_double(0x7ff8000000000000ll);
+    return false;
+  };
   for (int i = tid; i < nr * n; i += kGjThreads) M[i] = A[(long long)row0 * n + i];
   __syncthreads();
   if (row0 == 0)
     for (int j = tid; j < n; j += kGjThreads) __stcg(pub + j, M[j]);
-  if (!grid_barrier(bar, target)) return;
+  if (!barrier()) return;
   for (int k = 0; k < n; ++k) {
     const double *src = pub + (size_t)(k & 1) * n;
     double *dst = pub + (size_t)((k + 1) & 1) * n;
@@ -614,7 +619,7 @@ __global__ void __launch_bounds__(kGjThreads, 1) k_gj_whole(int32_t n, int32_t r
         if (i == next) __stcg(dst + j, v);
       }
     }
-    if (!grid_barrier(bar, target)) return;
+    if (!barrier()) return;
   }
   for (int i = tid; i < nr * n; i += kGjThreads) A[(long long)row0 * n + i] = M[i];
 }
@@ -647,13 +652,7 @@ int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_s
       int32_t nn = n, rr = rows;
       void *args[] = {(void *)&nn, (void *)&rr, (void *)&A, (void *)&fcol, (void *)&bar};
       const int st = launch_cooperative((const void *)k_gj_whole, (n + rows - 1) / rows, kGjThreads, args, smem, s);
-      if (st != DLP_OK && st != kNotLaunched) return st;
-      if (st == DLP_OK) {
-        int32_t lost = 0;  // setup reads back anyway; a wait that ran out must not pass as an inverse
-        DLP_CUDA(cudaMemcpyAsync(&lost, &bar->abort, sizeof(lost), cudaMemcpyDeviceToHost, s));
-        DLP_CUDA(cudaStreamSynchronize(s));
-        return lost ? DLP_ERR_DEVICE : DLP_OK;
-      }
+      if (st != kNotLaunched) return st;
     }
   }
   const int g1 = ceil_div_i(n, 256);

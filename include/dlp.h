@@ -623,7 +623,8 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
 /* The inverse of a dense symmetric positive definite fp64 matrix A (n x n, row-major), in place:
  * Gauss-Jordan elimination without pivoting (the coarsest AMG level's solve, dynlp/amg.py:105-108
  * inverts it with the library's LU): one cooperative launch that keeps the rows in shared memory up to
- * some 1,900 rows (synchronises the stream), two launches per pivot beyond.
+ * some 1,900 rows, two launches per pivot beyond. Asynchronous; where a wait on the device ran out, rows of
+ * NaN are left.
  * Workspace: dlp_dense_spd_inverse_workspace_bytes(n). */
 size_t dlp_dense_spd_inverse_workspace_bytes(int32_t n);
 int dlp_dense_spd_inverse(int32_t n, double *A, void *ws, size_t ws_bytes, dlp_stream_t stream);

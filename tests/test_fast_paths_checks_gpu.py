@@ -307,3 +307,31 @@ def test_batched_alpha_is_folded_once_for_many_tiles(K, dtype):
         assert status[0] == 5 and (status2 == 5).all() and it[0] == it2[1] < 64
         assert torch.equal(Z2[both.offsets[1]:], Z)
     assert launches[1] - launches[0] == 64
+
+
+@pytest.mark.parametrize("n", [300, 1928, 1929, 2100])
+def test_dense_inverse_is_queued_and_captured(n):
+    """The in-place inverse in one launch (up to 1,928 rows here) and with two launches a pivot, as it runs and
+    replayed from a captured graph, against numpy: n unit roundoffs times a condition number of at most 41."""
+    from dynlplus_b200 import _lib
+    from dynlplus_b200.backend import ptr
+    from dynlplus_b200.backend import stream as cur
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-1, 0, (n, n))
+    A = (A + A.T) / 2
+    np.fill_diagonal(A, 0)
+    A[np.arange(n), np.arange(n)] = np.abs(A).sum(1) * 1.05 + 0.01
+    want = np.linalg.inv(A)
+    tol = n * 2.3e-16 * 41 * np.abs(want).max()
+    A = torch.as_tensor(A).cuda()
+    D = A.clone()
+    ws = torch.empty(_lib.lib().dlp_dense_spd_inverse_workspace_bytes(n), dtype=torch.uint8, device="cuda")
+    _lib.call("dlp_dense_spd_inverse", n, ptr(D), ptr(ws), ws.numel(), cur())
+    assert np.abs(D.cpu().numpy() - want).max() <= tol
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        _lib.call("dlp_dense_spd_inverse", n, ptr(D), ptr(ws), ws.numel(), cur())
+    for _ in range(2):
+        D.copy_(A)
+        g.replay()
+        assert np.abs(D.cpu().numpy() - want).max() <= tol
