@@ -76,9 +76,15 @@ def stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def sync():
-    """Wait for the current stream (not the whole device: another thread may be capturing a CUDA
-    graph on its own stream, and a device-wide synchronisation would invalidate that capture)."""
+def sync(dev=None):
+    """Wait for the current stream, of `dev` when given (not the whole device: another thread may be
+    capturing a CUDA graph on its own stream, and a device-wide synchronisation would invalidate that
+    capture)."""
+    if dev is not None and have_cuda():
+        dev = torch.device(dev)
+        if dev.index is not None and dev.index != torch._C._cuda_getDevice():
+            torch.cuda.current_stream(dev).synchronize()  # another device's: its default stream has the same handle
+            return
     _lib.call("dlp_stream_synchronize", stream())
 
 

@@ -67,7 +67,7 @@ def _read_host(x):
     if h is None or h.numel() < x.numel():
         h = bufs[key] = torch.empty(max(x.numel(), 64), dtype=x.dtype, pin_memory=True)
     h[: x.numel()].copy_(x.reshape(-1), non_blocking=True)
-    sync()
+    sync(x.device)
     return h[: x.numel()].tolist()
 
 

@@ -580,7 +580,7 @@ class EdgeStream:
         h = self._h_stat
         h[0:12].copy_(self._stat, non_blocking=True)
         h[12:13].copy_(self._csr_ptr[self.n:self.n + 1], non_blocking=True)
-        sync()
+        sync(self.dev)
         v = h.tolist()
         return {"error": v[0], "overflow": v[1], "deleted": v[2], "inserted": v[3], "moved": v[7],
                 "ground_error": v[5], "changed": v[6], "active": v[8], "ungrounded": v[9], "sweeps": v[10],

@@ -80,3 +80,29 @@ def test_every_cooperative_launch_has_another_form():
     where = [(os.path.basename(f), n) for f in sorted(glob.glob(os.path.join(CSRC, "*.cu*")))
              for n in [len(re.findall(r"cudaLaunchCooperativeKernel\(", open(f).read()))] if n]
     assert where == [("common.cuh", 1)]
+
+
+def test_a_host_read_waits_for_the_stream_of_the_tensors_device(monkeypatch):
+    """A wait for another device's stream is that stream's own: the handle of a default stream names the current
+    device's."""
+    import torch
+    from dynlplus_b200 import backend
+    waited = []
+
+    class Stream:
+        def __init__(self, dev):
+            self.dev = dev
+
+        def synchronize(self):
+            waited.append(self.dev)
+    monkeypatch.setattr(backend, "have_cuda", lambda: True)
+    monkeypatch.setattr(backend, "stream", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream(str(dev)))
+    monkeypatch.setattr(backend._lib, "call", lambda name, handle: waited.append((name, handle)))
+    backend.sync()
+    backend.sync(torch.device("cuda", 0))
+    backend.sync("cuda")
+    backend.sync(torch.device("cuda", 1))
+    here = ("dlp_stream_synchronize", 0)
+    assert waited == [here, here, here, "cuda:1"]
