@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "block_pool.h"
 #include "common.cuh"
 
 namespace dlp {
@@ -504,14 +505,24 @@ int dlp_pcg_amg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, co
     DLP_CUDA(cudaMemcpyAsync(B.eps, e.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
     DLP_CUDA(cudaMemcpyAsync(B.rhsn, e.data() + C, sizeof(double) * C, cudaMemcpyHostToDevice, s));
   }
-  // the decision read back through a pinned word block of this thread (kept for its lifetime)
-  static thread_local GCtl *t_pin = nullptr;
-  if (!t_pin) DLP_CUDA(cudaHostAlloc((void **)&t_pin, sizeof(GCtl), cudaHostAllocPortable));
+  // the decision is read back through a pinned block, borrowed for the call
+  static BlockPool<GCtl> pool;
+  struct Pinned {
+    GCtl *p;
+    ~Pinned() { pool.give(p); }  // every copy into it has been waited for
+  } pin{pool.borrow([]() -> GCtl * {
+    GCtl *q = nullptr;
+    const cudaError_t e = cudaHostAlloc((void **)&q, sizeof(GCtl), cudaHostAllocPortable);
+    if (e == cudaSuccess) return q;
+    set_cuda_error(e);
+    return nullptr;
+  })};
+  if (!pin.p) return DLP_ERR_CUDA;
   GCtl cur{};
   auto read = [&]() -> int {
-    DLP_CUDA(cudaMemcpyAsync(t_pin, B.ctl, sizeof(cur), cudaMemcpyDeviceToHost, s));
+    DLP_CUDA(cudaMemcpyAsync(pin.p, B.ctl, sizeof(cur), cudaMemcpyDeviceToHost, s));
     DLP_CUDA(cudaStreamSynchronize(s));
-    cur = *t_pin;
+    cur = *pin.p;
     return DLP_OK;
   };
   // the initial residual and its decision

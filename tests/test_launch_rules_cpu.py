@@ -16,7 +16,7 @@ def run_cpp(tmp_path, body):
         pytest.skip("no host compiler")
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
     src.write_text(body.lstrip())
-    subprocess.run([gxx, "-std=c++17", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    subprocess.run([gxx, "-std=c++17", "-Wall", "-Werror", "-pthread", "-I", CSRC, str(src), "-o", str(exe)], check=True)
     subprocess.run([str(exe)], check=True, timeout=60)
 
 
@@ -106,3 +106,45 @@ def test_a_host_read_waits_for_the_stream_of_the_tensors_device(monkeypatch):
     backend.sync(torch.device("cuda", 1))
     here = ("dlp_stream_synchronize", 0)
     assert waited == [here, here, here, "cuda:1"]
+
+
+def test_host_blocks_are_kept_per_call_at_once_not_per_thread(tmp_path):
+    run_cpp(tmp_path, r"""
+#include <atomic>
+#include <cassert>
+#include <memory>
+#include <thread>
+#include "block_pool.h"
+int main() {
+  dlp::BlockPool<int> pool;
+  std::atomic<int> made{0}, in{0};
+  auto alloc = [&]() -> int * { ++made; return new int(0); };
+  for (int t = 0; t < 100; ++t)
+    std::thread([&] { int *p = pool.borrow(alloc); *p = 1; pool.give(p); }).join();
+  assert(made == 1);
+  std::vector<std::thread> ts;
+  for (int t = 0; t < 8; ++t)
+    ts.emplace_back([&] {
+      for (int k = 0; k < 2000; ++k) {
+        int *p = pool.borrow(alloc);
+        const int v = ++*p;
+        std::this_thread::yield();
+        assert(*p == v);  // nobody else has the block
+        pool.give(p);
+      }
+    });
+  for (auto &t : ts) t.join();
+  assert(made >= 1 && made <= 8);
+  int *none = pool.borrow([]() -> int * { return nullptr; });
+  pool.give(none);
+  for (int k = 0; k < 9; ++k) none = pool.borrow([]() -> int * { return nullptr; });
+  assert(none == nullptr);
+  pool.give(none);
+  assert(pool.borrow([]() -> int * { return nullptr; }) == nullptr);
+}
+""")
+
+
+def test_no_pinned_block_belongs_to_a_thread_of_the_amg_loop():
+    src = open(os.path.join(CSRC, "amg_pcg.cu")).read()
+    assert "thread_local" not in src and "BlockPool" in src
