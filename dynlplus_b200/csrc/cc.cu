@@ -4,7 +4,6 @@
 // root of each component is its minimum vertex id, whatever the schedule: the result is the
 // reference's canonical labelling before its rank relabel (cc.py:22), bit-exact.
 #include <algorithm>
-#include <cstdlib>
 
 #include "common.cuh"
 
@@ -83,10 +82,10 @@ __global__ void __launch_bounds__(kCcThreads)
 // The edge list's components in rounds, one cooperative launch: every edge whose ends have different roots
 // offers the smaller root to the larger one (atomicMin: the smallest offer of the round stands, an edge whose
 // offer did not is seen again in the next round), then every vertex is pointed at its root. Ends with a
-// round that saw no such edge. The offers spread over the larger roots and no thread retries, where the
-// lock-free unions (k_cc_edges) of a forming giant component meet on a few roots and chase chains that
-// change under them: n = 2M, 1.5M edges (a giant component of half the vertices) 850 -> 188 us; n = 1M, 4M
-// edges 390 -> 260.
+// round that saw no such edge, or after kCcRounds with one pass of unions. The offers spread over the larger
+// roots and no thread retries, where the lock-free unions (k_cc_edges) of a forming giant component meet on a
+// few roots and chase chains that change under them: n = 2M, 1.5M edges (a giant component of half the
+// vertices) 850 -> 188 us; n = 1M, 4M edges 390 -> 260.
 struct CcCtl {
   GridBar bar;
   int32_t open[2];  // the round of each parity saw an edge between two roots
@@ -97,12 +96,20 @@ __device__ __forceinline__ int32_t ld_l1(const int32_t *p) {
   asm volatile("ld.global.ca.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-constexpr int kCcRounds = 64;
+// Rounds before the edges still open are joined by the lock-free unions. A giant component has formed by then and its
+// many edges are closed; the unions of the rest meet on no common root, while further rounds would read every edge
+// again for them (us, 4 / 5 / 6 / 64 rounds: 800,000 vertices of degree 1.26, the slowest of five graphs, 356 / 174 /
+// 177 / 176; 2M in a path in random order 314 / 333 / 358 / 543, the unions alone 298; a grid of 2M in random order
+// 812 / 740 / 454 / 489, the unions alone 2,124).
+constexpr int kCcRounds = 5;
 constexpr int32_t kCcLost = -DLP_ERR_DEVICE;  // *err of a lost wait (an edge's end out of range: DLP_ERR_DEVICE)
-// Where the rounds are used: half a million edges on, and a mean degree above one, where a giant component
-// can form. Below, the unions meet on no common root and are done sooner (whole calls, us, unions / rounds:
-// n = 2M, degree 0.8, 148 / 218; n = 400,000, degree 1.2, 153 / 169; n = 2M, degree 1.5, 1,136 / 298).
+// Where the rounds are used: half a million edges on, a mean degree above 1.25, where a giant component forms, and up
+// to 12M vertices, whose parents the L2 holds beside the edges that pass through. Elsewhere the unions are done sooner
+// (whole calls, us, unions / rounds: n = 2M, degree 0.8, 148 / 218; 4M, 1.05, 285 / 377; 8M, 1.2, 571 / 674; 30M, 1.5,
+// 2,793 / 3,708; 60M, 4, 9,449 / 17,529; inside: n = 1M, degree 1.33, 226 / 199; 2M, 1.5, 878 / 269; 4M, 4, 1,504 / 561;
+// 8M, 1.5, 1,183 / 763; 8M, 10, 3,026 / 1,390; 16M, 1.5, 1,236 / 1,440; 16M, 10, 4,535 / 2,735).
 constexpr int64_t kCcRoundEdges = 500000;
+constexpr int32_t kCcRoundRows = 12000000;
 __global__ void __launch_bounds__(kCcRoundThreads, 2)
     k_cc_rounds(int32_t n, const int32_t *__restrict__ rows, const int32_t *__restrict__ cols, long long m,
                 int32_t *parent, int32_t *err, CcCtl *ctl) {
@@ -130,7 +137,7 @@ __global__ void __launch_bounds__(kCcRoundThreads, 2)
       if (round < kCcRounds) {
         if (__ldcg(parent + hi) > lo) atomicMin(parent + hi, lo);  // most offers to a large root come too late
       } else {
-        unite(parent, a, b, err);  // far past the rounds any graph was seen to take: exact in one pass
+        unite(parent, a, b, err);  // exact in one pass
       }
     }
     if (t0 == 0) ctl->open[(round + 1) & 1] = 0;
@@ -684,7 +691,7 @@ size_t dlp_cc_edges_workspace_bytes(void) { return 256; }
 int dlp_cc_edges_ws(int32_t n, const int32_t *rows, const int32_t *cols, int64_t m, int32_t *parent, int32_t *err,
                     void *ws, size_t ws_bytes, dlp_stream_t stream) {
   if (!ws || ws_bytes < dlp_cc_edges_workspace_bytes() || !err) return DLP_ERR_WORKSPACE;
-  if (n <= 0 || m < kCcRoundEdges || 2 * m <= n) return dlp_cc_edges(n, rows, cols, m, parent, err, stream);
+  if (n <= 0 || n > kCcRoundRows || m < kCcRoundEdges || 8 * m <= 5 * (int64_t)n) return dlp_cc_edges(n, rows, cols, m, parent, err, stream);
   if (!parent || !rows || !cols) return DLP_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
   CcCtl *ctl = (CcCtl *)ws;

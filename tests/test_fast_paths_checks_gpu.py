@@ -335,3 +335,37 @@ def test_dense_inverse_is_queued_and_captured(n):
         D.copy_(A)
         g.replay()
         assert np.abs(D.cpu().numpy() - want).max() <= tol
+
+
+@pytest.mark.parametrize("shape", ["path", "reversed path", "two paths", "grid", "star", "binary tree"])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_components_of_long_and_narrow_graphs(shape, shuffled):
+    """Edge lists whose components take more rounds than are run (the unions join the rest) and those of a few, with
+    vertices in order and in random order, against SciPy; tails of isolated vertices."""
+    import scipy.sparse as ssp
+    from scipy.sparse.csgraph import connected_components
+    n, k = 700_000, np.arange(600_000)
+    if shape == "path":
+        u, v = k[:-1], k[1:]
+    elif shape == "reversed path":
+        u, v = k[::-1][:-1], k[::-1][1:]
+    elif shape == "two paths":
+        u, v = k[:-2], k[2:]
+    elif shape == "grid":
+        s = 770
+        g = np.arange(s * s)
+        u, v = np.r_[g[g % s < s - 1], g[: s * (s - 1)]], np.r_[g[g % s < s - 1] + 1, g[: s * (s - 1)] + s]
+    elif shape == "star":
+        u, v = np.full(k.size - 1, k.size - 1), k[:-1]
+    else:
+        u, v = k[1:], (k[1:] - 1) // 2
+    rng = np.random.default_rng(0)
+    if shuffled:
+        p = rng.permutation(n)
+        u, v = p[u], p[v]
+    _, want = connected_components(ssp.coo_matrix((np.ones(len(u)), (u, v)), (n, n)), directed=False)
+    first = np.full(want.max() + 1, n)
+    np.minimum.at(first, want, np.arange(n))
+    want = np.argsort(np.argsort(first))[want]
+    lab, nc = cc.connected_components(n, torch.as_tensor(u.astype(np.int32)).cuda(), torch.as_tensor(v.astype(np.int32)).cuda())
+    assert nc == want.max() + 1 and np.array_equal(lab.cpu().numpy(), want)
