@@ -27,6 +27,7 @@ __device__ __forceinline__ double fmaa(double a, double b, double c) { return fm
 
 struct Layout {
   int G, LV, NV, VW, VPL;
+  bool two;  // one entry slot where there were two: lanes keep two sums (gather_row's TWO)
 };
 
 constexpr int kThreads = 256;
@@ -44,9 +45,17 @@ static inline int choose_layout(int C, size_t elem, const void *X, int64_t ld, i
   // Measured on B200 (SpMM, degree 16, us): 32 fp32 columns, n = 250,000: 109 -> 75; 16 columns,
   // n = 500,000: 151 -> 99; 5 fp64 columns (three of four lanes), n = 300,000: 75 -> 58; but 17 columns
   // (five of eight lanes) 137 -> 174, 33 columns (nine of sixteen) 100 -> 150.
-  // 33 fp64 columns (seventeen of 32 lanes, n = 250,000): 283 -> 249.
-  const bool spread = L->NV >= 4 ? L->NV <= 32 && ((L->NV & (L->NV - 1)) == 0 || (vec && elem == 8 && L->NV > 16))
-                                 : L->NV == 3 && (elem == 8 || !vec);
+  // 33 fp64 columns (seventeen of 32 lanes, n = 250,000): 283 -> 249; seventeen and more only between the degrees
+  // where that holds (34 columns, n = 100,000: degree 4 38 -> 43, 10 79 -> 70; n = 30,000, degree 100 152 -> 178).
+  // Wider than four vectors they are for rows of few entries (32 fp32 columns, n = 30,000, degree 100: 83 -> 96).
+  // Three values of a row without vectors stay on one lane (fp32, degree 24: 27 -> 33; fp64, degree 100: 56 -> 76),
+  // and so do four bf16 ones (n = 100,000, degree 16: 31 -> 35).
+  const bool pow2 = (L->NV & (L->NV - 1)) == 0;
+  bool spread = false;
+  if (L->NV == 3) spread = vec && elem == 8;
+  else if (L->NV == 4) spread = vec || elem != 2;
+  else if (L->NV > 4 && L->NV <= 32 && avg_deg < 48.0)
+    spread = pow2 || (vec && elem == 8 && L->NV > 16 && avg_deg >= 8.0);
   L->LV = spread ? next_pow2(L->NV) : L->NV <= 4 ? 1 : std::min(32, next_pow2((L->NV + 3) / 4));
   int vpl = (L->NV + L->LV - 1) / L->LV;
   if (vpl > 4) vpl = vpl <= 8 ? 8 : -1;
@@ -58,7 +67,8 @@ static inline int choose_layout(int C, size_t elem, const void *X, int64_t ld, i
   int p = 1;
   while (p * 2 <= es) p *= 2;  // power of two
   es = std::min(p, 32 / L->LV);
-  if (group <= 0 && spread && L->NV >= 8) es = 1;  // 32 columns: 75 us against 86 with two entry slots
+  L->two = group <= 0 && spread && L->NV >= 8;
+  if (L->two) es = 1;  // 32 columns: 75 us against 86 with two entry slots
   if (es < 1) es = 1;
   L->G = L->LV * es;
   return DLP_OK;
@@ -295,8 +305,9 @@ __device__ __forceinline__ void gather_row(const int32_t *__restrict__ col, cons
   for (int k = 0; k < VPL; ++k)
 #pragma unroll
     for (int i = 0; i < VW; ++i) acc[k][i] = TA(0);
-  // TWO (the SpMM and the PCG apply): fp32 lanes of one vector (several lanes per row, then with few entry slots)
-  // keep two sums, of every other entry: the rounding of two slots, whose chains of additions are half as long
+  // TWO (the SpMM and the PCG apply on layouts of one entry slot): fp32 lanes keep two sums, of every other entry: the
+  // rounding of two slots, whose chains of additions are half as long. Its registers cost rows of one lane a fifth of
+  // their rate (bf16, 8 columns, degree 100: 61 -> 78 us), so other layouts are compiled without
   constexpr bool kTwo = TWO && VPL == 1 && ROW == kRowVec && sizeof(TA) == 4 && U % 2 == 0;
   TA odd[kTwo ? VW : 1];
   if constexpr (kTwo) {

@@ -275,7 +275,7 @@ __device__ __forceinline__ float warp_scatter12(const float (&v)[12], int lane) 
   return v1 + __shfl_xor_sync(0xffffffffu, v1, 1);
 }
 
-template <class T, int VW, int VPL, int ROWP = kRowVec, bool FUSE = false>
+template <class T, int VW, int VPL, int ROWP = kRowVec, bool FUSE = false, bool TWO = false>
 __global__ void __launch_bounds__(kThreads, (apply_min_blocks<T, VW, VPL>())) k_pcg_apply(ApplyArgs<T> p) {
   using TA = typename T::TA;
   PcgCtl *ctl = p.B.ctl;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, (apply_min_blocks<T, VW, VPL>())) k_
     // per iteration at n = 1M against two), two 12-float rows
     gather_row<typename T::TW, typename T::TX, TA, VW, VPL,
                (ROWP == kRow8F ? 4 : WHOLE ? 2 : gather_batch_lean<TA, VW, VPL>()),
-               (WHOLE ? ROWP : kRowVec), false, true>(
+               (WHOLE ? ROWP : kRowVec), false, TWO>(
         p.col, p.w, p.P, p.ldp, beg, end, es, ES, cl, LV, NV, G, acc);
     // FUSE: this row's P . AP and AP^2 / diag per column (0 past C and on invalid lanes)
     float pv_[FUSE ? 12 : 1], qv[FUSE ? 12 : 1];
@@ -1397,7 +1397,14 @@ static int launch_apply(const PcgProblem &q, const PcgBufs &B, cudaStream_t s, b
     if (launch) k_pcg_apply<T, VW_, VPL_><<<sm_count() * per, kThreads, 0, s>>>(a);     \
     break;                                                                              \
   }
+#define DLP_APPLY_TWO(VW_)                                                              \
+  {                                                                                     \
+    static const int per = resident_per_sm(k_pcg_apply<T, VW_, 1, kRowVec, false, true>, kThreads); \
+    if (launch) k_pcg_apply<T, VW_, 1, kRowVec, false, true><<<sm_count() * per, kThreads, 0, s>>>(a); \
+    return launch ? check_launch() : DLP_OK;                                            \
+  }
 #define DLP_APPLY_CASE(VW_)                                                             \
+  if (L.VPL == 1 && L.two) DLP_APPLY_TWO(VW_)                                           \
   switch (L.VPL) {                                                                      \
     DLP_APPLY_ONE(VW_, 1)                                                               \
     DLP_APPLY_ONE(VW_, 2)                                                               \
@@ -1443,6 +1450,7 @@ static int launch_apply(const PcgProblem &q, const PcgBufs &B, cudaStream_t s, b
     DLP_APPLY_CASE(VWV)
   }
 #undef DLP_APPLY_CASE
+#undef DLP_APPLY_TWO
 #undef DLP_APPLY_ONE
   return launch ? check_launch() : DLP_OK;
 }

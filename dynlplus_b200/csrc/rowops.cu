@@ -84,7 +84,7 @@ struct SpmmArgs {
 // ROW as in gather_row. kRow12F runs with two rows in flight per lane (measured on B200 at n = 1M,
 // degree 10, C = 9: 133 us against 137 us for per-vector loads with four in flight and 157 us for the
 // two-load path with four).
-template <class T, int VW, int VPL, int ROW = kRowVec>
+template <class T, int VW, int VPL, int ROW = kRowVec, bool TWO = false>
 __global__ void __launch_bounds__(kThreads) k_spmm(SpmmArgs<T> p) {
   using TA = typename T::TA;
   using TX = typename T::TX;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kThreads) k_spmm(SpmmArgs<T> p) {
     // rows (the fp64 residual 278 -> 267 us against two), two 12-float rows (three: 121 -> 133 us)
     gather_row<typename T::TW, TX, TA, VW, VPL,
                (ROW == kRow12F ? 2 : ROW == kRow16H ? 4 : ROW == kRow10D ? 4 : gather_batch_wide<TA, VW, VPL>()),
-               ROW, false, true>(
+               ROW, false, TWO>(
         p.col, p.w, p.X, p.ldx, beg, end, es, ES, cl, LV, NV, G, acc);
     if constexpr (ROW == kRow10D) {
       if (valid && es == 0) {  // same arithmetic, in the same order, as the per-column epilogue below
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads) k_spmm(SpmmArgs<T> p) {
 }
 
 template <class T, int VW>
-static int launch_spmm_vw(const SpmmArgs<T> &a, int VPL, dlp_stream_t s) {
+static int launch_spmm_vw(const SpmmArgs<T> &a, int VPL, bool two, dlp_stream_t s) {
   const int grid = grid_for(a.n_rows, a.G);
   constexpr bool kRow12 =
       VW == 4 && std::is_same<typename T::TX, float>::value && std::is_same<typename T::TA, float>::value;
@@ -264,7 +264,10 @@ static int launch_spmm_vw(const SpmmArgs<T> &a, int VPL, dlp_stream_t s) {
   constexpr bool kRow16 =
       VW == 8 && std::is_same<typename T::TX, bf16>::value && std::is_same<typename T::TA, float>::value;
   switch (VPL) {
-    case 1: k_spmm<T, VW, 1><<<grid, kThreads, 0, (cudaStream_t)s>>>(a); break;
+    case 1:
+      if (two) k_spmm<T, VW, 1, kRowVec, true><<<grid, kThreads, 0, (cudaStream_t)s>>>(a);
+      else k_spmm<T, VW, 1><<<grid, kThreads, 0, (cudaStream_t)s>>>(a);
+      break;
     case 2:
       // bf16 rows of 16 values held whole by one lane: one 256-bit load per gathered row
       if (kRow16 && a.LV == 1 && (uintptr_t)a.X % 32 == 0 && (a.ldx * 2) % 32 == 0) {
@@ -341,8 +344,8 @@ static int run_spmm(const int32_t *rbeg, const int32_t *rend, const int32_t *col
     p.y10 = rows10(Y, ldy);
   }
   constexpr int VWV = 16 / sizeof(typename T::TX);
-  if (L.VW == 1) return launch_spmm_vw<T, 1>(p, L.VPL, s);
-  return launch_spmm_vw<T, VWV>(p, L.VPL, s);
+  if (L.VW == 1) return launch_spmm_vw<T, 1>(p, L.VPL, L.two, s);
+  return launch_spmm_vw<T, VWV>(p, L.VPL, L.two, s);
 }
 
 // Rows of C values copied to a 16-byte pitch, the padding zero: one thread per output vector. Bound by

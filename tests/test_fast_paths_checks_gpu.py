@@ -369,3 +369,27 @@ def test_components_of_long_and_narrow_graphs(shape, shuffled):
     want = np.argsort(np.argsort(first))[want]
     lab, nc = cc.connected_components(n, torch.as_tensor(u.astype(np.int32)).cuda(), torch.as_tensor(v.astype(np.int32)).cuda())
     assert nc == want.max() + 1 and np.array_equal(lab.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float64"])
+@pytest.mark.parametrize("deg", [3, 7, 9, 47, 49])
+def test_spmm_layouts_by_degree(deg, dtype):
+    """Products on both sides of the degrees where the lane layout changes (8 and 48), at the widths that change it,
+    for rows on a vector pitch, packed rows and an offset view, with the library's entry slots and a given number,
+    against the same product in fp64: unit roundoff of the accumulation times the row's length and weight sum."""
+    n, dt = 3001, getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(deg)
+    W = random_csr(n, deg, deg)
+    W = CSR(W.data.to(dt), W.indices, W.indptr, W.shape)
+    W64 = CSR(W.data.double(), W.indices, W.indptr, W.shape)
+    a = torch.rand(n, generator=g, device="cuda").to(torch.float32 if dtype == "bfloat16" else dt)
+    tol = (deg + 2) ** 2 * (2.0 ** -53 if dtype == "float64" else 2.0 ** -24)
+    for C in (3, 4, 6, 16, 17, 32, 34, 48, 63, 64):
+        base = torch.rand((n, C + 8), generator=g, device="cuda").to(dt)
+        padded = solvers.padded_empty(n, C, dt, "cuda", 0.0)
+        padded.copy_(base[:, :C])
+        for X in (padded, base[:, :C].contiguous(), base[:, 1:C + 1]):
+            want = kernels.spmm_axpy(W64, X.double(), a=a.double(), b=-1.0, group=1)
+            for group in ("auto", 1, 4):
+                Y = kernels.spmm_axpy(W, X, a=a, b=-1.0, group=group)
+                assert float((Y.double() - want).abs().max()) <= tol
