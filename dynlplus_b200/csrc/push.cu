@@ -79,12 +79,13 @@ struct PushArgs {
 // The entries of a row are read one per lane of its group and then added CL lanes per entry, a lane for
 // every CL-th column: the adds to a neighbour's row are one run of bytes, one line where a lane per entry
 // touched a line per column (a run of 14 rounds at 17 columns, n = 60,000: 803 -> 434 us; of 11 at 9, n = 1M:
-// 417 -> 363).
+// 417 -> 363). Rows of one and two columns have as many lanes (n = 1M, all rows pushed in six rounds, fp32: 2,502 ->
+// 2,268 and 2,846 -> 2,614).
 template <typename TW, typename T, int CMAX>
 __device__ __forceinline__ void push_scatter(const PushArgs<T> &a, int p, int nf) {
   PushCtl *ctl = a.ctl;
   const TW *__restrict__ w = (const TW *)a.w;
-  constexpr int G = kPushGroup, CL = CMAX <= 4 ? 4 : 8, DC = (CMAX + CL - 1) / CL, ES = G / CL;
+  constexpr int G = kPushGroup, CL = CMAX <= 2 ? CMAX : CMAX <= 4 ? 4 : 8, DC = (CMAX + CL - 1) / CL, ES = G / CL;
   const int lane = lane_id();
   const int gl = lane % G, g0 = lane - gl;  // lane within the row's group
   const int cl = gl % CL, sub = gl / CL;
@@ -387,6 +388,11 @@ static PushArgs<T> push_args(const PushProblem &q, const PushWs &W, const int32_
 // columns, us a run: 215 and 440 with one, 216 and 434 with two, 250 and 563 with four; n = 1M, 9 columns:
 // 401, 363, 451).
 constexpr int kPushPerSm = 2;
+// From so many candidates on the rounds are launched: their phases then want more blocks in flight than a barrier can
+// join cheaply (n = 1M, fp64, us, launched / one launch: 1M candidates, 1 column 15,100 / 22,200, 5 columns 28,500 /
+// 36,300, 17 columns 81,800 / 88,300; 333,000, 1 column 8,040 / 9,990; n = 200,000, all, 1 column 4,620 / 4,700;
+// but 100,000 of 1M 404 / 344).
+constexpr int kPushLaunchRows = 200000;
 
 // What is launched: one round of parity p (its two phases), or the whole run (p < 0).
 struct PushLaunch {
@@ -421,6 +427,8 @@ static int launch_push_t(const PushArgs<T> &a, const PushLaunch &l) {
 
 template <typename TW, typename T>
 static int launch_push_c(const PushProblem &q, const PushArgs<T> &a, const PushLaunch &l) {
+  if (q.C == 1) return launch_push_t<TW, T, 1>(a, l);
+  if (q.C == 2) return launch_push_t<TW, T, 2>(a, l);
   if (q.C <= 4) return launch_push_t<TW, T, 4>(a, l);
   if (q.C <= 12) return launch_push_t<TW, T, 12>(a, l);
   if (q.C <= 20) return launch_push_t<TW, T, 20>(a, l);
@@ -482,7 +490,7 @@ int dlp_fused_push(const int32_t *rbeg, const int32_t *rend, const int32_t *col,
   DLP_CUDA(cudaMemcpyAsync(W.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   const int words = (int)(((long long)n + 31) / 32);
   PushCtl out{};
-  if (use_graph) {
+  if (use_graph && ncand < kPushLaunchRows) {
     DLP_TRY(launch_push(q, W, cancel, PushLaunch{-1, ncand, words, cand, s}));
   } else {
     DLP_CUDA(cudaMemsetAsync(W.bits, 0, sizeof(uint32_t) * (size_t)words, s));

@@ -484,9 +484,9 @@ int dlp_ground_update(int32_t n, const int32_t *parent, const uint8_t *vmask, ui
  * then pushes R[v,:] += w_uv d over their live entries, and the touched rows with
  * any_c |R[v,c]| > eps[c] * diag[v] (compared in the working precision) form the next frontier,
  * until the frontier is empty or max_rounds rounds ran. The frontiers are those of the synchronous
- * push up to the order of the floating-point atomic sums. With use_graph != 0 all rounds run in one
- * cooperative launch (check_every unused); otherwise the host launches each round and
- * reads the control block every check_every rounds. eps is a HOST array of C doubles. C <= 33.
+ * push up to the order of the floating-point atomic sums. With use_graph != 0 and fewer than 200,000
+ * candidates all rounds run in one cooperative launch (check_every unused); otherwise the host launches each
+ * round and reads the control block every check_every rounds. eps is a HOST array of C doubles. C <= 33.
  * (dtype, w_dtype) in {(f32,f32), (f64,f32), (f64,f64)}. Workspace: dlp_fused_push_workspace_bytes.
  * Synchronous: *rounds_out, *converged_out (1 = no row violates), *edges_out (stored entries of the
  * frontier rows, the reference's edge visits). Returns DLP_ERR_CAP when rows still violate after

@@ -393,3 +393,29 @@ def test_spmm_layouts_by_degree(deg, dtype):
             for group in ("auto", 1, 4):
                 Y = kernels.spmm_axpy(W, X, a=a, b=-1.0, group=group)
                 assert float((Y.double() - want).abs().max()) <= tol
+
+
+@pytest.mark.parametrize("count", [199_999, 200_000])
+def test_push_rounds_of_many_candidates_are_launched(count):
+    """On both sides of the number of candidates from which rounds are launched: the launches say which form ran, and
+    both forms' rounds, edge visits and results equal those of the rounds launched on request."""
+    from dynlplus_b200 import _lib
+    n, C = 210_000, 2
+    ds = graphs.er_graph(n, 6, 4, seed=2)
+    lab = torch.as_tensor(graphs.label_mask(n, 0.02, seed=2)).cuda()
+    S = stream.build_system(ds, torch.ones_like(lab), lab, dtype="float64")
+    cand = torch.arange(count, dtype=torch.int32, device="cuda")
+    g = torch.Generator().manual_seed(0)
+    base = torch.rand((S.n_u, C), generator=g, dtype=torch.float64).cuda()
+    out = []
+    for whole in (True, False):
+        Z, R = torch.zeros_like(base), base.clone()
+        before = _lib.lib().dlp_launch_count()
+        rounds, ok, edges = kernels.FusedPush(S.W, C).run(Z, R, S.diag, [5e-2] * C, cand, 12, use_graph=whole)
+        out.append((_lib.lib().dlp_launch_count() - before, rounds, edges, Z, R))
+    (la, ra, ea, za, xa), (lb, rb, eb, zb, xb) = out
+    assert (ra, ea) == (rb, eb) and ra >= 2
+    assert (la == 1) == (count < 200_000) and (la == lb) == (count >= 200_000)
+    # every value is a sum of at most 64 rounded terms a round, each no larger than the largest score times its weight
+    lim = 64 * ra * 2.0 ** -53 * float(S.diag.max()) * float(za.abs().max())
+    assert float((za - zb).abs().max()) <= lim and float((xa - xb).abs().max()) <= lim
