@@ -307,7 +307,7 @@ __global__ void k_cc_gather_rank(const int32_t *__restrict__ parent, int32_t n, 
 // marks nothing ends it (the reached set is then closed under adjacency, i.e. whole components).
 // ------------------------------------------------------------------------------------------------
 // The whole grounding in one cooperative launch: bottom-up sweeps until one reaches nothing new (at most
-// kReachMaxSweeps), the union-find over every live edge where they do not settle (long chains), and the
+// kReachMaxSweeps), the union-find over the rows they left where they do not settle (long chains), and the
 // membership update, with a grid barrier where a launch boundary or a host read was. A settled graph takes
 // four sweeps; launch by launch, each batch of sweeps ended in a host read in the middle of the patch.
 // Bound by the first sweep's row scans (n = 1M, degree 10: 183 us in all) and, below, by the sweeps' number
@@ -361,27 +361,41 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
     settled = __ldcg(flags + sweeps) == 0;
     ++sweeps;
   }
+  // The union-find over what the sweeps left. Every vertex next to the sink was reached by the first sweep, so the sink
+  // itself has no part in it: the reached vertices, all of one component, stand as one, r0, the smallest of them, and
+  // only the rows of the others are walked, both directions of an edge (one alone leaves a path in order as one long
+  // chain: n = 60,000 0.5 -> 4.6 ms). n = 1M, one labelled vertex, us, every row / these: a grid 1,500 / 1,210, in random
+  // order 2,720 / 2,150; a path 1,190 / 880. (The smallest is kept as the largest n - v, of words cleared to zero.)
+  int32_t *least = flags + kReachMaxSweeps;
+  int32_t r0 = n;
   if (!settled) {
-    for (long long v = t0; v <= n; v += step) parent[v] = (int32_t)v;
+    int near = 0;
+    for (long long v = t0; v < n; v += step) {
+      parent[v] = (int32_t)v;
+      if (reached[v]) near = max(near, (int)(n - v));
+    }
+    near = __reduce_max_sync(0xffffffffu, near);
+    if ((threadIdx.x & 31) == 0 && near) atomicMax(least, near);
     if (!barrier()) return;
+    r0 = n - __ldcg(least);
     for (long long u = t0; u < n; u += step) {
-      if (vmask && !vmask[u]) continue;
+      if ((vmask && !vmask[u]) || reached[u]) continue;
       bar_announce(bar, rend[u] - rbeg[u], walked);
       for (int j = rbeg[u]; j < rend[u]; ++j) {
         if (!live(w, j)) continue;
         const int32_t v = col[j];
-        if ((unsigned)v >= (unsigned)n) continue;  // flagged by the sweeps
-        if (!vmask || vmask[v]) unite(parent, (int32_t)u, v, err);
-        else if (sink && sink[v]) unite(parent, (int32_t)u, n, err);
+        if ((unsigned)v >= (unsigned)n || (vmask && !vmask[v])) continue;  // out of range: flagged by the sweeps
+        unite(parent, (int32_t)u, reached[v] ? r0 : v, err);
       }
     }
     if (!barrier()) return;
   }
-  const int32_t root = settled ? 0 : find_root(parent, n, err);
+  // without a reached vertex there is no root to share (r0 is n)
+  const int32_t root = settled || r0 >= n ? -1 : find_root(parent, r0, err);
   int changes = 0, active = 0, lost = 0;
   for (long long v = t0; v < n; v += step) {
     const bool m = !vmask || vmask[v];
-    const bool nu = m && (settled ? reached[v] != 0 : find_root(parent, (int32_t)v, err) == root);
+    const bool nu = m && (reached[v] != 0 || (!settled && find_root(parent, (int32_t)v, err) == root));
     const bool ch = nu != (umask[v] != 0);
     umask[v] = nu ? 1 : 0;
     in_t[v] = ch ? 1 : 0;
@@ -840,8 +854,8 @@ int dlp_ground_reach_async(int32_t n, const int32_t *rbeg, const int32_t *rend, 
   uint8_t *reached = (uint8_t *)base;
   int32_t *flags = (int32_t *)(base + off_flags);
   int32_t *parent = (int32_t *)(base + off_parent);
-  GridBar *bar = (GridBar *)(flags + kReachMaxSweeps);  // in the flags' 256 bytes
-  static_assert(kReachMaxSweeps * sizeof(int32_t) + sizeof(GridBar) <= 256, "flags and barrier share a line of 256 bytes");
+  GridBar *bar = (GridBar *)(flags + kReachMaxSweeps + 1);  // in the flags' 256 bytes, after r0's word
+  static_assert((kReachMaxSweeps + 1) * sizeof(int32_t) + sizeof(GridBar) <= 256, "flags and barrier share a line of 256 bytes");
   DLP_CUDA(cudaMemsetAsync(reached, 0, off_flags + 256, s));  // reached, the flags and the barrier
   auto launch = [&](auto kern, auto *wp) -> int {
     static const int per = [&] {

@@ -419,3 +419,46 @@ def test_push_rounds_of_many_candidates_are_launched(count):
     # every value is a sum of at most 64 rounded terms a round, each no larger than the largest score times its weight
     lim = 64 * ra * 2.0 ** -53 * float(S.diag.max()) * float(za.abs().max())
     assert float((za - zb).abs().max()) <= lim and float((xa - xb).abs().max()) <= lim
+
+
+@pytest.mark.parametrize("shape,n,sinks", [("path", 3000, 1), ("path", 200_000, 3), ("grid", 40_000, 1), ("grid", 250_000, 2),
+                                           ("shuffled grid", 40_000, 1), ("shuffled path", 30_000, 2)])
+def test_grounding_that_sweeps_do_not_settle(shape, n, sinks):
+    """Long graphs, in order and shuffled, with inert entries that cut parts off and vertices outside the mask: the
+    grounded set, its changes and counts against SciPy's components, and the union-find did finish it."""
+    import scipy.sparse as ssp
+    from scipy.sparse.csgraph import connected_components
+    rng = np.random.default_rng(n)
+    k = np.arange(n)
+    if "path" in shape:
+        u, v = k[:-1], k[1:]
+    else:
+        s = int(round(n ** 0.5))
+        u = np.r_[k[k % s < s - 1], k[: s * (s - 1)]]
+        v = np.r_[k[k % s < s - 1] + 1, k[: s * (s - 1)] + s]
+    ends = np.sort(rng.choice(n, sinks, replace=False))
+    cut = rng.random(len(u)) < (0.3 / n ** 0.5 if "path" in shape else 0.05)
+    if shape.startswith("shuffled"):
+        p = rng.permutation(n)
+        u, v, ends = p[u], p[v], p[ends]
+    A = ssp.coo_matrix((np.where(cut, 2.0, 1.0).astype(np.float32), (u, v)), (n, n)).tocsr()
+    A = (A + A.T).tocsr()
+    W = CSR.from_scipy(A)
+    W.data[W.data == 2.0] = 0.0  # stored, inert
+    sink = np.zeros(n, np.uint8)
+    sink[ends] = 1
+    vmask = 1 - sink
+    vmask[rng.integers(0, n, 3)] = 0
+    live = ssp.coo_matrix((np.ones((~cut).sum()), (u[~cut], v[~cut])), (n, n)).tocoo()
+    r, c = np.r_[live.row, live.col], np.r_[live.col, live.row]
+    keep = (vmask[r] > 0) & ((vmask[c] > 0) | (sink[c] > 0))
+    _, lab = connected_components(ssp.coo_matrix((np.ones(keep.sum()), (r[keep], np.where(vmask[c[keep]] > 0, c[keep], n))),
+                                                 (n + 1, n + 1)), directed=False)
+    want = (vmask > 0) & (lab[:n] == lab[n])
+    old = rng.random(n) < 0.5
+    T = lambda x: torch.as_tensor(x.astype(np.uint8)).cuda()  # noqa: E731
+    umask, in_t = T(old), T(np.zeros(n))
+    changes, sweeps = cc.ground_reach(W, T(vmask), T(sink), umask, in_t, w=W.data)
+    assert sweeps == -32 and 0 < want.sum() < n - sinks
+    assert np.array_equal(umask.cpu().numpy() != 0, want)
+    assert changes == (want != old).sum() and np.array_equal(in_t.cpu().numpy() != 0, want != old)
