@@ -505,17 +505,19 @@ struct BProblem {
   int group;
 };
 
-// Mean degree the gather layout is chosen for (two entry slots per row): a fixed one, so that an instance's sums
-// do not depend on the degrees of the others in its batch. (24 fresh systems: 15.1 ms with the batch's own mean,
-// 15.3 with this; 48 with few columns: 10.5 and 10.7.)
-constexpr double kBDegree = 8.0;
+// Mean degree the gather layout is chosen for: a fixed one, so that an instance's sums do not depend on the degrees of
+// the others in its batch. fp32 rows take four entry slots: with two, a row's chains of rounded additions are twice as
+// long, which the corrections' scores show (24 systems of degree 8 to 24 to 1e-6, four seeds, mean of the largest
+// errors 4.97e-8 against 4.69e-8; degree 64 2.75e-8 against 1.52e-8; 15.1 ms against 15.4). fp64 rows take two (48
+// systems 10.7 ms against 11.5).
+constexpr double kBDegree32 = 16.0, kBDegree64 = 8.0;
 
 template <class T>
 static int b_launch_apply(const BProblem &q, const BTiles &tl, const BCtl &c, cudaStream_t s) {
   using TX = typename T::TX;
   Layout L;
-  DLP_TRY(choose_layout(q.C, sizeof(TX), q.P, q.ldp, q.group, kBDegree, &L));
   constexpr bool f32 = sizeof(TX) == 4;
+  DLP_TRY(choose_layout(q.C, sizeof(TX), q.P, q.ldp, q.group, f32 ? kBDegree32 : kBDegree64, &L));
   auto rows = [&](const void *p, int64_t ld, int align, int width) {
     return (uintptr_t)p % align == 0 && (ld * (int64_t)sizeof(TX)) % align == 0 && ld >= width;
   };
@@ -566,7 +568,7 @@ template <class T>
 static int b_launch_residual(int phase, const BProblem &q, const BTiles &tl, const BCtl &c, cudaStream_t s) {
   using TX = typename T::TX;
   Layout L;
-  DLP_TRY(choose_layout(q.C, sizeof(TX), q.Z, q.ldz, q.group, kBDegree, &L));
+  DLP_TRY(choose_layout(q.C, sizeof(TX), q.Z, q.ldz, q.group, kBDegree64, &L));  // (fp64 sums)
   BApply<T> a{q.indptr, q.col, (const typename T::TW *)q.w, q.C, (const TX *)q.Z, q.ldz,
               (const typename T::TV *)q.diag, (typename T::TY *)q.R, q.ldr, tl, c, L.G, L.LV, L.NV};
   const int grid = std::min(tl.ntiles, sm_count() * 8);
@@ -691,7 +693,7 @@ int dlp_pcg_batched(const int32_t *indptr, const int32_t *col, const float *w, i
   BProblem q{indptr, col, w, N, C, diag, rhs, ldrhs, Z, ldz, R, ldr, P, ldp, AP, ldap, dtype, group};
   const size_t iB = 4 * (size_t)ninst;
   (void)use_graph;  // the host drives the loop either way
-  (void)avg_deg;    // (kBDegree)
+  (void)avg_deg;    // (kBDegree32, kBDegree64)
   k_b_init<<<ceil_div_i((long long)ninst * C, 256), 256, 0, s>>>(ninst, C, eps_dev, rhs_norm_dev, c);
   DLP_TRY(check_launch());
   bp.mode = mode & 3;

@@ -462,3 +462,19 @@ def test_grounding_that_sweeps_do_not_settle(shape, n, sinks):
     assert sweeps == -32 and 0 < want.sum() < n - sinks
     assert np.array_equal(umask.cpu().numpy() != 0, want)
     assert changes == (want != old).sum() and np.array_equal(in_t.cpu().numpy() != 0, want != old)
+
+
+@pytest.mark.parametrize("K", [1, 4, 8, 11])
+def test_batched_fp32_rows_are_summed_in_four_slots(K):
+    """The fp32 batched solve adds a row's products in four chains (an accuracy of the scores, whatever the degrees of
+    the batch): bit for bit what four entry slots on request give, at degrees from 6 to 60."""
+    for n, deg in ((3000, 6), (2000, 16), (1000, 60)):
+        ds = graphs.er_graph(n, deg, max(K, 2), seed=n)
+        S = stream.build_system(ds, torch.ones(n, dtype=torch.bool, device="cuda"),
+                                torch.as_tensor(graphs.label_mask(n, 0.05, seed=n)).cuda(), dtype="float32")
+        if K == 1:
+            assert S.C == 1
+        bs = batched.BatchedSystems([S], dtype=torch.float32)
+        a = bs.solve(target_relres=1e-5)
+        b = bs.solve(target_relres=1e-5, group=4)
+        assert a[1][0] == b[1][0] and torch.equal(a[0], b[0])
