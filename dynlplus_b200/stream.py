@@ -49,7 +49,9 @@ class System:
     changed: object = None   # global-index systems: rows whose equation changed
     moved: object = None     # global-index systems: rows that entered or left U this batch
     rhs_h: object = None     # (n, C+1) [rhs | diag], the DynLP+ right-hand side with the h column
-    solved_count: object = None  # global-index systems: the number of solved rows, where it is known
+    # global-index systems: the number of solved rows, where the stream knows it; not handed on by replace(), which
+    # may bring another mask
+    solved_count: object = field(default=None, init=False, repr=False, compare=False)
     _conv: dict = field(default_factory=dict, repr=False, compare=False)
 
     n_u = property(lambda self: int(self.U.numel()))
@@ -75,6 +77,7 @@ class System:
             W = self.W.astype(dt) if isinstance(self.W, CSR) and dt != torch.float64 else self.W
             rh = self.rhs_h.to(dt) if self.rhs_h is not None else None
             self._conv[dt] = replace(self, W=W, rhs_h=rh, _conv={}, **cast)
+            self._conv[dt].solved_count = self.solved_count
         return self._conv[dt]
 
 
@@ -699,7 +702,6 @@ class EdgeStream:
                       eta=self.eta,
                       n_inserted=self.n_ins, n_deleted=self.n_del, n_active=int(n_active),
                       n_ungrounded=int(n_ungrounded), solved=um,
-                      solved_count=int(n_active) - self._n_labeled - int(n_ungrounded),
                       changed=self.last_changed, moved=self.last_moved)
         ch = C + (1 if self.with_h else 0)
         # the grounding stays fp64 in every precision (its one reader, the AMG setup, works in fp64)
@@ -709,6 +711,7 @@ class EdgeStream:
                    **common)
         S._conv[torch.float64] = System(s=s64, diag=self.diag64, B=self.B, rhs=self.rhs64[:, :C], prior=self.prior64,
                                         rhs_h=self.rhs64[:, :ch], **common)
+        S.solved_count = S._conv[torch.float64].solved_count = int(n_active) - self._n_labeled - int(n_ungrounded)
         return S
 
 
