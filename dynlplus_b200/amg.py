@@ -72,8 +72,8 @@ def coarsen(W: CSR, s, agg, nc, off=None, mem=None):
         off, mem = members(agg, nc)
     key = torch.empty(max(m, 1), dtype=torch.int64, device=dev)
     val = torch.empty(max(m, 1), dtype=torch.float64, device=dev)
-    _lib.call("dlp_amg_coarse_keys", n, ptr(W.indptr), ptr(W.indices), ptr(W.data.float().contiguous()),
-              ptr(agg.to(torch.int32).contiguous()), nc, ptr(key), ptr(val), stream())
+    w, agg = W.data.float().contiguous(), agg.to(torch.int32).contiguous()  # bound: the kernel gets bare addresses
+    _lib.call("dlp_amg_coarse_keys", n, ptr(W.indptr), ptr(W.indices), ptr(w), ptr(agg), nc, ptr(key), ptr(val), stream())
     key, val = key[:m], val[:m]
     if m > 1:  # stable radix sort by coarse entry; the "no entry" marker sorts last
         kt = torch.empty_like(key)

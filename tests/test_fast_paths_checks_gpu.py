@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from dynlplus_b200 import batched, cc, graphs, kernels, solvers, stream
+from dynlplus_b200 import amg, batched, cc, graphs, kernels, solvers, stream
 from dynlplus_b200.backend import CSR
 
 pytestmark = pytest.mark.gpu
@@ -478,3 +478,14 @@ def test_batched_fp32_rows_are_summed_in_four_slots(K):
         a = bs.solve(target_relres=1e-5)
         b = bs.solve(target_relres=1e-5, group=4)
         assert a[1][0] == b[1][0] and torch.equal(a[0], b[0])
+
+
+def test_coarse_operator_of_converted_inputs():
+    """Weights and aggregates that are converted on the way give the coarse operator of their fp32 and int32 copies."""
+    n, nc = 200_000, 50
+    W = random_csr(n, 1, 3)  # as many entries as rows: the copies are of one size
+    agg = torch.randint(0, nc, (n,), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    want, _ = amg.coarsen(W, None, agg.to(torch.int32), nc)
+    wide = torch.stack([agg, agg], 1)[:, 0]  # int64, strided
+    got, _ = amg.coarsen(CSR(W.data.double(), W.indices, W.indptr, W.shape), None, wide, nc)
+    assert all(torch.equal(a, b) for a, b in ((got.indptr, want.indptr), (got.indices, want.indices), (got.data, want.data)))
