@@ -55,7 +55,7 @@ class BatchedSystems:
         self.diag = self.diag64.to(dtype)
         # from each system's own rhs and diag (its [rhs | diag] copy does not follow a replaced right-hand side)
         self.rhs64 = torch.empty((N, self.Ch), dtype=torch.float64, device=dev)
-        torch.cat([s.rhs for s in s64], out=self.rhs64[:, :self.C])
+        self.rhs64[:, :self.C] = torch.cat([s.rhs for s in s64])  # (into the columns directly: a copy per system)
         if with_h:
             self.rhs64[:, self.C] = self.diag64
         self.rhs = self.rhs64.to(dtype)
