@@ -8,13 +8,14 @@
 //   (a) AP = diag P - W P, pAp;   all-to-all sum, alpha
 //   (b) R -= alpha AP, rz, ||R||^2, violation;   all-to-all sum, stop decision, beta
 //   (c) Z += alpha P, P = R / diag + beta P;   barrier
-// What bounds it: the L1's rate of gathered lines (about one line per two cycles and SM, whatever a lane
-// takes of it), so the rows are spread over every SM and a lane gathers 32 bytes in one access where the
-// rows allow; and the three grid barriers (some 3,000 cycles each on this chip: a store or an atomic takes
-// about 1,000 to be seen by another SM's load). Each block folds all blocks' partial sums itself, in the
-// same order: the same bits everywhere, so each takes the same decision and none has to publish it. (Words
-// of value and tag that every block polls for every other, one trip instead of three, measured 8,000
-// cycles at 148 blocks: the polls of all blocks meet on the same lines.) All waits are bounded.
+// What bounds it: the three grid barriers (some 3,000 cycles each on this chip: a store or an atomic takes about
+// 1,000 to be seen by another SM's load); at n = 30,000 and 5 columns waiting warps there are four times those
+// waiting for loads, with the L1 18% busy. Towards the largest systems the gathers count (about one line per two
+// cycles and SM, whatever a lane takes of it), so the rows are spread over every SM and a lane gathers 32 bytes in
+// one access where the rows allow. Each block folds all blocks' partial sums itself, in the same order: the same
+// bits everywhere, so each takes the same decision and none has to publish it. (Words of value and tag that every
+// block polls for every other, one trip instead of three, measured 8,000 cycles at 148 blocks: the polls of all
+// blocks meet on the same lines.) All waits are bounded.
 #pragma once
 
 namespace dlp {

@@ -419,8 +419,8 @@ def push(sys: System, Z, R, eps, ops: FrontierOps, st: Stats, budget_edges=None,
 
 def _comp_avg(lab, nc, S_rows, T_rows, fallback):
     """Per component of the new vertices: sum of S over sum of T (T = 0: fallback)
-    (dynlp/solvers.py:128-135). Summed in fp64, so the order of the atomic additions does not reach the
-    working precision: a last-bit difference here decides which rows a frontier sweep's threshold lets
+    (dynlp/solvers.py:128-135). Summed in fp64, so the order of the atomic additions seldom reaches an
+    fp32 working precision: a last-bit difference here decides which rows a frontier sweep's threshold lets
     move, and two runs of one stream differed by 1e-4."""
     lab = lab.long()
     S = torch.zeros((nc,) + tuple(S_rows.shape[1:]), dtype=F64, device=S_rows.device).index_add_(0, lab, S_rows.to(F64))
