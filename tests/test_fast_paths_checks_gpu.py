@@ -489,3 +489,8 @@ def test_coarse_operator_of_converted_inputs():
     wide = torch.stack([agg, agg], 1)[:, 0]  # int64, strided
     got, _ = amg.coarsen(CSR(W.data.double(), W.indices, W.indptr, W.shape), None, wide, nc)
     assert all(torch.equal(a, b) for a, b in ((got.indptr, want.indptr), (got.indices, want.indices), (got.data, want.data)))
+
+
+def test_rows_are_taken_by_ids_on_the_host():
+    X, idx = torch.randn(100, 5, device="cuda", dtype=torch.float64), torch.tensor([3, 99, 0])
+    assert torch.equal(kernels.rows_take(X, idx, torch.float32), X[idx].float())
