@@ -24,10 +24,13 @@ class BlockPool {
     }
     return alloc();
   }
-  void give(T *p) {
+  void give(T *p) noexcept {
     if (!p) return;
-    std::lock_guard<std::mutex> lk(mu_);
-    free_.push_back(p);
+    try {
+      std::lock_guard<std::mutex> lk(mu_);
+      free_.push_back(p);
+    } catch (...) {  // no room for the pointer: the block is not lent again
+    }
   }
 
  private:
