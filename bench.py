@@ -944,7 +944,7 @@ def wl_kernels(a):
         _, frows, trows, _ = fp.counts()
         sz = 8 if dt == torch.float64 else 4
         algo = frows * (12 + 4 * C * sz + 4) + edges * (8 + 4 + 2 * C * sz) + trows * (8 + C * sz + sz)
-        out[name] = line("k_push_whole (the whole dlp_fused_push call)", algo, float(np.median(ms)),
+        out[name] = line("push rounds (the whole dlp_fused_push call)", algo, float(np.median(ms)),
                          rounds=rounds, converged=ok, candidates=int(cand.numel()), frontier_rows=frows,
                          touched_rows=trows, entries=edges)
     del ct
