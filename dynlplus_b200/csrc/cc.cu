@@ -333,10 +333,11 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
     return false;
   };
   int sweeps = 0;
-  uint32_t walked = 0;
+  uint32_t walked;
   bool settled = false;
   while (!settled && sweeps < kReachMaxSweeps) {  // flags and reached were cleared before the launch
     bool any = false;
+    walked = 0;
     for (long long u = t0; u < n; u += step) {
       if ((vmask && !vmask[u]) || reached[u]) continue;
       const int beg = rbeg[u], end = rend[u];
@@ -378,6 +379,7 @@ __global__ void __launch_bounds__(kGroundThreads, 2)
     if ((threadIdx.x & 31) == 0 && near) atomicMax(least, near);
     if (!barrier()) return;
     r0 = n - __ldcg(least);
+    walked = 0;
     for (long long u = t0; u < n; u += step) {
       if ((vmask && !vmask[u]) || reached[u]) continue;
       bar_announce(bar, rend[u] - rbeg[u], walked);

@@ -184,7 +184,7 @@ constexpr int kBarSpins = 1 << 22;
 constexpr unsigned long long kBarPerEntry = 16;
 constexpr int kBarLongRow = 1 << 15;  // a row of so many entries is announced
 
-// `mine`: the entries in long rows that this thread has walked since the kernel began.
+// `mine`: the entries in long rows that this thread walks between two barriers (its caller zeroes it after each).
 __device__ __forceinline__ void bar_announce(GridBar *b, int entries, uint32_t &mine) {
   if (entries < kBarLongRow) return;
   mine = mine + (uint32_t)entries < mine ? 0xffffffffu : mine + (uint32_t)entries;

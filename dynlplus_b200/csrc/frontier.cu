@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int r0 = __ldcg(&ctl->round);
-  uint32_t bar = 0, walked = 0;
+  uint32_t bar = 0;
   unsigned long long edges = 0;
   int done = 0, status = 0;
   for (; done < p.max_rounds; ++done) {
@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
       ctl->ucnt[sn] = 0;
     }
     const int32_t *front = p.front[rd & 1];
+    uint32_t walked = 0;
     for (long long g0 = warp * gpw; g0 < nf; g0 += nwarps * gpw) {
       const long long gi = g0 + lane / G;
       const bool valid = gi < nf;
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kFrThreads) k_frontier_rounds(FrArgs<T> p) {
     }
     // eight lanes per changed row; entry 0 is the row itself
     int32_t *next = p.front[(rd + 1) & 1];
+    walked = 0;
     for (long long g0 = warp * 4; g0 < nu; g0 += nwarps * 4) {
       const long long i = g0 + (lane >> 3);
       const bool valid = i < nu;
