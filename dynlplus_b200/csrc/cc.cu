@@ -434,8 +434,8 @@ struct FhCtl {
   int32_t bad;            // an edge's end outside [-m, m): nothing is merged
 };
 
-__device__ __forceinline__ uint32_t float_order(float x) {  // monotone in the float's order
-  const uint32_t b = __float_as_uint(x);
+__device__ __forceinline__ uint32_t float_order(float x) {  // monotone in the float's order (x + 0: both zeros are equal)
+  const uint32_t b = __float_as_uint(__fadd_rn(x, 0.f));
   return b & 0x80000000u ? ~b : b | 0x80000000u;
 }
 

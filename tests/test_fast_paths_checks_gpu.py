@@ -186,6 +186,15 @@ def test_fh_components_checks_its_edges(m):
                 cc.fh_components(m, *ends, d, 0.3, ground)
 
 
+@pytest.mark.parametrize("first", [0.0, -0.0])
+def test_fh_components_takes_both_zeros_as_equal(first):
+    """Of two lightest edges, one of weight 0 and one of weight -0, the one to the smaller component is taken."""
+    rows, cols = torch.tensor([[0, 1, 0, 2], [1, 0, 2, 0]], device="cuda")
+    d = torch.tensor([first, first, -first, -first], device="cuda")
+    lab, nc = cc.fh_components(3, rows, cols, d, -1.0, torch.tensor([0.0, 1.0, 1.0], device="cuda"))
+    assert nc == 2 and lab.tolist() == [0, 0, 1]
+
+
 LOST_WAIT = r"""
 #include "cc.cu"
 // The grounding kernel as it is launched, on two blocks, with its barrier's `abort` set beforehand: a block that has to
