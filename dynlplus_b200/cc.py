@@ -106,6 +106,13 @@ def ground_reach(G, vmask, sink, umask, in_t, w=None):
 # ---------------------------------------------------------------------------------------------
 # adaptive components of new vertices (dynlp/cc.py:26-83)
 # ---------------------------------------------------------------------------------------------
+def _ids32(ids):
+    """int32 ids; one past int32 becomes its lowest or highest value, out of range for the kernel too."""
+    if ids.dtype == torch.int64:
+        ids = ids.clamp(-2**31, 2**31 - 1)
+    return ids.to(torch.int32).contiguous()
+
+
 def fh_components(m, rows, cols, d, k, ground=None):
     """Felzenszwalb-Huttenlocher merging in Boruvka rounds (dynlp/cc.py:37-73): each round every
     component takes its lightest outgoing edge (ties to the smallest other side) and merges across it
@@ -119,7 +126,7 @@ def fh_components(m, rows, cols, d, k, ground=None):
         raise IndexError(f"{tuple(rows.shape)}, {tuple(cols.shape)} and {tuple(d.shape)} edge ends and weights")
     if ground is not None and ground.shape != (m,):
         raise IndexError(f"ground of shape {tuple(ground.shape)} for {m} vertices")
-    rows, cols = rows.to(torch.int32).contiguous(), cols.to(torch.int32).contiguous()
+    rows, cols = _ids32(rows), _ids32(cols)
     d = d.to(torch.float32).contiguous()
     g = ground.to(torch.float32).contiguous() if ground is not None else None
     root = torch.empty(m, dtype=torch.int32, device=dev)

@@ -186,6 +186,14 @@ def test_fh_components_checks_its_edges(m):
                 cc.fh_components(m, *ends, d, 0.3, ground)
 
 
+@pytest.mark.parametrize("end", [2**32 + 1, -2**32 + 1, 2**31, 2**63 - 1])
+def test_fh_components_refuses_ends_past_int32(end):
+    rows, cols = torch.tensor([[0, 1, 0, 2], [1, 0, 2, 0]], device="cuda")
+    cols[0] = end
+    with pytest.raises(IndexError):
+        cc.fh_components(3, rows, cols, torch.ones(4, device="cuda"), 0.5)
+
+
 @pytest.mark.parametrize("first", [0.0, -0.0])
 def test_fh_components_takes_both_zeros_as_equal(first):
     """Of two lightest edges, one of weight 0 and one of weight -0, the one to the smaller component is taken."""
