@@ -115,7 +115,7 @@ __global__ void k_rows_take(long long total, int32_t C, long long n_src, const T
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
     const long long r = t / C;
     const int c = (int)(t - r * C);
-    const long long q = idx[r];
+    const long long i = idx[r], q = i < 0 ? i + n_src : i;  // a negative index counts from the last row
     // an index outside the source gives NaN, not a read out of range
     dst[r * ldd + c] = q >= 0 && q < n_src ? (TD)src[q * lds + c] : (TD)__longlong_as_double(0x7ff8000000000000ll);
   }

@@ -220,7 +220,7 @@ class FrontierOps:
 
 
 def rows_take(X, idx, dtype, out=None):
-    """X[idx] (row ids) in `dtype`, into `out` when given."""
+    """X[idx] (row ids) in `dtype`, into `out` when given. Rows of ids on the device that X does not have are NaN."""
     floats = (torch.float32, torch.float64)
     if not X.is_cuda or not idx.is_cuda or idx.dtype != torch.int64 or X.dtype not in floats or dtype not in floats or X.stride(1) != 1:
         Y = X[idx].to(dtype)

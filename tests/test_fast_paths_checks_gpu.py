@@ -511,3 +511,11 @@ def test_coarse_operator_of_converted_inputs():
 def test_rows_are_taken_by_ids_on_the_host():
     X, idx = torch.randn(100, 5, device="cuda", dtype=torch.float64), torch.tensor([3, 99, 0])
     assert torch.equal(kernels.rows_take(X, idx, torch.float32), X[idx].float())
+
+
+@pytest.mark.parametrize("C", [1, 5])
+def test_rows_are_taken_by_negative_ids(C):
+    X = torch.randn(100, C, device="cuda", dtype=torch.float64)
+    idx = torch.tensor([-1, 0, -100, 99, -37], device="cuda")
+    assert torch.equal(kernels.rows_take(X, idx, torch.float32), X[idx].float())
+    assert torch.isnan(kernels.rows_take(X, torch.tensor([100, -101], device="cuda"), torch.float32)).all()
