@@ -426,7 +426,8 @@ int dlp_cols_scale(int32_t n, int32_t C, const void *X, int64_t ldx, int x_dtype
                    void *Y, int64_t ldy, int y_dtype, dlp_stream_t stream);
 
 /* dst[i, 0..C) = src[idx[i], 0..C) (a solver's rows U of its resident scores), converted between f32 and
- * f64; an index outside [0, n_src) gives NaN. src and dst must not overlap. */
+ * f64; a negative index counts from the last row, one outside [-n_src, n_src) gives NaN. src and dst must
+ * not overlap. */
 int dlp_rows_take(int64_t n, int32_t C, int64_t n_src, const void *src, int64_t lds, int src_dtype, const int64_t *idx,
                   void *dst, int64_t ldd, int dst_dtype, dlp_stream_t stream);
 
