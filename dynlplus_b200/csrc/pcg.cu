@@ -1899,7 +1899,15 @@ int dlp_pcg(const int32_t *rbeg, const int32_t *rend, const int32_t *col, const 
   // its predicted beta recovers from a failed recheck where the three-kernel arithmetic of the whole solve drifts
   // off (relative residual 1e-6 on 10,000 x 8 and 60,000 x 8: 27 and 31 iterations against 426 and a lost iterate;
   // violation 6e-8 there: 22 and 21 against 419 and 420, violations of 30 and 1e8 times the bound).
-  const bool floor_recheck = q.fused && !(mode & 16);
+  // So does, with the three launched kernels, one of another width that is asked for less than its precision resolves
+  // (25 epsilons: 3e-6 in fp32). It rechecks until its patience ends and keeps what it then has, which drifts further
+  // from the one launch's sums (1e-6, 1 to 4 columns: of 36 solves at n = 3,000 6 end above 1e-4, 17 in one launch, the
+  // worst at 1.9e-3 and 0.13; the last batches of a stream, n = 20,000, above 5e-2 in 1 of 120 runs and 15). From 3e-6
+  // on every one of 205 solves converged in either form.
+  const double reach = 25.0 * (dtype == DLP_F32 ? 1.1920928955078125e-07 : 2.220446049250313e-16);
+  bool beyond = (mode & 2) && target_relres < reach;
+  for (int c = 0; c < C && (mode & 1); ++c) beyond = beyond || eps[c] < reach;
+  const bool floor_recheck = (q.fused || beyond) && !(mode & 16);
   if (use_graph && !(mode & 8) && !floor_recheck && whole_fits(q, &whole)) {
     const int st = whole_solve(q, B, whole, (mode & 4) != 0, !(mode & 16), s);
     if (st != DLP_OK && st != kNotLaunched) return st;

@@ -328,8 +328,9 @@ int dlp_residual_stats(int32_t n, int32_t C, const void *R, int64_t ldr, const v
  * use_graph != 0 the iteration loop runs on the device as one CUDA graph with a conditional WHILE
  * node (cached per problem; the host reads the control block once per loop and once per recheck);
  * where conditional nodes are unavailable, chunks of check_every iterations are replayed as graphs.
- * Small systems (up to 100,000 rows and a few MB of scores; no bf16 mirror, bit 3 clear, not the two-kernel
- * iteration with its own rechecks (bit 4 clear), P's rows whole 16- or 32-byte vectors) run the whole solve in one cooperative launch instead, with the three-kernel
+ * Small systems (up to 100,000 rows and a few MB of scores; no bf16 mirror, bit 3 clear, P's rows whole 16- or
+ * 32-byte vectors; with rechecks of its own (bit 4 clear) neither the two-kernel iteration nor a target or bound
+ * under 25 epsilons of the precision) run the whole solve in one cooperative launch instead, with the three-kernel
  * iteration's arithmetic; AP is not used there.
  * use_graph == 0 launches the kernels directly and reads the control block every check_every
  * iterations.

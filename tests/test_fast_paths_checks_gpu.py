@@ -299,6 +299,24 @@ def test_violation_stops_near_the_fp32_floor(n, K, weights):
         assert out[0] == out[1] and out[0][1] <= 2.0
 
 
+@pytest.mark.parametrize("rule", ["relres", "violation"])
+@pytest.mark.parametrize("n,K", [(3000, 2), (3000, 3), (20_000, 4), (3000, 16)])
+def test_solves_beyond_their_precision_keep_the_launched_loop(n, K, rule):
+    """A solve that rechecks its stops and is asked for less than fp32 resolves ends where the launched kernels end, bit
+    for bit: the sums of the one launch drift further before its patience ends."""
+    ds = graphs.er_graph(n, 10, K, seed=n + K)
+    S = stream.build_system(ds, torch.ones(n, dtype=torch.bool, device="cuda"),
+                            torch.as_tensor(graphs.label_mask(n, 0.02, seed=n)).cuda(), dtype="float32")
+    eps, target = ([1e-7] * S.C, None) if rule == "violation" else (None, 1e-6)
+    out = []
+    for use_graph in (None, False):
+        Z, st = solvers.padded_empty(S.n_u, S.C, torch.float32, "cuda", fill=0.5), solvers.Stats()
+        solvers.pcg(S, Z, S.rhs.contiguous(), eps, solvers.jacobi_M(S), 100_000, st, target_relres=target,
+                    use_graph=use_graph)
+        out.append((st.iters, Z.clone()))
+    assert out[0][0] == out[1][0] and torch.equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("K,dtype", [(3, "float32"), (8, "float64")])
 def test_batched_alpha_is_folded_once_for_many_tiles(K, dtype):
     """Instances of 1,024 and 1,025 tiles (where the alphas change from a fold in every tile's block to one of their
